@@ -31,6 +31,7 @@
 #include <omp.h>
 #include <type_traits>
 
+#include "bulk.cuh"
 #include "closed_inverse.cuh"
 #include "common.cuh"
 
@@ -42,6 +43,17 @@ constexpr long long NONE = LLONG_MAX;
 // ------------------------------------------------------------------------------------------------------------------
 // Plan
 // ------------------------------------------------------------------------------------------------------------------
+// The "runs" schedule of one storage type (column_runs.cuh)
+struct RunSchedule {
+  bool ok = false;
+  int exact = 0;   // DR of the exact-size kernel (6 to 9, with d_e = 3), 0: k_runs_any
+  int64_t items = 0;
+  int tile_bytes = 0, blob_bytes = 0, smem = 0, wr = 0, ts = 0, mdr = 0, mde = 0;
+  int grid = 0;    // resident CTAs per SM x SMs (set at the first launch)
+  DevBuf items_d, segs, blob;
+  int64_t bytes() const { return (int64_t)(items_d.bytes + segs.bytes + blob.bytes); }
+};
+
 struct SchurPlan {
   bls_ctx* ctx = nullptr;
   int64_t nrblocks = 0, neblocks = 0, nr = 0, ne = 0, ncoup = 0, E_length = 0, C_length = 0;
@@ -75,7 +87,7 @@ struct SchurPlan {
   // {visit within the item | c1's index within its point << 16}, 0 past a lane's unit (stg_pairs).
   // One schedule per storage type (index 0 FP32, 1 FP64): FP32 items fit two 256-thread CTAs per SM, FP64 items (half
   // the visits) two 128-thread CTAs.
-  bool stage_ok = false;
+  bool stage_ok[2] = {false, false};   // per storage type: its schedule is built (at plan creation where "stage" takes it)
   // per schedule, the unit size (measured on the 1M-point scene: FP32 1.73 ms at 16, 1.62 at 20, 1.68 at 24; FP64
   // 3.07 ms at 16, 3.30 at 20; on the 200k-point scene FP32 0.318 / 0.303 / 0.300 ms and FP64 0.468 ms at 16)
   int stage_unit[2] = {20, 16};
@@ -84,6 +96,9 @@ struct SchurPlan {
     DevBuf stg_items, stg_ibat, stg_bat, stg_lane, stg_pairs;
   };
   StageSchedule stage[2];
+  RunSchedule runs[2];          // the "runs" schedule, FP32 and FP64
+  bool runs_first[2] = {false, false};   // "stage" takes k_runs, not k_stage36, for a sparse S of 6 x 6 blocks
+  bool points3 = false;         // every e_dim is 3 and eoffsets are canonical (9 e): k_factor36 serves the plan
   int stage_grid[2] = {0, 0};   // persistent CTAs of k_stage36 (FP32, FP64): resident blocks per SM x SMs
   DevBuf EZ;   // per point E' = s_e E^-1 s_e (9, column-major) and z' = s_e .* z (3), FP64, for k_stage36
   // a batch of independent problems in one plan (bls_schur_plan_set_problems): per problem the lowest failing point
@@ -158,6 +173,7 @@ __global__ void k_check_scaling(const double* __restrict__ sc, int64_t n, Status
 __device__ __forceinline__ bool args_ok(const Status* st) { return st->einval_r == NONE && st->einval_e == NONE; }
 // The reduction's failure word starts clear when the arguments are valid
 __global__ void k_arm(Status* st) {
+  st->pad = 0;   // the work queue of k_runs_any
   if (args_ok(st)) st->failed = NONE;
 }
 
@@ -1766,6 +1782,8 @@ __global__ void __launch_bounds__(stage_nt<T>(), 2) k_stage36(
   }
 }
 
+#include "column_runs.cuh"
+
 // One column-owned schedule of k_stage36 (SchurPlan::stage[sd], sd 0 for FP32 and 1 for FP64), from the structure:
 // each column's pairs grouped by block slot, each block's in visit order. An item is a run of one block column's
 // visits: its shared memory holds the column's S tile (6 H entries) and per visit W = E' C_c2 (18 entries) and the
@@ -2178,13 +2196,49 @@ static SchurPlan* plan_create(bls_ctx* ctx, const bls_schur_plan_desc* d) {
       }
     }
   }
-  // the column-owned schedule (k_stage36), sparse S only
-  if (P->fast36 && P->has_sparse) {
-    bool ok = true;
-    for (int sd = 0; sd < 2 && ok; ++sd)
-      ok = build_stage_schedule(P.get(), sd, s, nrb, rptr, rentry, entry_elim, d->eliminated_ptr, d->entry_retained, bcolptr,
-                                browval, brow_off, col_h);
-    P->stage_ok = ok;
+  {
+    P->points3 = true;
+    for (int64_t e = 0; e < neb && P->points3; ++e) P->points3 = d->e_dims[e] == 3 && d->eoffsets[e] == 9 * e;
+    const RunInput in{nrb, neb, clen, d->r_dims, d->e_dims, d->eliminated_ptr, d->entry_retained, d->coffsets, &rptr, &rentry, &entry_elim, &bcolptr, &browval};
+    const bool contiguous = runs_contiguous(in);
+    int run_exact = 0;
+    if (contiguous) {
+      // the exact-size kernels: one retained size of 6 to 9, canonical point and coupling storage
+      int exact = P->points3 && P->max_dr >= 6 && P->max_dr <= 9 ? P->max_dr : 0;
+      for (int64_t r = 0; r < nrb && exact; ++r) exact = d->r_dims[r] == exact ? exact : 0;
+      for (int64_t c = 0; c < nc && exact; ++c) exact = d->coffsets[c] == 3 * exact * c ? exact : 0;
+      run_exact = exact;
+    }
+    const bool gather = P->fast36 && P->has_sparse;
+    if (gather) {
+      // k_runs against k_stage36 for a sparse S of 6 x 6 blocks (against the block-owned pairs it is ahead everywhere).
+      // k_stage36 keeps a column's point operands in shared memory for the whole column and adds a block to its tile
+      // once, so it is ahead where columns are long and there are enough of them; k_runs, whose items are parts of
+      // columns, is ahead on short or few columns and, in FP32, on long ones of few blocks. us, k_stage36 / k_runs, FP32 and FP64: 1000 cameras of 1200 visits and 61 blocks 320 / 250 and 401 /
+      // 461; 10,000 of 766 and 121 1553 / 1760; 3000 of 766 and 121 483 / 590 and 933 / 1165; 300 of 583 and 57 44 / 51
+      // and 79 / 86; 200 of 345 and 31 34 / 28 and 38 / 40; 1500 of 200 and 121 127 / 87 and 160 / 150; 3000 of 200 and
+      // 41 303 / 131 and 325 / 219; 40 of 1100 and 40 54 / 25 and 48 / 34.
+      int64_t cols = 0;
+      for (int64_t r = 0; r < nrb; ++r) cols += rptr[r + 1] > rptr[r];
+      const double visits = cols ? (double)nc / cols : 0.0, blocks = (double)nb / nrb;
+      P->runs_first[0] = !(visits >= 512 && cols >= 148 && (blocks >= 90 || visits < 900));
+      P->runs_first[1] = !(visits >= 300 && cols >= 148);
+    }
+    // a plan of 6 x 6 blocks for a sparse S builds per storage type the schedule that "stage" takes (the other one when it
+    // cannot be built, or when it is chosen by name: ensure_gather, ensure_runs); every other plan has the runs only
+    for (int sd = 0; sd < 2; ++sd) {
+      auto runs = [&] {
+        return contiguous && (sd == 0 ? build_run_schedule<float>(P->runs[0], in, run_exact, P->max_dr, P->max_de, s)
+                                      : build_run_schedule<double>(P->runs[1], in, run_exact, P->max_dr, P->max_de, s));
+      };
+      auto stage = [&] {
+        return P->stage_ok[sd] = build_stage_schedule(P.get(), sd, s, nrb, rptr, rentry, entry_elim, d->eliminated_ptr, d->entry_retained,
+                                                      bcolptr, browval, brow_off, col_h);
+      };
+      if (!gather) runs();
+      else if (P->runs_first[sd]) { if (!runs()) stage(); }
+      else if (!stage()) runs();
+    }
   }
   // staged work items for the host-buffer reduction: stage j holds points [stage_pt[j], stage_pt[j + 1]); a block's
   // pairs ascend in point within its slot, so its pairs of one stage are a contiguous run, cut into items of at most
@@ -2309,10 +2363,8 @@ static SchurPlan* plan_create(bls_ctx* ctx, const bls_schur_plan_desc* d) {
   if (!P->fast36) P->Einv32.alloc(sizeof(float) * std::max<int64_t>(P->E_length, 1));
   P->z.alloc(sizeof(double) * std::max<int64_t>(ne, 1));
   if (P->fast36) P->Einv12.alloc(sizeof(double) * 12 * neb);   // sized for FP64; the FP32 form uses half
-  if (P->stage_ok) {
-    P->EZ.alloc(sizeof(double) * 12 * neb);
-    P->kernel = 5;   // the column-owned schedule is the default where it applies
-  }
+  if (P->stage_ok[0] || P->stage_ok[1] || P->runs[0].ok || P->runs[1].ok) P->kernel = 5;   // column-owned: the default
+  if (P->points3) P->EZ.alloc(sizeof(double) * 12 * neb);
   P->status.alloc(sizeof(Status));
   Status init{NONE, NONE, NONE, 0};
   BLS_CUDA(cudaMemcpyAsync(P->status.p, &init, sizeof(Status), cudaMemcpyHostToDevice, s));
@@ -2329,6 +2381,7 @@ static int64_t plan_bytes(const SchurPlan* P) {
                           &P->Einv64, &P->Einv32, &P->z, &P->status};
   int64_t b = 0;
   for (auto* x : bufs) b += (int64_t)x->bytes;
+  for (const RunSchedule& r : P->runs) b += r.bytes();
   return b;
 }
 
@@ -2345,6 +2398,7 @@ static int read_status(SchurPlan* P, int64_t* failed_block) {
     if (failed_block) *failed_block = 0;
     return BLS_EINVAL;
   }
+  if (st.failed == kCopyFault) throw Error(BLS_ECUDA, "a bulk copy of the reduction did not complete within its wait limit");
   if (st.failed != NONE) {
     if (failed_block) *failed_block = st.failed + 1;
     return BLS_NOT_PD;
@@ -2474,6 +2528,135 @@ static void ensure_points(SchurPlan* P) {
   P->points_ok = true;
 }
 
+// k_runs / k_runs_any on the plan's schedule of this storage type: the kernel of the plan's sizes, and as many persistent
+// CTAs as fit the SMs
+template <class T>
+static void launch_runs(SchurPlan* P, T* S, bool dense, double* g, const T* C, const double* s_r, const double* s_e, const int32_t* poc,
+                        const long long* pf) {
+  constexpr bool F32 = sizeof(T) == 4;
+  RunSchedule& R = P->runs[F32 ? 0 : 1];
+  void (*kern)(RunArgs<T>) = nullptr;
+  switch (R.exact) {
+    case 6: kern = k_runs<T, 6, 6>; break;
+    case 7: kern = k_runs<T, 7, 7>; break;
+    case 8: kern = k_runs<T, 8, F32 ? 8 : 4>; break;
+    case 9: kern = k_runs<T, 9, F32 ? 9 : 3>; break;
+    default: kern = R.mdr <= 9 ? k_runs_any<T, 9, F32 ? 9 : 5> : k_runs_any<T, 16, F32 ? 8 : 4>;
+  }
+  BLS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, R.smem));
+  if (R.grid == 0) {
+    int per_sm = 0, nsm = 0, dev = 0;
+    BLS_CUDA(cudaGetDevice(&dev));
+    BLS_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+    BLS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kRunThreads, R.smem));
+    R.grid = std::max(1, per_sm) * nsm;
+  }
+  RunArgs<T> a;
+  a.items = R.items_d.as<int4>();
+  a.segs = R.segs.as<int4>();
+  a.blob = R.blob.as<uint4>();
+  a.nitems = R.items;
+  a.Clen = P->C_length;
+  a.dense_nr = P->nr;
+  a.block_base = dense ? P->block_base_dense.as<int64_t>() : P->block_base_sparse.as<int64_t>();
+  a.block_stride = dense ? nullptr : P->block_stride_sparse.as<int32_t>();
+  a.block_r1 = P->block_r1.as<int32_t>();
+  a.boffsets_r = P->boffsets_r.as<int32_t>();
+  a.C = C;
+  a.EZ = P->EZ.as<double>();
+  a.Einv = P->Einv64.as<double>();
+  a.z = P->z.as<double>();
+  a.s_r = s_r;
+  a.s_e = s_e;
+  a.r_dims = P->r_dims.as<int32_t>();
+  a.e_dims = P->e_dims.as<int32_t>();
+  a.eoffsets = P->eoffsets.as<int32_t>();
+  a.boffsets_e = P->boffsets_e.as<int32_t>();
+  a.S = S;
+  a.g = g;
+  a.st = P->status.as<Status>();
+  a.prob_of_cam = poc;
+  a.prob_fail = pf;
+  a.queue = reinterpret_cast<unsigned long long*>(&P->status.as<Status>()->pad);
+  a.tile_bytes = R.tile_bytes;
+  a.blob_bytes = R.blob_bytes;
+  a.wr = R.wr;
+  a.ts = R.ts;
+  a.mdr = R.mdr;
+  a.mde = R.mde;
+  kern<<<(unsigned)std::min<int64_t>(R.items, R.grid), kRunThreads, R.smem, P->ctx->stream>>>(a);
+}
+
+// A 6/3 plan's layout, read back from its device copies (for a schedule that is built after plan creation). Synchronises.
+struct PlanLayout {
+  std::vector<int32_t> rptr, rentry, entry_elim;
+  std::vector<int64_t> eptr, eret, bcolptr, browval, brow_off, col_h;
+};
+static PlanLayout download_layout(SchurPlan* P) {
+  cudaStream_t s = P->ctx->stream;
+  const int64_t nrb = P->nrblocks, neb = P->neblocks, nc = P->ncoup, nb = P->nblocks;
+  auto down32 = [&](const DevBuf& b, int64_t n) {
+    std::vector<int32_t> v((size_t)n);
+    if (n) BLS_CUDA(cudaMemcpyAsync(v.data(), b.p, (size_t)n * sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+    return v;
+  };
+  PlanLayout L;
+  L.rptr = down32(P->retained_ptr, nrb + 1);
+  L.rentry = down32(P->retained_entry, nc);
+  L.entry_elim = down32(P->entry_eliminated, nc);
+  const std::vector<int32_t> ep32 = down32(P->eliminated_ptr, neb + 1), er32 = down32(P->entry_retained, nc), ch = down32(P->col_h, nrb);
+  const std::vector<int32_t> b_r1 = down32(P->block_r1, nb), b_r2 = down32(P->block_r2, nb);
+  std::vector<int64_t> b_base((size_t)nb), cbase((size_t)nrb);
+  if (nb) BLS_CUDA(cudaMemcpyAsync(b_base.data(), P->block_base_sparse.p, (size_t)nb * sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+  BLS_CUDA(cudaMemcpyAsync(cbase.data(), P->col_base.p, (size_t)nrb * sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+  BLS_CUDA(cudaStreamSynchronize(s));
+  L.eptr.assign(ep32.begin(), ep32.end());
+  L.eret.assign(er32.begin(), er32.end());
+  L.col_h.assign(ch.begin(), ch.end());
+  L.bcolptr.assign(nrb + 1, 0);
+  L.browval.resize(nb);
+  L.brow_off.resize(nb);
+  for (int64_t k = 0; k < nb; ++k) {
+    L.bcolptr[b_r2[k] + 1] += 1;
+    L.browval[k] = b_r1[k];
+    L.brow_off[k] = b_base[k] - cbase[b_r2[k]];
+  }
+  for (int64_t r = 0; r < nrb; ++r) L.bcolptr[r + 1] += L.bcolptr[r];
+  return L;
+}
+static bool build_gather(SchurPlan* P, const PlanLayout& L, int sd) {
+  return build_stage_schedule(P, sd, P->ctx->stream, P->nrblocks, L.rptr, L.rentry, L.entry_elim, L.eptr.data(), L.eret.data(), L.bcolptr,
+                              L.browval, L.brow_off, L.col_h);
+}
+// The schedules of a 6/3 plan for a sparse S that its "stage" choice does not use, built when they are chosen by name
+static void ensure_gather(SchurPlan* P) {
+  if (!P->fast36 || !P->has_sparse || (P->stage_ok[0] && P->stage_ok[1])) return;
+  const PlanLayout L = download_layout(P);
+  for (int sd = 0; sd < 2; ++sd)
+    if (!P->stage_ok[sd]) P->stage_ok[sd] = build_gather(P, L, sd);
+}
+static void ensure_runs(SchurPlan* P) {
+  if (!P->fast36 || !P->has_sparse || (P->runs[0].ok && P->runs[1].ok)) return;
+  const PlanLayout L = download_layout(P);
+  const std::vector<int64_t> rd(P->nrblocks, 6), ed(P->neblocks, 3);
+  std::vector<int64_t> co(P->ncoup);
+  for (int64_t c = 0; c < P->ncoup; ++c) co[c] = 18 * c;
+  const RunInput in{P->nrblocks, P->neblocks, P->C_length, rd.data(), ed.data(), L.eptr.data(), L.eret.data(), co.data(), &L.rptr, &L.rentry,
+                    &L.entry_elim, &L.bcolptr, &L.browval};
+  if (!P->runs[0].ok) build_run_schedule<float>(P->runs[0], in, 6, 6, 3, P->ctx->stream);
+  if (!P->runs[1].ok) build_run_schedule<double>(P->runs[1], in, 6, 6, 3, P->ctx->stream);
+}
+
+// Whether the plan's choice of kernel is k_runs / k_runs_any (where its schedule exists): always for block sizes other
+// than 6 and 3 (the alternative there, k_pairs, is a thread per work item: 1510 us against 264 on 803 cameras of nine
+// variables); "runs", and "stage" where the plan prefers it or S is dense.
+static bool runs_chosen(const SchurPlan* P, int sd, bool dense) {
+  if (!P->fast36) return true;
+  if (P->kernel == 6) return true;
+  const bool stage = P->kernel == 5 || (P->nprob > 0 && !dense && P->kernel != 1 && P->kernel != 7);
+  return stage && (dense || !P->stage_ok[sd] || P->runs_first[sd]);
+}
+
 template <class T>
 static int reduce(SchurPlan* P, T* S, bool dense, double* g, const double* b_r, const double* b_e, const double* sc_e, double lambda,
                   const T* E, const T* C, const double* s_r, const double* s_e, int64_t* failed_block) {
@@ -2487,21 +2670,25 @@ static int reduce(SchurPlan* P, T* S, bool dense, double* g, const double* b_r, 
   const bool c16 = (reinterpret_cast<uintptr_t>(C) & 31) == 0;   // 32-byte loads of C
   const bool batch = P->nprob > 0 && !dense;
   // a batch runs the column-owned schedule unless the block-owned pair lists are chosen (both keep per-problem failure)
-  const bool use_stage = P->fast36 && (P->kernel == 5 || (batch && P->kernel != 1)) && !dense && P->stage_ok && c16 &&
+  const RunSchedule& RS = P->runs[sizeof(T) == 4 ? 0 : 1];
+  const bool c_runs = RS.ok && (reinterpret_cast<uintptr_t>(C) & 15) == 0;   // k_runs copies C in 16-byte chunks
+  const bool use_runs = c_runs && runs_chosen(P, sizeof(T) == 4 ? 0 : 1, dense);
+  const bool use_stage = P->fast36 && !use_runs && (P->kernel >= 5 || (batch && P->kernel != 1)) && !dense && P->stage_ok[sizeof(T) == 4 ? 0 : 1] && c16 &&
                          (!s_r || P->S_rowval.p);
+  const bool record = use_stage || (use_runs && RS.exact);   // the kernel reads E' and z' from the factor kernel's record
   const int32_t* poc = batch ? P->prob_of_cam.as<int32_t>() : nullptr;
   long long* pf = batch ? P->prob_fail.as<long long>() : nullptr;
   if (batch) {
     k_prob_arm<<<grid_for(P->nprob, 256), 256, 0, s>>>(pf, P->nprob);
     P->launches += 1;
   }
-  if (P->fast36) {
+  if (P->fast36 || (use_runs && RS.exact)) {
     using TE = typename EinvOf<T>::type;
     k_arm36<<<1, 1, 0, s>>>(st);
     if (P->neblocks > 0)
       k_factor36<T><<<grid_for(P->neblocks, 128), 128, 0, s>>>(0, P->neblocks, E, b_e, sc_e, lambda, s_e, P->Einv64.as<double>(),
-                                                             use_stage ? nullptr : P->Einv12.as<TE>(), P->z.as<double>(),
-                                                             use_stage ? P->EZ.as<double>() : nullptr,
+                                                             record || use_runs ? nullptr : P->Einv12.as<TE>(), P->z.as<double>(),
+                                                             record ? P->EZ.as<double>() : nullptr,
                                                              batch ? P->prob_of_point.as<int32_t>() : nullptr, pf, st);
   } else {
     begin_checked(P, sc_e, P->ne, 1);
@@ -2517,7 +2704,13 @@ static int reduce(SchurPlan* P, T* S, bool dense, double* g, const double* b_r, 
     BLS_CUDA(cudaEventCreate(&ev0));
     BLS_CUDA(cudaEventCreate(&ev1));
   }
-  if (use_stage) {
+  if (use_runs) {
+    k_g_init<<<grid_for(P->nr, 256), 256, 0, s>>>(g, b_r, s_r, P->nr, st, poc, pf);
+    P->launches += 2;
+    if (ev0) BLS_CUDA(cudaEventRecord(ev0, s));
+    launch_runs<T>(P, S, dense, g, C, s_r, s_e, poc, pf);
+    if (ev1) BLS_CUDA(cudaEventRecord(ev1, s));
+  } else if (use_stage) {
     k_g_init<<<grid_for(P->nr, 256), 256, 0, s>>>(g, b_r, s_r, P->nr, st, poc, pf);
     P->launches += 1;
     const SchurPlan::StageSchedule& SS = P->stage[sizeof(T) == 4 ? 0 : 1];
@@ -3024,56 +3217,36 @@ int bls_reduce_schur_dense(bls_schur_plan* P, int dtype, void* S, double* g, con
 }
 
 int bls_schur_plan_set_kernel(bls_schur_plan* P, int which) {
-  if (!P || which < 0 || which > 5) return BLS_EINVAL;
+  if (!P || which < 0 || which > 7) return BLS_EINVAL;
   BLS_GUARD({
     if (which == 4) ensure_points(P);
+    if (which == 6) ensure_runs(P);
+    if (which == 7) ensure_gather(P);
     P->kernel = which;
     return BLS_OK;
   })
 }
 
-// Rebuild the column-owned schedule with units of at most `unit` pairs, from the plan's device copies of the structure
-// (the schedule is a plan-time product; this is the autotuner's knob). On failure the previous schedule stays.
+// The unit size of the "gather" schedules: the ones that are built are built again (the schedule is a plan-time product;
+// this is the autotuner's knob), the others take it when they are. On failure the previous schedule stays.
 int bls_schur_plan_set_stage_unit(bls_schur_plan* P, int unit) {
   if (!P || unit < 1 || unit > 4096) return BLS_EINVAL;
   BLS_GUARD({
-    if (!P->fast36 || !P->has_sparse || !P->stage_ok) throw Error(BLS_EUNSUPPORTED, "the plan has no column-owned schedule");
+    if (!P->fast36 || !P->has_sparse || !(P->stage_ok[0] || P->stage_ok[1] || P->runs[0].ok || P->runs[1].ok))
+      throw Error(BLS_EUNSUPPORTED, "the plan has no column-owned schedule");
     if (unit == P->stage_unit[0] && unit == P->stage_unit[1]) return BLS_OK;
-    cudaStream_t s = P->ctx->stream;
-    const int64_t nrb = P->nrblocks, neb = P->neblocks, nc = P->ncoup;
-    const int64_t nb = P->nblocks;
-    auto down32 = [&](const DevBuf& b, int64_t n) {
-      std::vector<int32_t> v((size_t)n);
-      if (n) BLS_CUDA(cudaMemcpyAsync(v.data(), b.p, (size_t)n * sizeof(int32_t), cudaMemcpyDeviceToHost, s));
-      return v;
-    };
-    std::vector<int32_t> rptr = down32(P->retained_ptr, nrb + 1), rentry = down32(P->retained_entry, nc);
-    std::vector<int32_t> entry_elim = down32(P->entry_eliminated, nc), ep32 = down32(P->eliminated_ptr, neb + 1);
-    std::vector<int32_t> er32 = down32(P->entry_retained, nc), b_r1 = down32(P->block_r1, nb), b_r2 = down32(P->block_r2, nb);
-    std::vector<int32_t> ch = down32(P->col_h, nrb);
-    std::vector<int64_t> b_base((size_t)nb), cbase((size_t)nrb);
-    if (nb) BLS_CUDA(cudaMemcpyAsync(b_base.data(), P->block_base_sparse.p, (size_t)nb * sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-    BLS_CUDA(cudaMemcpyAsync(cbase.data(), P->col_base.p, (size_t)nrb * sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-    BLS_CUDA(cudaStreamSynchronize(s));
-    std::vector<int64_t> eptr(ep32.begin(), ep32.end()), eret(er32.begin(), er32.end());
-    std::vector<int64_t> bcolptr(nrb + 1, 0), browval(nb), brow_off(nb), col_h(ch.begin(), ch.end());
-    for (int64_t k = 0; k < nb; ++k) {
-      bcolptr[b_r2[k] + 1] += 1;
-      browval[k] = b_r1[k];
-      brow_off[k] = b_base[k] - cbase[b_r2[k]];
-    }
-    for (int64_t r = 0; r < nrb; ++r) bcolptr[r + 1] += bcolptr[r];
     const int old0 = P->stage_unit[0], old1 = P->stage_unit[1];
     P->stage_unit[0] = P->stage_unit[1] = unit;
-    // each schedule is replaced only when its rebuild succeeds (a schedule with the old unit size stays valid)
-    bool ok = true;
-    for (int sd = 0; sd < 2; ++sd)
-      ok = build_stage_schedule(P, sd, s, nrb, rptr, rentry, entry_elim, eptr.data(), eret.data(), bcolptr, browval, brow_off,
-                                col_h) && ok;
-    if (!ok) {
-      P->stage_unit[0] = old0;
-      P->stage_unit[1] = old1;
-      throw Error(BLS_EUNSUPPORTED, "the schedule does not fit this unit size");
+    if (P->stage_ok[0] || P->stage_ok[1]) {
+      const PlanLayout L = download_layout(P);
+      bool ok = true;
+      for (int sd = 0; sd < 2; ++sd)
+        if (P->stage_ok[sd]) ok = build_gather(P, L, sd) && ok;
+      if (!ok) {
+        P->stage_unit[0] = old0;
+        P->stage_unit[1] = old1;
+        throw Error(BLS_EUNSUPPORTED, "the schedule does not fit this unit size");
+      }
     }
     P->stage_grid[0] = P->stage_grid[1] = 0;
     return BLS_OK;
@@ -3085,7 +3258,9 @@ int bls_schur_plan_phase2_kernel(bls_schur_plan* P, int dtype, int dense, int sc
   if (!P || !buf || cap < 1 || (dtype != BLS_F64 && dtype != BLS_F32)) return BLS_EINVAL;
   const std::string t = dtype == BLS_F32 ? "<float>" : "<double>";
   std::string name;
-  if (P->fast36 && (P->kernel == 5 || (P->nprob > 0 && P->kernel != 1)) && !dense && P->stage_ok) name = "k_stage36" + t;
+  const RunSchedule& R = P->runs[dtype == BLS_F32 ? 0 : 1];
+  if (R.ok && runs_chosen(P, dtype == BLS_F32 ? 0 : 1, dense != 0)) name = (R.exact ? "k_runs" : "k_runs_any") + t;
+  else if (P->fast36 && (P->kernel >= 5 || (P->nprob > 0 && P->kernel != 1)) && !dense && P->stage_ok[dtype == BLS_F32 ? 0 : 1]) name = "k_stage36" + t;
   else if (P->fast36 && P->nprob > 0 && !dense) name = "k_pairs36" + t;
   else if (P->fast36 && P->kernel == 0) name = std::string("k_columns36") + t;
   else if (P->fast36 && P->kernel == 3 && !dense && !scaled && P->tiles_ok) name = "k_tiles36" + t;

@@ -114,17 +114,18 @@ class SchurReductionWorkspace:
         return int(_lib.gpu().bls_schur_plan_device_bytes(self._h))
 
     def set_kernel(self, which: str) -> None:
-        """Phase-2 kernel of the 6/3 fast path: "stage" (block-column owned: the column's point-side operands staged in
-        shared memory, a thread per 6 x 6 block accumulating in registers; the default for a sparse S), "pairs" (block
-        owned, six lanes per pair list; the default for a dense S), "lanes" (block owned, a lane per pair, a warp per
+        """Phase-2 kernel of the 6/3 fast path: "stage" (block-column owned, the default: one of the next two, by a rule
+        on the plan's sizes), "runs" (the couplings of a column's points staged in shared memory segment by segment),
+        "gather" (sparse S; the column's point-side operands staged, the other couplings gathered per pair; a thread
+        per 6 x 6 block accumulating in registers in both), "pairs" (block owned, six lanes per pair list), "lanes" (block owned, a lane per pair, a warp per
         pair list), "columns" (block-column owned, a warp per visit), "tiles" (block-column owned, visits staged in
         chunks; sparse S without conditioning scales, else "pairs") or "points" (point-major, six lanes per pair,
         vector reductions into S)."""
         check(_lib.gpu().bls_schur_plan_set_kernel(self._h, {"columns": 0, "pairs": 1, "lanes": 2, "tiles": 3, "points": 4,
-                                                             "stage": 5}[which]))
+                                                             "stage": 5, "runs": 6, "gather": 7}[which]))
 
     def set_stage_unit(self, unit: int) -> None:
-        """Rebuild the "stage" schedule of both storage types with units of at most `unit` pairs (one thread's run of
+        """Rebuild the "gather" schedule of both storage types with units of at most `unit` pairs (one thread's run of
         one S block's pairs between two writes to the column tile); 20 for FP32 storage and 16 for FP64 at plan
         creation."""
         check(_lib.gpu().bls_schur_plan_set_stage_unit(self._h, int(unit)))
