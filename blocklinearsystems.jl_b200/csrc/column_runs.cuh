@@ -54,14 +54,6 @@ __host__ __device__ inline int run_chunks(int x, int y, int64_t Clen) {
   return whole < n ? (int)whole : n;
 }
 
-__device__ __forceinline__ void run_cp16(void* smem, const void* gmem, int bytes) {
-  const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gmem), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void run_cp_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void run_cp_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
-
 // Copies a segment's record into shared memory.
 __device__ __forceinline__ void run_blob(uint4* dst, const uint4* __restrict__ blob, const int4& seg) {
   for (int i = threadIdx.x; i < seg.y; i += kRunThreads) run_cp16(dst + i, blob + seg.x + i, 16);

@@ -30,6 +30,17 @@ struct Status {
 template <class T>
 __device__ __forceinline__ T ldg(const T* p) { return __ldg(p); }
 
+#ifdef __CUDACC__
+// An asynchronous 16-byte global -> shared copy of `bytes` bytes (the rest zero-filled), both on 16-byte boundaries
+__device__ __forceinline__ void run_cp16(void* smem, const void* gmem, int bytes) {
+  const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gmem), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void run_cp_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void run_cp_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
+#endif
+
 inline int grid_for(int64_t n, int threads) { return (int)((n + threads - 1) / threads); }
 
 // A device buffer that frees itself.
