@@ -1,12 +1,13 @@
 // Dense Cholesky factorisation and solve of the reduced system on sm_100a: the reduced solve that follows
 // reduce_schur_dense! when S is small enough to hold dense (the reference hands its dense S to DampedLinearSolve's
 // Cholesky, src/schur_linear_systems.jl:312-320). S is read from its upper triangle in its storage type (FP64 or the
-// mixed form's FP32), mirrored into an FP64 working matrix owned by the solver, and factored in place as S = L L' by a
-// right-looking blocked Cholesky with 64-column panels: per panel, one launch factors the diagonal tile (in every
-// CTA's shared memory) and solves the rows below it, then the trailing lower triangle is updated in 64 x 64 tiles. A
-// pivot that is not positive (or not finite) stops the factorisation; its column is reported, 1-based. The solve runs
-// the two triangular substitutions as one launch per 64-row tile: all CTAs apply the last solved tile to the rows it
-// feeds, and CTA 0, whose rows are the next diagonal tile, then solves that tile.
+// mixed form's FP32) into the lower triangle of an FP64 working matrix owned by the solver, padded to whole 64 x 64
+// tiles with an identity, and factored in place as S = L L' by a blocked Cholesky: panels of 64 columns in groups of
+// four. One CTA factors the diagonal tiles one after the other; beside it, the rows below a tile are solved against it and
+// the panel updates the group's remaining columns and the next group's first one (rank 64), and a finished group updates everything right of
+// those (rank 256) beside the next panels. A pivot that is not positive (or
+// not finite) stops the factorisation; its column is reported, 1-based. The solve is one cooperative kernel: a CTA owns
+// tiles of 64 rows, the tiles' solutions pass from owner to all others through memory.
 #include <algorithm>
 #include <cmath>
 #include <memory>
@@ -15,61 +16,77 @@
 
 namespace bls {
 
-constexpr int NB = 64;   // panel width and tile size
-constexpr int kFusedPanelTiles = 32;   // panels with at most this many 64-row tiles below run as one launch
+constexpr int NB = 64;      // panel width and tile size
+constexpr int GROUP = 4;    // panels per group
+constexpr int TS = NB + 2;  // row stride of a tile in shared memory (16-byte rows)
 
 struct DenseSolver {
   bls_ctx* ctx = nullptr;
-  int64_t n = 0;
-  DevBuf W;        // n x n FP64, column-major; L in its lower triangle after a successful factorisation
-  DevBuf dinv;     // n FP64: 1 / L[j, j], written by the factorisation
+  int64_t n = 0, ld = 0;   // ld: n rounded up to whole tiles, the order and leading dimension of W
+  DevBuf W;        // ld x ld FP64, column-major; L in its lower triangle after a successful factorisation
+  DevBuf rows;     // the 64 rows below the next diagonal tile, two buffers
+  DevBuf inv16;    // per panel the inverses of its diagonal tile's four 16 x 16 diagonal blocks (column-major)
+  DevBuf inv;      // per panel the inverse of its 64 x 64 diagonal tile (column-major), for the solve
   DevBuf status;   // [0]: first failing column (0-based) or -1
   bool factored = false;
-  // The next panel's diagonal tile and triangular solve run on a high-priority stream while the rest of the trailing
-  // update runs on the caller's stream (created at the first factorisation).
+  // The diagonal tiles run on one high-priority stream, the panels below them and the updates they wait for on another,
+  // while the rest of a group's update runs on the caller's stream (created at the first factorisation).
   cudaStream_t panel_stream = nullptr;
-  cudaEvent_t ev_join = nullptr, ev_panel = nullptr;
+  cudaStream_t update_stream = nullptr;
+  cudaEvent_t ev_join = nullptr, ev_panel = nullptr, ev_next = nullptr, ev_tile = nullptr, ev_update = nullptr;
   int panel_priority = 0;
   // Everything after the load of S (the launches depend on n only) as one CUDA graph, captured at the first
   // factorisation; the panel kernels carry the high priority as a launch attribute, so the graph keeps it.
-  cudaGraphExec_t factor_graph = nullptr;
-  // The solve's launches (two per 64-row tile) as one CUDA graph on the solver's own right-hand side y, captured at
-  // the first solve: g is copied into y, the graph replayed, y copied out to x.
-  DevBuf y;
   cudaStream_t cap_stream = nullptr;
-  cudaGraphExec_t solve_graph = nullptr;
+  cudaGraphExec_t factor_graph = nullptr;
+  DevBuf y;               // the solve's exchange: ld forward and ld backward values, all bits set until written
+  int solve_grid = 0;     // resident CTAs of k_solve (set at the first solve)
   ~DenseSolver() {
-    if (solve_graph) cudaGraphExecDestroy(solve_graph);
     if (factor_graph) cudaGraphExecDestroy(factor_graph);
     if (cap_stream) cudaStreamDestroy(cap_stream);
     if (ev_join) cudaEventDestroy(ev_join);
     if (ev_panel) cudaEventDestroy(ev_panel);
+    for (cudaEvent_t e : {ev_next, ev_tile, ev_update})
+      if (e) cudaEventDestroy(e);
+    if (update_stream) cudaStreamDestroy(update_stream);
     if (panel_stream) cudaStreamDestroy(panel_stream);
   }
 };
 
-// W = S mirrored from its upper triangle, in FP64, plus lambda s_r[j] on the diagonal when s_r is given
+// The lower triangle of W = S' (S's upper triangle), in FP64, plus lambda s_r[j] on the diagonal when s_r is given, and
+// the identity in the padding; a CTA per 32 x 32 tile on or below the diagonal, turned in shared memory so that both
+// sides are read and written in contiguous runs.
 template <class T>
-__global__ void k_dense_load(int64_t n, const T* __restrict__ S, double* __restrict__ W, double lambda, const double* __restrict__ s_r,
-                             long long* __restrict__ status) {
-  if (blockIdx.x == 0 && threadIdx.x == 0) status[0] = -1;
-  for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < n * n; q += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t i = q % n, j = q / n;
-    double v = (double)(i <= j ? S[i + n * j] : S[j + n * i]);
-    if (s_r && i == j) v += lambda * s_r[j];
-    W[q] = v;
+__global__ void __launch_bounds__(256) k_dense_load(int64_t n, int64_t ld, const T* __restrict__ S, double* __restrict__ W, double lambda,
+                                                    const double* __restrict__ s_r, long long* __restrict__ status) {
+  __shared__ double t[32][33];
+  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) status[0] = -1;
+  if (blockIdx.y > blockIdx.x) return;
+  const int64_t i0 = 32 * (int64_t)blockIdx.x, j0 = 32 * (int64_t)blockIdx.y;   // rows i0.., columns j0.. of W
+  const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
+#pragma unroll
+  for (int k = 0; k < 32; k += 8) {
+    const int64_t j = j0 + x, i = i0 + y + k;
+    t[y + k][x] = j <= i && i < n ? (double)S[j + n * i] : i == j ? 1.0 : 0.0;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < 32; k += 8) {
+    const int64_t i = i0 + x, j = j0 + y + k;
+    double v = t[x][y + k];
+    if (s_r && i == j && i < n) v += lambda * s_r[j];
+    W[i + ld * j] = v;
   }
 }
 
-// The lower triangle of the diagonal tile [d0, d0 + dnb) of L into t by 256 threads, all 16 loads of a thread in flight
-// (zeros elsewhere)
-__device__ __forceinline__ void load_tile(double (*t)[NB + 1], const double* __restrict__ W, int64_t n, int64_t d0, int dnb,
-                                          int tid) {
+// The lower triangle of the diagonal tile [d0, d0 + 64) of W into t by 256 threads, all 16 loads of a thread in flight
+// (zeros above the diagonal)
+__device__ __forceinline__ void load_tile(double (*t)[TS], const double* __restrict__ W, int64_t ld, int64_t d0, int tid) {
   double v[NB * NB / 256];
 #pragma unroll
   for (int k = 0; k < NB * NB / 256; ++k) {
     const int e = tid + 256 * k, rr = e & 63, cc = e >> 6;
-    v[k] = (rr < dnb && cc <= rr) ? W[(d0 + rr) + n * (d0 + cc)] : 0.0;
+    v[k] = cc <= rr ? W[(d0 + rr) + ld * (d0 + cc)] : 0.0;
   }
 #pragma unroll
   for (int k = 0; k < NB * NB / 256; ++k) {
@@ -78,493 +95,497 @@ __device__ __forceinline__ void load_tile(double (*t)[NB + 1], const double* __r
   }
 }
 
-// An asynchronous 8-byte global -> shared copy (cp.async); `bytes` 0 writes a zero and reads nothing.
-__device__ __forceinline__ void cp_async8(double* smem, const double* gmem, int bytes) {
+// An asynchronous 8-byte global -> shared copy (cp.async).
+__device__ __forceinline__ void cp_async8(double* smem, const double* gmem) {
   const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(s), "l"(gmem), "r"(bytes) : "memory");
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gmem) : "memory");
 }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
-// The diagonal tile T (lower triangle of its first nb rows and columns, in shared memory) factored in place by
-// 256 threads, by 16-column sub-panels: warp 0 factors a sub-panel's rows (lane i holds rows c0 + i and c0 + 32 + i
-// of its 16 columns in registers) with no barrier: per column the pivot comes from its lane by shuffle,
-// L[j, j] = pivot * rsqrt(pivot), and each later column's entry of L is shuffled from its lane to update the rows
-// below; then all threads subtract the sub-panel's rank-16 product from the rest of the tile. 1 / L[j, j] goes to dv.
-// Returns (to every thread) the first column whose pivot is not positive or not finite, or -1.
-__device__ int factor_tile(double (*T)[NB + 1], double* dv, int nb, int* failed) {
-  const int tid = threadIdx.x, lane = tid & 31;
-  for (int c0 = 0; c0 < nb; c0 += 16) {
-    const int w = nb - c0 < 16 ? nb - c0 : 16;
-    if (tid < 32) {
-      const int r0 = c0 + lane, r1 = c0 + 32 + lane;
-      double a0[16], a1[16];
+// The diagonal tile T (lower triangle, in shared memory) factored in place by 256 threads, by 16-column sub-panels: warps 0
+// and 1 factor a sub-panel's rows (lane i holds row c0 + i, in warp 1 row c0 + 32 + i, of its 16 columns in registers): per
+// column warp 0 forms L[j, j] = pivot * rsqrt(pivot) and the entries below it, which go to T, and both warps update their
+// rows with them, read back as broadcasts; the next pivot is row j + 1's own, so the chain of a column is rsqrt, a product,
+// the exchange through shared memory and one multiply-add. The test of a pivot is off it: a bad one only makes what follows
+// useless. (One warp holding two rows a lane and shuffling the 15 entries of a column: a 64-bit shuffle takes 11 cycles of
+// issue and an FP64 multiply-add 5, 430 cycles a column.) Then all warps subtract the sub-panel's rank-16
+// product from the rest of the tile (3 x 3 entries a thread, or 2 x 2, or one) after which the last inverts the sub-panel's 16 x
+// 16 diagonal block into V (column-major; a lane per column). Returns (to every thread) the first column whose pivot is not
+// positive or not finite, or -1.
+template <int NA>
+__device__ __forceinline__ void rank16(double (*T)[TS], int c0, int tid) {   // rows and columns c0 + 16 .. c0 + 16 + 16 NA
+  const int tx = tid & 15, ty = tid >> 4, base = c0 + 16;
+  double acc[NA][NA];
 #pragma unroll
-      for (int k = 0; k < 16; ++k) {
-        a0[k] = r0 < NB ? T[r0][c0 + k] : 0.0;
-        a1[k] = r1 < NB ? T[r1][c0 + k] : 0.0;
-      }
+  for (int a = 0; a < NA; ++a)
+#pragma unroll
+    for (int b = 0; b < NA; ++b) acc[a][b] = 0.0;
+#pragma unroll
+  for (int c = 0; c < 16; c += 2) {
+    double2 x[NA], y[NA];
+#pragma unroll
+    for (int a = 0; a < NA; ++a) {
+      x[a] = *reinterpret_cast<const double2*>(&T[base + tx + 16 * a][c0 + c]);
+      y[a] = *reinterpret_cast<const double2*>(&T[base + ty + 16 * a][c0 + c]);
+    }
+#pragma unroll
+    for (int a = 0; a < NA; ++a)
+#pragma unroll
+      for (int b = 0; b <= a; ++b) acc[a][b] = fma(x[a].y, y[b].y, fma(x[a].x, y[b].x, acc[a][b]));
+  }
+#pragma unroll
+  for (int a = 0; a < NA; ++a)
+#pragma unroll
+    for (int b = 0; b <= a; ++b)
+      if (a > b || ty <= tx) T[base + tx + 16 * a][base + ty + 16 * b] -= acc[a][b];
+}
+
+__device__ int factor_tile(double (*T)[TS], double* dv, double (*V)[16][16], int* failed) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  for (int c0 = 0; c0 < NB; c0 += 16) {
+    if (warp < 2) {
+      const int r = c0 + 32 * warp + lane;
+      const bool own = r < NB;
+      double a[16];
+#pragma unroll
+      for (int k = 0; k < 16; ++k) a[k] = own ? T[r][c0 + k] : 0.0;
       int bad = -1;
+      double d = __shfl_sync(0xffffffffu, a[0], 0);   // warp 0: the pivot
 #pragma unroll
       for (int j = 0; j < 16; ++j) {
-        if (j < w && bad < 0) {   // uniform (no break, so the loop unrolls and a0, a1 stay in registers)
-          const double d = __shfl_sync(0xffffffffu, a0[j], j);
-          if (!(d > 0.0) || !isfinite(d)) {   // uniform
-            bad = c0 + j;
-          } else {
-            const double inv = rsqrt(d);
-            const double l0 = (lane == j ? d : a0[j]) * inv, l1 = a1[j] * inv;
-            if (lane >= j) a0[j] = l0;
-            a1[j] = l1;
-            if (lane == j) dv[c0 + j] = inv;
-#pragma unroll
-            for (int k = j + 1; k < 16; ++k) {
-              const double lk = __shfl_sync(0xffffffffu, l0, k);
-              if (lane >= k) a0[k] -= l0 * lk;
-              a1[k] -= l1 * lk;
-            }
-          }
+        double l = 0.0;
+        if (warp == 0) {
+          if (bad < 0 && (!(d > 0.0) || !isfinite(d))) bad = c0 + j;   // uniform
+          const double inv = rsqrt(d);
+          l = a[j] * inv;
+          if (own && lane >= j) T[r][c0 + j] = l;
+          if (lane == j) dv[c0 + j] = inv;
+          if (j < 15) d = __shfl_sync(0xffffffffu, fma(-l, l, a[j + 1 < 16 ? j + 1 : 15]), j + 1);
         }
-      }
+        asm volatile("bar.sync 1, 64;" ::: "memory");   // column j is in T for both warps
+        if (warp == 1) {
+          l = a[j] * dv[c0 + j];
+          if (own) T[r][c0 + j] = l;
+        }
 #pragma unroll
-      for (int k = 0; k < 16; ++k) {
-        if (r0 < NB && k <= lane) T[r0][c0 + k] = a0[k];
-        if (r1 < NB) T[r1][c0 + k] = a1[k];
+        for (int k = j + 1; k < 16; ++k) a[k] = fma(-l, T[c0 + k][c0 + j], a[k]);
       }
-      if (lane == 0) *failed = bad;
+      if (tid == 0) *failed = bad;
     }
     __syncthreads();
     if (*failed >= 0) return *failed;   // uniform
-    // the rest of the tile's lower triangle: T[i, k] -= sum over the sub-panel's columns of L[i, c] L[k, c]
-    const int base = c0 + 16, m = nb > base ? nb - base : 0;
-    for (int e = tid; e < m * m; e += 256) {
-      const int i = base + e / m, k = base + e % m;
-      if (k > i) continue;
-      double s0 = 0.0, s1 = 0.0;
+    if (c0 == 0) rank16<3>(T, 0, tid);
+    else if (c0 == 16) rank16<2>(T, 16, tid);
+    else if (c0 == 32) rank16<1>(T, 32, tid);
+    if (warp == 7 && lane < 16) {   // column `lane` of the inverse: v[i] = s[i] / L[i, i], then s[k] -= L[k, i] v[i] below it
+      double v[16];
 #pragma unroll
-      for (int c = 0; c < 16; c += 2) {
-        s0 = fma(T[i][c0 + c], T[k][c0 + c], s0);
-        s1 = fma(T[i][c0 + c + 1], T[k][c0 + c + 1], s1);
+      for (int i = 0; i < 16; ++i) v[i] = i == lane ? 1.0 : 0.0;
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        v[i] *= dv[c0 + i];
+#pragma unroll
+        for (int k = i + 1; k < 16; ++k) v[k] = fma(-T[c0 + k][c0 + i], v[i], v[k]);
       }
-      T[i][k] -= s0 + s1;
+#pragma unroll
+      for (int i = 0; i < 16; ++i) V[c0 / 16][lane][i] = v[i];
     }
-    __syncthreads();
+    // the next sub-panel's warps wait for the product only; the inverses are done by the barrier at the end
+    if (c0 + 16 < NB) __syncthreads();
   }
+  __syncthreads();
   return -1;
 }
 
-// One row of the panel below the tile solved against L_kk' (x L_kk' = a): x holds the row's 64 entries; L[c2, c] is
-// read from the factored tile as a broadcast.
-__device__ __forceinline__ void solve_row(double (&x)[NB], const double (*T)[NB + 1], const double* dv) {
+// The 64 rows of X solved against the factored tile (X L' = A), by 256 threads in four steps of 16 columns: a thread
+// holds 4 columns of one row, subtracts the products of the columns already solved, and the 16 x 16 diagonal block is
+// applied through its inverse. X[c][r] in place; Z is scratch. (A thread per row with its 64 entries in registers, fully
+// unrolled, was bound by fetching its 64 KB of instructions: 25 us a panel.)
+__device__ __forceinline__ void solve_rows(double (*X)[NB], double (*Z)[NB], const double (*T)[TS], const double (*V)[16][16], int tid) {
+  const int r = tid & 63, q = 4 * (tid >> 6);
+  for (int b = 0; b < NB; b += 16) {
+    double acc[4];
 #pragma unroll
-  for (int c = 0; c < NB; ++c) {
-    x[c] *= dv[c];
+    for (int j = 0; j < 4; ++j) acc[j] = X[b + q + j][r];
+#pragma unroll 4
+    for (int k = 0; k < b; k += 2) {
+      const double x0 = X[k][r], x1 = X[k + 1][r];
 #pragma unroll
-    for (int c2 = c + 1; c2 < NB; ++c2) x[c2] -= x[c] * T[c2][c];
+      for (int j = 0; j < 4; ++j) {
+        const double2 l = *reinterpret_cast<const double2*>(&T[b + q + j][k]);
+        acc[j] = fma(-x1, l.y, fma(-x0, l.x, acc[j]));
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) Z[q + j][r] = acc[j];
+    __syncthreads();
+    double out[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll 4
+    for (int k = 0; k < q + 4; ++k) {   // the inverse is lower triangular: column q + j takes k <= q + j
+      const double z = Z[k][r];
+#pragma unroll
+      for (int j = 0; j < 4; j += 2) {
+        const double2 v = *reinterpret_cast<const double2*>(&V[b / 16][k][q + j]);
+        out[j] = fma(z, v.x, out[j]);
+        out[j + 1] = fma(z, v.y, out[j + 1]);
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) X[b + q + j][r] = out[j];
+    __syncthreads();
   }
 }
 
-// The diagonal tile [k0, k0 + nb) alone, in one CTA (followed by k_trsm_panel when many rows lie below it). A
-// non-positive or non-finite pivot records its column and W is not written. 1 / L[j, j] goes to dinv.
-__global__ void __launch_bounds__(256, 1) k_potrf_tile(int64_t n, double* __restrict__ W, double* __restrict__ dinv, int64_t k0,
-                                                       int nb, long long* __restrict__ status) {
-  __shared__ double T[NB][NB + 1];
-  __shared__ double dv[NB];
-  __shared__ int failed;
-  if (status[0] >= 0) return;   // uniform across the CTA
-  const int tid = threadIdx.x;
-  load_tile(T, W, n, k0, nb, tid);
-  if (tid == 0) failed = -1;
-  __syncthreads();
-  const int bad = factor_tile(T, dv, nb, &failed);
-  if (bad >= 0) {
-    if (tid == 0) status[0] = k0 + bad;
-    return;
-  }
+// shared memory of the panel kernels: the diagonal tile, the 16 x 16 inverses, 1 / L[j, j], the CTA's 64 panel rows and
+// their scratch
+struct PanelSmem {
+  double T[NB][TS];
+  double V[NB / 16][16][16];
+  double dv[NB];
+  double X[NB][NB];   // X[column][row]
+  double Z[16][NB];
+};
+
+// The CTA's 64 x 64 inverse: the identity solved against the tile (X L' = I, so X[i][j] = inverse[i][j]), for the solve.
+__device__ __forceinline__ void tile_inverse(PanelSmem& s, double* __restrict__ inv, int64_t k0, int tid) {
 #pragma unroll
   for (int k = 0; k < NB * NB / 256; ++k) {
-    const int e = tid + 256 * k, rr = e & 63, cc = e >> 6;
-    if (rr < nb && cc <= rr) W[(k0 + rr) + n * (k0 + cc)] = T[rr][cc];
+    const int e = tid + 256 * k;
+    s.X[e >> 6][e & 63] = (e >> 6) == (e & 63) ? 1.0 : 0.0;
   }
-  if (tid < nb) dinv[k0 + tid] = dv[tid];
-}
-
-// The panel below the diagonal tile factored by k_potrf_tile: rows [k0 + NB, n) of columns [k0, k0 + NB), a thread
-// per row with its 64 entries in registers, the tile in shared memory.
-__global__ void __launch_bounds__(NB) k_trsm_panel(int64_t n, double* __restrict__ W, const double* __restrict__ dinv_g,
-                                                   int64_t k0, const long long* __restrict__ status) {
-  __shared__ double T[NB][NB + 1];
-  __shared__ double dv[NB];
-  if (status[0] >= 0) return;
-  const int t = threadIdx.x;
-  const int64_t r = k0 + NB + (int64_t)blockIdx.x * NB + t;
-  // the row's 64 entries and the tile (16 columns at a time), every load of a batch in flight
-  double x[NB];
-#pragma unroll
-  for (int c = 0; c < NB; ++c) x[c] = r < n ? W[r + n * (k0 + c)] : 0.0;
-#pragma unroll
-  for (int c0 = 0; c0 < NB; c0 += 16) {
-    double v[16];
-#pragma unroll
-    for (int c = 0; c < 16; ++c) v[c] = W[(k0 + t) + n * (k0 + c0 + c)];
-#pragma unroll
-    for (int c = 0; c < 16; ++c) T[t][c0 + c] = v[c];
-  }
-  dv[t] = dinv_g[k0 + t];
   __syncthreads();
-  if (r >= n) return;
-  solve_row(x, T, dv);
-#pragma unroll
-  for (int c = 0; c < NB; ++c) W[r + n * (k0 + c)] = x[c];
-}
-
-// shared memory of k_panel: the diagonal tile, the CTA's 64 panel rows, 1 / L[j, j]
-constexpr int PANEL_SMEM = (2 * NB * (NB + 1) + NB) * (int)sizeof(double);
-
-// One panel [k0, k0 + nb) in one launch of max(1, ceil(rows below / 64)) CTAs of 256 threads, for panels with few
-// rows below: every CTA factors the diagonal tile in its own shared memory (the same operations on the same values,
-// so every copy is identical; CTA 0 writes it and 1 / L[j, j] back) while its 64 rows below the tile arrive by
-// cp.async, then a thread per row solves it. A non-positive or non-finite pivot is seen by every CTA: CTA 0 records
-// its column and nothing is written.
-__global__ void __launch_bounds__(256, 1) k_panel(int64_t n, double* __restrict__ W, double* __restrict__ dinv, int64_t k0,
-                                                  int nb, long long* __restrict__ status) {
-  extern __shared__ __align__(16) double panel_smem[];
-  double (*T)[NB + 1] = reinterpret_cast<double (*)[NB + 1]>(panel_smem);
-  double (*X)[NB + 1] = reinterpret_cast<double (*)[NB + 1]>(panel_smem + NB * (NB + 1));
-  double* dv = panel_smem + 2 * NB * (NB + 1);
-  __shared__ int failed;
-  if (status[0] >= 0) return;   // uniform across the grid
-  const int tid = threadIdx.x;
-  const int64_t row0 = k0 + nb + (int64_t)blockIdx.x * NB;   // this CTA's rows below the tile
+  solve_rows(s.X, s.Z, s.T, s.V, tid);
 #pragma unroll
   for (int k = 0; k < NB * NB / 256; ++k) {
-    const int e = tid + 256 * k, r = e & 63, c = e >> 6;
-    const bool v = row0 + r < n;
-    cp_async8(&X[r][c], v ? W + (row0 + r) + n * (k0 + c) : W, v ? 8 : 0);
+    const int e = tid + 256 * k, i = e & 63, j = e >> 6;
+    inv[NB * k0 + i + NB * j] = s.X[i][j];
   }
-  cp_async_commit();
-  load_tile(T, W, n, k0, nb, tid);
-  if (tid == 0) failed = -1;
-  __syncthreads();
-  const int bad = factor_tile(T, dv, nb, &failed);
-  if (bad >= 0) {
-    cp_async_wait<0>();
-    if (blockIdx.x == 0 && tid == 0) status[0] = k0 + bad;
-    return;
-  }
-  if (blockIdx.x == 0) {
+}
+
+// The diagonal tiles, one CTA after the other: the chain that every panel waits for. For panel k (k0 = 64 k) it solves the
+// 64 rows below the diagonal tile (a copy of them, `rows`: k_trsm_panel solves the same rows in W meanwhile), subtracts
+// their rank-64 product from the next diagonal tile and factors that; `first`: it factors tile 0. A non-positive or
+// non-finite pivot records its column and nothing is written. Bound by the latency of its 64 columns, one after another
+// (14 us a tile; 17 to 21 before, with the rows' 10 us and the update's 9 us as launches of their own between the tiles):
+// a factorisation takes 30 us a panel where the updates do not bound it (n = 1000: 0.535 -> 0.484 ms), 40 before.
+struct StepSmem {
+  PanelSmem p;
+  double next[NB][TS];
+};
+__global__ void __launch_bounds__(256, 1) k_step(int64_t ld, double* __restrict__ W, const double* __restrict__ rows, double* __restrict__ inv16,
+                                                 int64_t k0, int first, long long* __restrict__ status) {
+  extern __shared__ __align__(16) unsigned char dense_smem[];
+  StepSmem& s = *reinterpret_cast<StepSmem*>(dense_smem);
+  __shared__ int failed;
+  if (status[0] >= 0) return;   // uniform
+  const int tid = threadIdx.x;
+  const int64_t d0 = first ? k0 : k0 + NB;   // the tile to factor
+  if (!first) {
 #pragma unroll
     for (int k = 0; k < NB * NB / 256; ++k) {
-      const int e = tid + 256 * k, rr = e & 63, cc = e >> 6;
-      if (rr < nb && cc <= rr) W[(k0 + rr) + n * (k0 + cc)] = T[rr][cc];
+      const int e = tid + 256 * k, r = e & 63, c = e >> 6;
+      cp_async8(&s.p.X[c][r], rows + e);
+      cp_async8(&s.p.T[r][c], W + (k0 + r) + ld * (k0 + c));   // entries above the diagonal are not used
     }
-    if (tid < nb) dinv[k0 + tid] = dv[tid];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) cp_async8(&s.p.V[0][0][0] + tid + 256 * k, inv16 + k0 * 16 + tid + 256 * k);
   }
-  cp_async_wait<0>();
+  run_cp_commit();
+  load_tile(s.next, W, ld, d0, tid);
+  if (tid == 0) failed = -1;
+  run_cp_wait<0>();
   __syncthreads();
-  const int64_t r = row0 + tid;
-  if (tid >= NB || r >= n) return;   // rows below the tile exist only when nb == NB
-  double x[NB];
+  if (!first) {
+    solve_rows(s.p.X, s.p.Z, s.p.T, s.p.V, tid);
+    // next -= X X', 4 x 4 entries a thread: rows 2 tx + {0, 1, 32, 33}, columns 2 ty + {0, 1, 32, 33}
+    const int tx = tid & 15, ty = tid >> 4;
+    double acc[4][4];
 #pragma unroll
-  for (int c = 0; c < NB; ++c) x[c] = X[tid][c];
-  solve_row(x, T, dv);
+    for (int p = 0; p < 4; ++p)
 #pragma unroll
-  for (int c = 0; c < NB; ++c) W[r + n * (k0 + c)] = x[c];
-}
-
-constexpr int SYRK_KC = 16, SYRK_STAGES = 3;
-constexpr int SYRK_SMEM = SYRK_STAGES * 2 * SYRK_KC * NB * (int)sizeof(double);   // a ring of 16-column chunks of both panels
-
-// The trailing lower triangle: W[i, j] -= sum_c L[i, c] L[j, c] over the panel's 64 columns, for i >= j >= k0 + NB,
-// in two launches: `rest` == 0 the first tile column (the next panel), `rest` == 1 the tile columns after it.
-// One CTA of 256 threads per 64 x 64 output tile of the lower triangle (tiles listed by their index in it). The two
-// row panels pass through a three-stage ring of 16-column chunks in shared memory, copied asynchronously (cp.async,
-// rows past n zero-filled) two chunks ahead of the products (48 KB and at most 64 registers a thread, so four CTAs fit
-// an SM), and the output tile is fetched the same way into the two free stages during the last chunk. Each thread
-// accumulates a 4 x 4 block (rows 2 tx + {0, 1, 32, 33}, columns 2 ty + {0, 1, 32, 33}) from 16-byte shared loads with
-// FP64 fused multiply-adds (the FP64 tensor-core form, mma.sync m8n8k4 fragments per warp, measured 1.3x slower here).
-__global__ void __launch_bounds__(256, 4) k_syrk_tiles(int64_t n, double* __restrict__ W, int64_t k0, int rest,
-                                                       const long long* __restrict__ status) {
-  constexpr int KC = SYRK_KC, NCH = NB / KC;
-  extern __shared__ __align__(16) double syrk_smem[];
-  auto Pi = [&](int stage) { return reinterpret_cast<double (*)[NB]>(syrk_smem + stage * 2 * KC * NB); };
-  auto Pj = [&](int stage) { return reinterpret_cast<double (*)[NB]>(syrk_smem + stage * 2 * KC * NB + KC * NB); };
-  if (status[0] >= 0) return;
-  const int64_t t = blockIdx.x;
-  int64_t ti = t, tj = 0;
-  if (rest) {
-    ti = (int64_t)((sqrt(8.0 * (double)t + 1.0) - 1.0) * 0.5);
-    while ((ti + 1) * (ti + 2) / 2 <= t) ++ti;
-    while (ti * (ti + 1) / 2 > t) --ti;
-    tj = t - ti * (ti + 1) / 2 + 1;
-    ti += 1;
-  }
-  const int64_t bi = k0 + NB + ti * NB, bj = k0 + NB + tj * NB;
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  auto issue = [&](int ch) {
-    double (*A)[NB] = Pi(ch % SYRK_STAGES);
-    double (*B)[NB] = Pj(ch % SYRK_STAGES);
-#pragma unroll
-    for (int k = 0; k < KC * NB / 256; ++k) {
-      const int e = tid + 256 * k, c = e >> 6, r = e & 63;
-      const int64_t col = n * (k0 + KC * ch + c);
-      const bool vi = bi + r < n, vj = bj + r < n;
-      cp_async8(&A[c][r], vi ? W + bi + r + col : W, vi ? 8 : 0);
-      cp_async8(&B[c][r], vj ? W + bj + r + col : W, vj ? 8 : 0);
-    }
-    cp_async_commit();
-  };
-  issue(0);
-  issue(1);
-  double acc[4][4];
-#pragma unroll
-  for (int p = 0; p < 4; ++p)
-#pragma unroll
-    for (int q = 0; q < 4; ++q) acc[p][q] = 0.0;
-  static_assert(NCH == 4 && SYRK_STAGES == 3, "the output tile is prefetched into stages 1 and 2 during the last chunk");
-  double (*O)[NB] = reinterpret_cast<double (*)[NB]>(syrk_smem + 2 * KC * NB);   // stages 1 and 2: 64 x 64, O[col][row]
-  for (int ch = 0; ch < NCH; ++ch) {
-    if (ch + 2 < NCH) issue(ch + 2);   // into the stage chunk ch - 1 used: every thread passed the barrier after it
-    else cp_async_commit();           // an empty group keeps the count of groups in flight uniform
-    cp_async_wait<2>();
-    __syncthreads();
-    if (ch == NCH - 1) {
-      // stages 1 and 2 are free (chunks 1 and 2 are done): fetch the output tile for the read-modify-write while the
-      // last chunk's products run
-#pragma unroll
-      for (int k = 0; k < NB * NB / 256; ++k) {
-        const int e = tid + 256 * k, col = e >> 6, row = e & 63;
-        const bool v = bi + row < n && bj + col < n;
-        cp_async8(&O[col][row], v ? W + (bi + row) + n * (bj + col) : W, v ? 8 : 0);
-      }
-      cp_async_commit();
-    }
-    double (*A)[NB] = Pi(ch % SYRK_STAGES);
-    double (*B)[NB] = Pj(ch % SYRK_STAGES);
+      for (int q = 0; q < 4; ++q) acc[p][q] = 0.0;
 #pragma unroll 4
-    for (int c = 0; c < KC; ++c) {
-      const double2 a0 = *reinterpret_cast<const double2*>(&A[c][2 * tx]);
-      const double2 a1 = *reinterpret_cast<const double2*>(&A[c][32 + 2 * tx]);
-      const double2 b0 = *reinterpret_cast<const double2*>(&B[c][2 * ty]);
-      const double2 b1 = *reinterpret_cast<const double2*>(&B[c][32 + 2 * ty]);
+    for (int c = 0; c < NB; ++c) {
+      const double2 a0 = *reinterpret_cast<const double2*>(&s.p.X[c][2 * tx]), a1 = *reinterpret_cast<const double2*>(&s.p.X[c][32 + 2 * tx]);
+      const double2 b0 = *reinterpret_cast<const double2*>(&s.p.X[c][2 * ty]), b1 = *reinterpret_cast<const double2*>(&s.p.X[c][32 + 2 * ty]);
       const double ra[4] = {a0.x, a0.y, a1.x, a1.y}, rb[4] = {b0.x, b0.y, b1.x, b1.y};
 #pragma unroll
       for (int p = 0; p < 4; ++p)
 #pragma unroll
         for (int q = 0; q < 4; ++q) acc[p][q] = fma(ra[p], rb[q], acc[p][q]);
     }
+#pragma unroll
+    for (int p = 0; p < 4; ++p)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int i = 2 * tx + (p & 1) + 32 * (p >> 1), j = 2 * ty + (q & 1) + 32 * (q >> 1);
+        if (j <= i) s.next[i][j] -= acc[p][q];
+      }
     __syncthreads();
   }
-  cp_async_wait<0>();
-  __syncthreads();
-#pragma unroll
-  for (int p = 0; p < 4; ++p)
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int ri = 2 * tx + (p & 1) + 32 * (p >> 1), cj = 2 * ty + (q & 1) + 32 * (q >> 1);
-      const int64_t oi = bi + ri, oj = bj + cj;
-      if (oi < n && oj <= oi) W[oi + n * oj] = O[cj][ri] - acc[p][q];
-    }
-}
-
-// The diagonal tile [d0, d0 + dnb) of L into t for one warp's substitution, by 256 threads (all 16 loads of a thread
-// in flight), pre-scaled so that a column step is one shuffle and one fused multiply-add: forward (rows_scaled = 0),
-// t[r][c] = L[r][c] / L[c][c] for r > c; backward (rows_scaled = 1), t[r][c] = L[r][c] / L[r][r] for r > c; zero on and
-// above the diagonal and outside the tile.
-__device__ __forceinline__ void load_scaled_tile(double (*t)[NB + 1], const double* __restrict__ W, const double* __restrict__ dinv,
-                                                 int64_t n, int64_t d0, int dnb, int rows_scaled, int tid) {
-  double v[NB * NB / 256];
+  const int bad = factor_tile(s.next, s.p.dv, s.p.V, &failed);
+  if (bad >= 0) {
+    if (tid == 0) status[0] = d0 + bad;
+    return;
+  }
 #pragma unroll
   for (int k = 0; k < NB * NB / 256; ++k) {
     const int e = tid + 256 * k, rr = e & 63, cc = e >> 6;
-    v[k] = (rr < dnb && cc < rr) ? W[(d0 + rr) + n * (d0 + cc)] * dinv[d0 + (rows_scaled ? rr : cc)] : 0.0;
+    if (cc <= rr) W[(d0 + rr) + ld * (d0 + cc)] = s.next[rr][cc];
   }
+#pragma unroll
+  for (int k = 0; k < 4; ++k) inv16[d0 * 16 + tid + 256 * k] = (&s.p.V[0][0][0])[tid + 256 * k];
+}
+
+// Copies the 64 rows below tile 0 for the first k_step.
+__global__ void __launch_bounds__(256) k_first_rows(int64_t ld, const double* __restrict__ W, double* __restrict__ rows) {
 #pragma unroll
   for (int k = 0; k < NB * NB / 256; ++k) {
-    const int e = tid + 256 * k;
-    t[e & 63][e >> 6] = v[k];
+    const int e = threadIdx.x + 256 * k;
+    rows[e] = W[(NB + (e & 63)) + ld * (e >> 6)];
   }
 }
 
-// The forward substitution of one diagonal tile [d0, d0 + dnb) by one warp, t from load_scaled_tile (forward): lanes
-// own rows lane and lane + 32 and start from ys (shared); per column the finished row value is shuffled from its lane
-// and every lane subtracts its scaled entry times it, so the column chain is a shuffle and a fused multiply-add; the
-// rows are multiplied by 1 / L[r][r] (dlo, dhi) once at the end and written to y.
-__device__ __forceinline__ void tile_forward(const double (*t)[NB + 1], double dlo, double dhi, const double* ys,
-                                             double* __restrict__ y, int64_t d0, int dnb, int lane) {
-  double y0 = ys[lane], y1 = ys[lane + 32];
-#pragma unroll 8
-  for (int c = 0; c < 32; ++c) {
-    const double yc = __shfl_sync(0xffffffffu, y0, c);
-    y0 = fma(-t[lane][c], yc, y0);
-    y1 = fma(-t[lane + 32][c], yc, y1);
-  }
-#pragma unroll 8
-  for (int c = 32; c < NB; ++c) {
-    const double yc = __shfl_sync(0xffffffffu, y1, c - 32);
-    y1 = fma(-t[lane + 32][c], yc, y1);
-  }
-  if (lane < dnb) y[d0 + lane] = y0 * dlo;
-  if (lane + 32 < dnb) y[d0 + 32 + lane] = y1 * dhi;
-}
-
-// The backward substitution (L' x = y) of one diagonal tile [d0, d0 + dnb), t from load_scaled_tile (backward), as
-// tile_forward from the last column to the first.
-__device__ __forceinline__ void tile_backward(const double (*t)[NB + 1], double dlo, double dhi, const double* ys,
-                                              double* __restrict__ y, int64_t d0, int dnb, int lane) {
-  double y0 = ys[lane], y1 = ys[lane + 32];
-#pragma unroll 8
-  for (int c = NB - 1; c >= 32; --c) {
-    const double yc = __shfl_sync(0xffffffffu, y1, c - 32);
-    y1 = fma(-t[c][lane + 32], yc, y1);
-    y0 = fma(-t[c][lane], yc, y0);
-  }
-#pragma unroll 8
-  for (int c = 31; c >= 0; --c) {
-    const double yc = __shfl_sync(0xffffffffu, y0, c);
-    y0 = fma(-t[c][lane], yc, y0);
-  }
-  if (lane < dnb) y[d0 + lane] = y0 * dlo;
-  if (lane + 32 < dnb) y[d0 + 32 + lane] = y1 * dhi;
-}
-
-// One forward step of L y = g, y in place: rows [d0, n) take the update from the solved tile [d0 - NB, d0) (when
-// `update`), CTA b the 64 rows from d0 + 64 b, four threads per row over 16 columns each; then CTA 0, whose rows are
-// the next diagonal tile [d0, d0 + dnb), solves it. Every global load of the step is issued before the first barrier,
-// and CTA 0 keeps its updated rows in shared memory, so the step costs one round trip to memory plus the tile's chain.
-__global__ void __launch_bounds__(256) k_fwd_step(int64_t n, const double* __restrict__ W, const double* __restrict__ dinv,
-                                                  double* __restrict__ y, int64_t d0, int dnb, int update) {
-  __shared__ double t[NB][NB + 1];
-  __shared__ double yk[NB];
-  __shared__ double part[4][NB];
-  __shared__ double ys[NB];
-  const int tid = threadIdx.x, r = tid & 63, q = tid >> 6;
-  const int64_t i = d0 + (int64_t)blockIdx.x * NB + r, k0 = d0 - NB;
-  double w[16];
-  double yi = 0.0, dlo = 0.0, dhi = 0.0;
-  if (update) {
-    if (i < n) {
+// The panel below the diagonal tile factored by k_step: a CTA per 64 rows, and one for the tile's inverse.
+__global__ void __launch_bounds__(256) k_trsm_panel(int64_t ld, double* __restrict__ W, const double* __restrict__ inv16,
+                                                    double* __restrict__ inv, int64_t k0, const long long* __restrict__ status) {
+  extern __shared__ __align__(16) unsigned char dense_smem[];
+  PanelSmem& s = *reinterpret_cast<PanelSmem*>(dense_smem);
+  if (status[0] >= 0) return;
+  const int tid = threadIdx.x;
+  const bool rows = blockIdx.x + 1 < gridDim.x;
+  const int64_t row0 = k0 + NB + (int64_t)blockIdx.x * NB;
 #pragma unroll
-      for (int c = 0; c < 16; ++c) w[c] = W[i + n * (k0 + 16 * q + c)];
-    }
-    if (tid < NB) yk[tid] = y[k0 + tid];
+  for (int k = 0; k < NB * NB / 256; ++k) {
+    const int e = tid + 256 * k, r = e & 63, c = e >> 6;
+    if (rows) cp_async8(&s.X[c][r], W + (row0 + r) + ld * (k0 + c));
+    cp_async8(&s.T[r][c], W + (k0 + r) + ld * (k0 + c));   // entries above the diagonal are not used
   }
-  if (q == 0 && i < n) yi = y[i];
-  if (blockIdx.x == 0) {
-    load_scaled_tile(t, W, dinv, n, d0, dnb, 0, tid);
-    if (tid < 32) {
-      if (tid < dnb) dlo = dinv[d0 + tid];
-      if (tid + 32 < dnb) dhi = dinv[d0 + 32 + tid];
-    }
-  }
+#pragma unroll
+  for (int k = 0; k < 4; ++k) cp_async8(&s.V[0][0][0] + tid + 256 * k, inv16 + k0 * 16 + tid + 256 * k);
+  run_cp_commit();
+  run_cp_wait<0>();
   __syncthreads();
-  if (update) {
-    double s = 0.0;
-    if (i < n) {
+  if (!rows) {
+    tile_inverse(s, inv, k0, tid);
+    return;
+  }
+  solve_rows(s.X, s.Z, s.T, s.V, tid);
 #pragma unroll
-      for (int c = 0; c < 16; ++c) s = fma(w[c], yk[16 * q + c], s);
+  for (int k = 0; k < NB * NB / 256; ++k) {
+    const int e = tid + 256 * k, r = e & 63, c = e >> 6;
+    W[(row0 + r) + ld * (k0 + c)] = s.X[c][r];
+  }
+}
+
+// W[i, j] -= sum over c in [k0, k0 + K) of L[i, c] L[j, c] for the lower triangle of the tile columns
+// [j0 + 64 blockIdx.y, + 64) of W: CTAs of 256 threads over tiles of MT x 64 (MT = 128: 8 x 4 entries a thread, MT = 64:
+// 4 x 4), those above the diagonal leave at once. The two row panels pass through a ring of three 16-column chunks in
+// shared memory (16-byte cp.async, two chunks ahead of the products). With 4 x 4 entries a thread a warp needs 6
+// shared-memory wavefronts per 32 cycles of FP64 multiply-adds, 24 of every 32 for the SM's four, with 8 x 4 half of that;
+// rank 256 reads and writes the output a quarter as often as rank 64 (n = 6000: 5.9 ms of updates before, 4.3 now, 20 TFLOP/s in the 128-row form).
+// The panels wait for the rank-64 updates on their stream: those (AHEAD) have all four chunks and the output tile in
+// flight at once, so that such a launch costs one round trip to memory.
+template <int MT, bool AHEAD>
+__host__ __device__ constexpr int syrk_smem() { return (AHEAD ? 4 : 3) * 16 * (MT + NB) * (int)sizeof(double); }
+template <int MT, bool AHEAD>
+__global__ void __launch_bounds__(256, AHEAD ? 3 : MT == 128 ? 2 : 4) k_syrk(int64_t ld, double* __restrict__ W, int64_t k0, int K, int64_t j0, double* __restrict__ rows,
+                                                                 const long long* __restrict__ status) {
+  constexpr int KC = 16, RM = MT / 16, ST = AHEAD ? 4 : 3;   // RM: rows a thread holds
+  extern __shared__ __align__(16) unsigned char dense_smem[];
+  double* ring = reinterpret_cast<double*>(dense_smem);
+  if (status[0] >= 0) return;
+  const int64_t bj = j0 + NB * (int64_t)blockIdx.y, bi = j0 + MT * (int64_t)blockIdx.x;
+  if (bi + MT <= bj) return;   // above the diagonal
+  if (AHEAD && blockIdx.x == 0 && blockIdx.y == 0) return;   // the next diagonal tile is k_step's
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  const int nch = K / KC;
+  auto A = [&](int ch) { return reinterpret_cast<double (*)[MT]>(ring + (ch % ST) * KC * (MT + NB)); };
+  auto B = [&](int ch) { return reinterpret_cast<double (*)[NB]>(ring + (ch % ST) * KC * (MT + NB) + KC * MT); };
+  auto issue = [&](int ch) {
+    if (ch < nch) {
+      const double* src = W + ld * (k0 + KC * ch);
+      auto a = A(ch);
+      auto b = B(ch);
+#pragma unroll
+      for (int k = 0; k < KC * MT / 512; ++k) {
+        const int e = tid + 256 * k, c = e / (MT / 2), r = 2 * (e % (MT / 2));
+        const bool in = MT == NB || bi + r < ld;   // the last 128-row tile may hang over W's end
+        run_cp16(&a[c][r], in ? src + ld * c + bi + r : src, in ? 16 : 0);
+      }
+#pragma unroll
+      for (int k = 0; k < KC * NB / 512; ++k) {
+        const int e = tid + 256 * k, c = e / (NB / 2), r = 2 * (e % (NB / 2));
+        run_cp16(&b[c][r], src + ld * c + bj + r, 16);
+      }
     }
+    run_cp_commit();   // an empty group keeps the count of groups in flight uniform
+  };
+  // rows bi + 2 tx + 32 (p / 2) + (p & 1), columns bj + 2 ty + 32 (q / 2) + (q & 1) are this thread's
+  auto out_row = [&](int p) { return bi + 2 * tx + 32 * (p >> 1) + (p & 1); };
+  auto out_col = [&](int q) { return bj + 2 * ty + 32 * (q >> 1) + (q & 1); };
+  auto is_out = [&](int p, int q) { return out_row(p) < ld && out_col(q) <= out_row(p); };
+#pragma unroll
+  for (int ch = 0; ch < ST - 1; ++ch) issue(ch);
+  double acc[RM][4];
+#pragma unroll
+  for (int p = 0; p < RM; ++p)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) acc[p][q] = 0.0;
+  double out[AHEAD ? RM : 1][4];
+  if constexpr (AHEAD) {
+    issue(ST - 1);
+#pragma unroll
+    for (int p = 0; p < RM; ++p)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) out[p][q] = is_out(p, q) ? W[out_row(p) + ld * out_col(q)] : 0.0;
+  }
+  for (int ch = 0; ch < nch; ++ch) {
+    run_cp_wait<ST - 2 + (AHEAD ? 1 : 0)>();
+    __syncthreads();   // chunk ch is in for every thread, and chunk ch - 1 has been used
+    if (AHEAD) run_cp_commit();   // nch is ST: nothing left to issue
+    else issue(ch + ST - 1);      // into the stage of chunk ch - 1
+    auto a = A(ch);
+    auto b = B(ch);
+#pragma unroll 4
+    for (int c = 0; c < KC; ++c) {
+      double ra[RM], rb[4];
+#pragma unroll
+      for (int p = 0; p < RM; p += 2) {
+        const double2 v = *reinterpret_cast<const double2*>(&a[c][2 * tx + 16 * p]);
+        ra[p] = v.x;
+        ra[p + 1] = v.y;
+      }
+#pragma unroll
+      for (int q = 0; q < 4; q += 2) {
+        const double2 v = *reinterpret_cast<const double2*>(&b[c][2 * ty + 16 * q]);
+        rb[q] = v.x;
+        rb[q + 1] = v.y;
+      }
+#pragma unroll
+      for (int p = 0; p < RM; ++p)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) acc[p][q] = fma(ra[p], rb[q], acc[p][q]);
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    double old[RM];
+#pragma unroll
+    for (int p = 0; p < RM; ++p) old[p] = AHEAD ? out[AHEAD ? p : 0][q] : is_out(p, q) ? W[out_row(p) + ld * out_col(q)] : 0.0;
+#pragma unroll
+    for (int p = 0; p < RM; ++p)
+      if (is_out(p, q)) {
+        W[out_row(p) + ld * out_col(q)] = old[p] - acc[p][q];
+        // the rows below the next diagonal tile, finished here, also for k_step
+        if (AHEAD && blockIdx.x == 1 && blockIdx.y == 0) rows[(out_row(p) - bi) + NB * (out_col(q) - bj)] = old[p] - acc[p][q];
+      }
+  }
+}
+
+// L L' x = g in one cooperative launch, CTA b owning the 64 rows of tile b. Forward: it takes y_k of every earlier tile in
+// order (polling it: each value is 8 bytes, all bits set until it is written), subtracts L[b, k] y_k from its rows, then
+// multiplies them by the inverse of its diagonal tile and posts y_b. Backward the same from the last tile up with L'. A
+// tile's 64 x 64 block of L is loaded before its poll. A poll that gives up passes NaNs on (nothing waits for ever).
+// n = 6000: 1.8 ms as two launches per tile with a substitution by one warp in each, 0.29 ms now.
+constexpr unsigned long long kUnwritten = ~0ull;
+__device__ __forceinline__ double poll_value(const double* p) {
+  unsigned long long v = kUnwritten;
+  for (int i = 0; i < (1 << 22); ++i) {
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    if (v != kUnwritten) break;
+  }
+  return v == kUnwritten ? __longlong_as_double(0x7ff8000000000000ll) : __longlong_as_double((long long)v);
+}
+__device__ __forceinline__ void post_value(double* p, double v) {
+  unsigned long long b = (unsigned long long)__double_as_longlong(v);
+  if (b == kUnwritten) b = 0x7ff8000000000000ull;   // a NaN of another payload
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(b) : "memory");
+}
+
+__global__ void __launch_bounds__(256) k_solve(int64_t n, int64_t ld, const double* __restrict__ W, const double* __restrict__ inv,
+                                               const double* g, double* x, double* y) {
+  __shared__ double rt[NB];   // the tile's current right-hand side
+  __shared__ double xk[NB];
+  __shared__ double part[4][NB];
+  const int tid = threadIdx.x, r = tid & 63, q = tid >> 6, lane = tid & 31, warp = tid >> 5;
+  const int nt = (int)(ld / NB), b = blockIdx.x;
+  const int64_t row0 = NB * (int64_t)b;
+  double* yf = y;
+  double* yb = y + ld;
+  if (tid < NB) rt[tid] = row0 + tid < n ? g[row0 + tid] : 0.0;
+  double w[16];   // a 64 x 64 block: row r, columns 16 q ..
+  auto load = [&](const double* M, int64_t stride) {
+#pragma unroll
+    for (int c = 0; c < 16; ++c) w[c] = M[r + stride * (16 * q + c)];
+  };
+  auto mul = [&](const double* xs) {   // (M xs)[r], in every thread
+    double s = 0.0;
+#pragma unroll
+    for (int c = 0; c < 16; ++c) s = fma(w[c], xs[16 * q + c], s);
     part[q][r] = s;
     __syncthreads();
-    if (q == 0) yi -= (part[0][r] + part[1][r]) + (part[2][r] + part[3][r]);
+    return (part[0][r] + part[1][r]) + (part[2][r] + part[3][r]);
+  };
+  for (int k = 0; k < b; ++k) {
+    load(W + row0 + ld * NB * (int64_t)k, ld);
+    if (tid < NB) xk[tid] = poll_value(yf + NB * (int64_t)k + tid);
+    __syncthreads();
+    const double v = mul(xk);
+    if (q == 0) rt[r] -= v;
+    // the next xk and part are written after the barrier that every thread passes once it has read these: mul's own
+    // barrier orders xk, the one below part and rt
+    __syncthreads();
   }
-  if (blockIdx.x != 0) {
-    if (update && q == 0 && i < n) y[i] = yi;
-    return;
-  }
-  if (q == 0) ys[r] = yi;
-  __syncthreads();
-  if (tid < 32) tile_forward(t, dlo, dhi, ys, y, d0, dnb, tid);
-}
-
-// One backward step of L' x = y, in place: rows [0, k0) take the update from the solved tile [k0, k0 + unb), CTA b
-// the 64 rows below k0 - 64 b, a warp per row reading that row's entries of the tile's rows of L (64 contiguous
-// values of one column of W); then CTA 0, whose rows are the tile [k0 - NB, k0), solves it. Loads are issued before
-// the first barrier and CTA 0's rows stay in shared memory, as in the forward step.
-__global__ void __launch_bounds__(256) k_bwd_step(int64_t n, const double* __restrict__ W, const double* __restrict__ dinv,
-                                                  double* __restrict__ y, int64_t k0, int unb) {
-  __shared__ double t[NB][NB + 1];
-  __shared__ double xk[NB];
-  __shared__ double ys[NB];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int64_t row0 = k0 - NB * (int64_t)(blockIdx.x + 1);   // this CTA's rows [row0, row0 + 64)
+  load(inv + NB * row0, NB);
+  __syncthreads();   // rt (b = 0: as it was read from g)
+  const double yv = mul(rt);
+  if (q == 0) post_value(yf + row0 + r, yv);
+  __syncthreads();   // every thread has read rt
+  if (q == 0) rt[r] = yv;
+  // backward: a block's column sums, a warp per 8 columns, lanes over its rows
   double w0[8], w1[8];
+  auto load_t = [&](const double* M, int64_t stride) {
 #pragma unroll
-  for (int m = 0; m < 8; ++m) {
-    const double* colj = W + n * (row0 + warp * 8 + m) + k0;
-    w0[m] = lane < unb ? colj[lane] : 0.0;
-    w1[m] = lane + 32 < unb ? colj[lane + 32] : 0.0;
-  }
-  if (tid < NB) xk[tid] = tid < unb ? y[k0 + tid] : 0.0;
-  const double yold = lane < 8 ? y[row0 + warp * 8 + lane] : 0.0;
-  double dlo = 0.0, dhi = 0.0;
-  if (blockIdx.x == 0) {
-    load_scaled_tile(t, W, dinv, n, row0, NB, 1, tid);
-    if (tid < 32) {
-      dlo = dinv[row0 + tid];
-      dhi = dinv[row0 + 32 + tid];
+    for (int m = 0; m < 8; ++m) {
+      w0[m] = M[lane + stride * (8 * warp + m)];
+      w1[m] = M[lane + 32 + stride * (8 * warp + m)];
     }
+  };
+  auto mul_t = [&](const double* xs) {   // (M' xs)[8 warp + lane] in lanes below 8
+    const double x0 = xs[lane], x1 = xs[lane + 32];
+    double v = 0.0;
+#pragma unroll
+    for (int m = 0; m < 8; ++m) {
+      double s = w0[m] * x0 + w1[m] * x1;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      if (lane == m) v = s;
+    }
+    return v;
+  };
+  for (int k = nt - 1; k > b; --k) {
+    load_t(W + NB * (int64_t)k + ld * row0, ld);
+    __syncthreads();   // every thread has read the previous xk (first: rt is written)
+    if (tid < NB) xk[tid] = poll_value(yb + NB * (int64_t)k + tid);
+    __syncthreads();
+    const double v = mul_t(xk);
+    if (lane < 8) rt[8 * warp + lane] -= v;
   }
+  load_t(inv + NB * row0, NB);
   __syncthreads();
-  const double x0 = xk[lane], x1 = xk[lane + 32];
-  double s[8];
-#pragma unroll
-  for (int m = 0; m < 8; ++m) s[m] = w0[m] * x0 + w1[m] * x1;
-#pragma unroll
-  for (int m = 0; m < 8; ++m) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s[m] += __shfl_xor_sync(0xffffffffu, s[m], o);
+  const double xv = mul_t(rt);
+  if (lane < 8) {
+    const int64_t i = row0 + 8 * warp + lane;
+    post_value(yb + i, xv);
+    if (i < n) x[i] = xv;
   }
-  double v = s[0];
-#pragma unroll
-  for (int m = 1; m < 8; ++m)
-    if (lane == m) v = s[m];
-  if (blockIdx.x != 0) {
-    if (lane < 8) y[row0 + warp * 8 + lane] = yold - v;
-    return;
-  }
-  if (lane < 8) ys[warp * 8 + lane] = yold - v;
-  __syncthreads();
-  if (tid < 32) tile_backward(t, dlo, dhi, ys, y, row0, NB, tid);
-}
-
-// The last diagonal tile [d0, n) of the backward pass (the only one that may be short), solved by one warp.
-__global__ void __launch_bounds__(32) k_bwd_last(int64_t n, const double* __restrict__ W, const double* __restrict__ dinv,
-                                                 double* __restrict__ y, int64_t d0) {
-  __shared__ double t[NB][NB + 1];
-  __shared__ double ys[NB];
-  const int lane = threadIdx.x, dnb = (int)(n - d0);
-  for (int e = lane; e < NB * NB; e += 32) {
-    const int rr = e & 63, cc = e >> 6;
-    t[rr][cc] = (rr < dnb && cc < rr) ? W[(d0 + rr) + n * (d0 + cc)] * dinv[d0 + rr] : 0.0;
-  }
-  ys[lane] = lane < dnb ? y[d0 + lane] : 0.0;
-  ys[lane + 32] = lane + 32 < dnb ? y[d0 + 32 + lane] : 0.0;
-  const double dlo = lane < dnb ? dinv[d0 + lane] : 0.0, dhi = lane + 32 < dnb ? dinv[d0 + 32 + lane] : 0.0;
-  __syncwarp();
-  tile_backward(t, dlo, dhi, ys, y, d0, dnb, lane);
-}
-
-// x = (L L')^-1 x in place: the forward steps, then the backward steps, on stream s
-static void launch_solve(cudaStream_t s, int64_t n, const double* W, const double* dv, double* x) {
-  // forward: tile [0, NB) first, then each step updates the rows below the tile it just solved and solves the next
-  k_fwd_step<<<1, 256, 0, s>>>(n, W, dv, x, 0, (int)std::min<int64_t>(NB, n), 0);
-  for (int64_t d0 = NB; d0 < n; d0 += NB)
-    k_fwd_step<<<(unsigned)((n - d0 + NB - 1) / NB), 256, 0, s>>>(n, W, dv, x, d0, (int)std::min<int64_t>(NB, n - d0), 1);
-  // backward: the last (possibly short) tile first, then upward
-  const int64_t kl = ((n - 1) / NB) * NB;
-  k_bwd_last<<<1, 32, 0, s>>>(n, W, dv, x, kl);
-  for (int64_t k0 = kl; k0 > 0; k0 -= NB)
-    k_bwd_step<<<(unsigned)(k0 / NB), 256, 0, s>>>(n, W, dv, x, k0, (int)std::min<int64_t>(NB, n - k0));
 }
 
 // Launches kernel on stream st with the given priority (a launch attribute, so that a captured graph keeps it).
 template <class... Args>
-static void launch_prio(void (*kernel)(Args...), unsigned grid, unsigned block, size_t smem, cudaStream_t st, int prio,
-                        Args... args) {
+static void launch_prio(void (*kernel)(Args...), dim3 grid, unsigned block, size_t smem, cudaStream_t st, int prio, Args... args) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
+  cfg.gridDim = grid;
   cfg.blockDim = dim3(block);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
@@ -576,42 +597,64 @@ static void launch_prio(void (*kernel)(Args...), unsigned grid, unsigned block, 
   BLS_CUDA(cudaLaunchKernelEx(&cfg, kernel, args...));
 }
 
-// The factorisation after the load of S into W: panels on the panel stream p, trailing updates on s, joined on s.
+// The factorisation after the load of S into W: the diagonal tiles on the panel stream p, the panels below them and the
+// updates that the next panels wait for on u, the rest of each group's update on s, joined on s.
 static void launch_factor_body(DenseSolver* D, cudaStream_t s, cudaStream_t p) {
-  const int64_t n = D->n;
+  const int64_t ld = D->ld, nt = ld / NB;
   double* W = D->W.as<double>();
-  double* dv = D->dinv.as<double>();
+  double* v16 = D->inv16.as<double>();
+  double* inv = D->inv.as<double>();
   long long* st = D->status.as<long long>();
+  const long long* cst = st;
   const int prio = D->panel_priority;
-  BLS_CUDA(cudaEventRecord(D->ev_join, s));
-  BLS_CUDA(cudaStreamWaitEvent(p, D->ev_join, 0));
-  // panel k: its diagonal tile and the rows below it, on the panel stream. With few rows below, one launch in which
-  // every CTA factors the tile itself (a launch less on the panel chain); with many, the tile in one CTA and then the
-  // rows (the redundant factorisations would take SMs from the trailing update running beside them).
-  auto panel = [&](int64_t k0) {
-    const int nb = (int)std::min<int64_t>(NB, n - k0);
-    const int64_t below = (n - k0 - nb + NB - 1) / NB;
-    if (below <= kFusedPanelTiles) {
-      launch_prio(k_panel, (unsigned)std::max<int64_t>(1, below), 256, PANEL_SMEM, p, prio, n, W, dv, k0, nb, st);
-    } else {
-      launch_prio(k_potrf_tile, 1, 256, 0, p, prio, n, W, dv, k0, nb, st);
-      launch_prio(k_trsm_panel, (unsigned)below, NB, 0, p, prio, n, W, (const double*)dv, k0, (const long long*)st);
-    }
-    BLS_CUDA(cudaEventRecord(D->ev_panel, p));
+  cudaStream_t u = D->update_stream;
+  double* rows = D->rows.as<double>();   // two buffers, by the parity of the panel
+  double* none = nullptr;
+  auto then = [](cudaStream_t from, cudaEvent_t ev, cudaStream_t to) {
+    BLS_CUDA(cudaEventRecord(ev, from));
+    BLS_CUDA(cudaStreamWaitEvent(to, ev, 0));
   };
-  panel(0);
-  // Lookahead by one panel: the trailing update of panel k updates the next panel's tile column first; the next panel
-  // is factored on the panel stream while the caller's stream updates the tile columns after it.
-  for (int64_t k0 = 0; n - k0 > NB; k0 += NB) {
-    const int64_t nt = (n - k0 - NB + NB - 1) / NB;
-    BLS_CUDA(cudaStreamWaitEvent(s, D->ev_panel, 0));
-    k_syrk_tiles<<<(unsigned)nt, 256, SYRK_SMEM, s>>>(n, W, k0, 0, st);
-    BLS_CUDA(cudaEventRecord(D->ev_join, s));
-    BLS_CUDA(cudaStreamWaitEvent(p, D->ev_join, 0));
-    panel(k0 + NB);
-    if (nt > 1) k_syrk_tiles<<<(unsigned)((nt - 1) * nt / 2), 256, SYRK_SMEM, s>>>(n, W, k0, 1, st);
+  then(s, D->ev_join, p);
+  BLS_CUDA(cudaStreamWaitEvent(u, D->ev_join, 0));
+  launch_prio(k_step, dim3(1), 256, sizeof(StepSmem), p, prio, ld, W, (const double*)rows, v16, (int64_t)0, 1, st);
+  if (nt > 1) launch_prio(k_first_rows, dim3(1), 256, 0, p, prio, ld, (const double*)W, rows);
+  bool next_pending = false;
+  for (int64_t g0 = 0; g0 < nt; g0 += GROUP) {
+    const int64_t g1 = std::min(nt, g0 + GROUP);   // the group's panels
+    for (int64_t k = g0; k < g1; ++k) {
+      const int64_t below = nt - k - 1;
+      // u: the panel's rows, once its tile is factored; p: the next tile, once the previous panel's update (and, for a
+      // group's first panel, the previous group's) is done
+      then(p, D->ev_tile, u);
+      if (k > 0) BLS_CUDA(cudaStreamWaitEvent(p, D->ev_update, 0));
+      if (k == g0 && next_pending) {
+        BLS_CUDA(cudaStreamWaitEvent(p, D->ev_next, 0));
+        BLS_CUDA(cudaStreamWaitEvent(u, D->ev_next, 0));
+      }
+      launch_prio(k_trsm_panel, dim3((unsigned)(below + 1)), 256, sizeof(PanelSmem), u, prio, ld, W, (const double*)v16, inv, k * NB, cst);
+      if (below == 0) break;
+      launch_prio(k_step, dim3(1), 256, sizeof(StepSmem), p, prio, ld, W, (const double*)(rows + (k & 1) * NB * NB), v16, k * NB, 0, st);
+      // the group's remaining columns and the next group's first one, which the next panels need
+      const int64_t cols = std::min(nt, g1 + 1) - k - 1;
+      launch_prio(k_syrk<64, true>, dim3((unsigned)below, (unsigned)cols), 256, (size_t)syrk_smem<64, true>(), u, prio, ld, W, k * NB, NB,
+                  (k + 1) * NB, rows + ((k + 1) & 1) * NB * NB, cst);
+      BLS_CUDA(cudaEventRecord(D->ev_update, u));
+    }
+    if (g1 + 1 >= nt) continue;
+    // everything right of that, beside the next panels: the next group's other columns first (they wait for them)
+    const int K = (int)((g1 - g0) * NB);
+    const int64_t j0 = g1 + 1, g2 = std::min(nt, g1 + GROUP + 1);
+    then(u, D->ev_panel, s);
+    k_syrk<64, false><<<dim3((unsigned)(nt - j0), (unsigned)(g2 - j0)), 256, syrk_smem<64, false>(), s>>>(ld, W, g0 * NB, K, j0 * NB, none, cst);
+    BLS_CUDA(cudaEventRecord(D->ev_next, s));
+    next_pending = true;
+    if (g2 < nt) {
+      const int64_t rest = nt - g2;
+      k_syrk<128, false><<<dim3((unsigned)((rest + 1) / 2), (unsigned)rest), 256, syrk_smem<128, false>(), s>>>(ld, W, g0 * NB, K, g2 * NB, none, cst);
+    }
   }
-  BLS_CUDA(cudaStreamWaitEvent(s, D->ev_panel, 0));
+  then(p, D->ev_tile, s);
+  then(u, D->ev_update, s);
 }
 
 template <class T>
@@ -628,10 +671,16 @@ static int factor(DenseSolver* D, const T* S, double lambda, const double* s_r, 
     BLS_CUDA(cudaStreamCreateWithPriority(&D->panel_stream, cudaStreamNonBlocking, hi));
     BLS_CUDA(cudaEventCreateWithFlags(&D->ev_join, cudaEventDisableTiming));
     BLS_CUDA(cudaEventCreateWithFlags(&D->ev_panel, cudaEventDisableTiming));
-    BLS_CUDA(cudaFuncSetAttribute(k_syrk_tiles, cudaFuncAttributeMaxDynamicSharedMemorySize, SYRK_SMEM));
-    BLS_CUDA(cudaFuncSetAttribute(k_panel, cudaFuncAttributeMaxDynamicSharedMemorySize, PANEL_SMEM));
+    for (cudaEvent_t* e : {&D->ev_next, &D->ev_tile, &D->ev_update}) BLS_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
+    BLS_CUDA(cudaStreamCreateWithPriority(&D->update_stream, cudaStreamNonBlocking, hi));
+    BLS_CUDA(cudaFuncSetAttribute(k_syrk<64, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, syrk_smem<64, true>()));
+    BLS_CUDA(cudaFuncSetAttribute(k_syrk<64, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, syrk_smem<64, false>()));
+    BLS_CUDA(cudaFuncSetAttribute(k_syrk<128, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, syrk_smem<128, false>()));
+    BLS_CUDA(cudaFuncSetAttribute(k_step, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(StepSmem)));
+    BLS_CUDA(cudaFuncSetAttribute(k_trsm_panel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(PanelSmem)));
   }
-  k_dense_load<T><<<(unsigned)std::max<int64_t>(1, std::min<int64_t>((n * n + 255) / 256, 148 * 8)), 256, 0, s>>>(n, S, W, lambda, s_r, st);
+  const unsigned tiles = (unsigned)(D->ld / 32);
+  k_dense_load<T><<<dim3(tiles, tiles), 256, 0, s>>>(n, D->ld, S, W, lambda, s_r, st);
   if (!D->factor_graph) {
     if (!D->cap_stream) BLS_CUDA(cudaStreamCreateWithFlags(&D->cap_stream, cudaStreamNonBlocking));
     BLS_CUDA(cudaStreamBeginCapture(D->cap_stream, cudaStreamCaptureModeThreadLocal));
@@ -687,8 +736,11 @@ int bls_dense_solver_create(bls_ctx* ctx, int64_t n, bls_dense_solver** out) {
     std::unique_ptr<bls_dense_solver> D(new bls_dense_solver());
     D->ctx = ctx;
     D->n = n;
-    D->W.alloc(sizeof(double) * (size_t)(n * n));
-    D->dinv.alloc(sizeof(double) * (size_t)n);
+    D->ld = (n + NB - 1) / NB * NB;
+    D->W.alloc(sizeof(double) * (size_t)(D->ld * D->ld));
+    D->rows.alloc(sizeof(double) * 2 * NB * NB);
+    D->inv16.alloc(sizeof(double) * 16 * (size_t)D->ld);
+    D->inv.alloc(sizeof(double) * NB * (size_t)D->ld);
     D->status.alloc(sizeof(long long));
     *out = D.release();
     return BLS_OK;
@@ -726,31 +778,24 @@ int bls_dense_cholesky_solve(bls_dense_solver* D, const double* g, double* x) {
     if (!D->factored) throw Error(BLS_EINVAL, "the solver holds no factorisation (bls_dense_cholesky first, and it must succeed)");
     const int64_t n = D->n;
     const double* W = D->W.as<double>();
-    const double* dv = D->dinv.as<double>();
     cudaStream_t s = D->ctx->stream;
-    if (!D->solve_graph) {
-      D->y.alloc(sizeof(double) * (size_t)n);
-      if (!D->cap_stream) BLS_CUDA(cudaStreamCreateWithFlags(&D->cap_stream, cudaStreamNonBlocking));
-      BLS_CUDA(cudaStreamBeginCapture(D->cap_stream, cudaStreamCaptureModeThreadLocal));
-      launch_solve(D->cap_stream, n, W, dv, D->y.as<double>());
-      cudaGraph_t gr = nullptr;
-      const cudaError_t e1 = cudaGetLastError();
-      const cudaError_t e2 = cudaStreamEndCapture(D->cap_stream, &gr);
-      if (e1 != cudaSuccess || e2 != cudaSuccess) {
-        if (gr) cudaGraphDestroy(gr);
-        throw Error(BLS_ECUDA, std::string("capturing the solve: ") + cudaGetErrorString(e1 != cudaSuccess ? e1 : e2));
-      }
-      const cudaError_t e3 = cudaGraphInstantiate(&D->solve_graph, gr, 0);
-      cudaGraphDestroy(gr);
-      if (e3 != cudaSuccess) {
-        D->solve_graph = nullptr;
-        throw Error(BLS_ECUDA, std::string("instantiating the solve: ") + cudaGetErrorString(e3));
-      }
+    // the tiles' CTAs must be resident at once (256 at the largest n)
+    const int64_t nt = D->ld / NB;
+    if (D->solve_grid == 0) {
+      int per_sm = 0, nsm = 0, dev = 0;
+      BLS_CUDA(cudaGetDevice(&dev));
+      BLS_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+      BLS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_solve, 256, 0));
+      if (nt > (int64_t)nsm * per_sm) throw Error(BLS_EUNSUPPORTED, "the device is too small for this system's solve");
+      D->y.alloc(sizeof(double) * 2 * (size_t)D->ld);
+      D->solve_grid = (int)nt;
     }
     double* y = D->y.as<double>();
-    BLS_CUDA(cudaMemcpyAsync(y, g, sizeof(double) * (size_t)n, cudaMemcpyDeviceToDevice, s));
-    BLS_CUDA(cudaGraphLaunch(D->solve_graph, s));
-    BLS_CUDA(cudaMemcpyAsync(x, y, sizeof(double) * (size_t)n, cudaMemcpyDeviceToDevice, s));
+    BLS_CUDA(cudaMemsetAsync(y, 0xff, sizeof(double) * 2 * (size_t)D->ld, s));
+    int64_t n_arg = n, ld_arg = D->ld;
+    const double* inv = D->inv.as<double>();
+    void* args[] = {&n_arg, &ld_arg, &W, &inv, &g, &x, &y};
+    BLS_CUDA(cudaLaunchCooperativeKernel((const void*)k_solve, dim3((unsigned)D->solve_grid), dim3(256), args, 0, s));
     BLS_CUDA(cudaGetLastError());
     return BLS_OK;
   })
