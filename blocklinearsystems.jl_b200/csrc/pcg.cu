@@ -13,6 +13,9 @@
 // per-row list built once per pattern (one warp per block row gathers its row: no atomics, deterministic). Vectors,
 // scalars and products are FP64 whatever S's storage type.
 //
+// With 6-column blocks the whole solve is one cooperative launch (k_pcg_cols); what follows is the form for every other
+// pattern, and for an S or x that cannot be read in pairs of entries.
+//
 // One PCG iteration is three kernels (four with the column product): (1) q = S p with the partial sums of p'q (the
 // column form takes a separate p'q pass); (2) alpha = (r'z)/(p'q), x += alpha p, r -= alpha q, z = M^-1 r (block
 // solves) with the partial sums of r'z and r'r; (3) beta, p = z + beta p, and the convergence test. Per-iteration scalars live in device slots, so a run of iterations can be replayed as one CUDA
@@ -22,7 +25,9 @@
 #include <algorithm>
 #include <cmath>
 #include <climits>
+#include <cstring>
 #include <memory>
+#include <type_traits>
 #include <vector>
 
 #include "pcg_plan.hpp"
@@ -409,6 +414,398 @@ __global__ void k_add(int64_t n, double* __restrict__ x, const double* __restric
 }
 
 // ---------------------------------------------------------------------------------------------------------------
+// The whole solve in one cooperative launch, for patterns whose retained blocks all have 6 columns
+// ---------------------------------------------------------------------------------------------------------------
+// The inverse of every 6 x 6 diagonal block of S (symmetric from its upper triangle), a thread per block in registers:
+// the Cholesky factor with k_factor_blocks's pivot test (the lowest failing block into *failed), its inverse, L^-T L^-1.
+template <class T>
+__global__ void __launch_bounds__(64) k_block_inverse6(int64_t nrb, const int64_t* __restrict__ dbase, const int32_t* __restrict__ dstride,
+                                                       const T* __restrict__ S, double* __restrict__ Minv, long long* __restrict__ failed) {
+  const int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (b >= nrb) return;
+  double L[6][6];
+  const T* B = S + dbase[b];
+  const int64_t stride = dstride[b];
+#pragma unroll
+  for (int j = 0; j < 6; ++j)
+#pragma unroll
+    for (int i = 0; i <= j; ++i) L[j][i] = (double)B[i + j * stride];
+  bool bad = false;
+#pragma unroll
+  for (int j = 0; j < 6; ++j) {
+    double s = L[j][j];
+#pragma unroll
+    for (int k = 0; k < j; ++k) s -= L[j][k] * L[j][k];
+    bad = bad || !(s > 0.0 && isfinite(s));
+    const double inv = 1.0 / sqrt(s);
+    L[j][j] = inv;   // the reciprocal of the pivot
+#pragma unroll
+    for (int i = j + 1; i < 6; ++i) {
+      double t = L[i][j];
+#pragma unroll
+      for (int k = 0; k < j; ++k) t -= L[i][k] * L[j][k];
+      L[i][j] = t * inv;
+    }
+  }
+  if (bad) {
+    atomicMin(failed, (long long)b);
+    return;
+  }
+#pragma unroll
+  for (int j = 0; j < 6; ++j) {   // L^-1 in place, column by column
+#pragma unroll
+    for (int i = j + 1; i < 6; ++i) {
+      double t = 0.0;
+#pragma unroll
+      for (int k = j; k < i; ++k) t -= L[i][k] * L[k][j];
+      L[i][j] = t * L[i][i];
+    }
+  }
+  double* M = Minv + 36 * b;
+#pragma unroll
+  for (int j = 0; j < 6; ++j)
+#pragma unroll
+    for (int i = 0; i < 6; ++i) {
+      double t = 0.0;
+#pragma unroll
+      for (int k = i > j ? i : j; k < 6; ++k) t += L[k][i] * L[k][j];
+      M[6 * j + i] = t;
+    }
+}
+
+// Scalars of a solve, zero on entry: the iterations' sums in four slots by turns (zeroed two iterations ahead), a start's
+// (its explicit residual) per start.
+struct PcgScalars {
+  double pq[4], rz[4], rr[4];
+  double srz[5], srr[5];
+  double gg;
+};
+struct PcgControl {
+  unsigned barrier, fault;
+  long long failed;      // the lowest block that is not positive definite (k_block_inverse6), LLONG_MAX: none
+  PcgScalars sum;
+  double out[4];         // iterations, squared residual, |g|^2, fault
+};
+template <class T>
+struct PcgArgs {
+  int64_t nrb, nr, nblk, maxit;
+  const int64_t *c_ptr, *c_base;
+  const int32_t *c_xo, *c_stride;
+  const T* S;
+  const double *g, *M;   // M: 6 x 6 preconditioner blocks, column-major
+  double *x, *r, *z, *p0, *p1, *q;
+  PcgControl* ctl;
+  double tol;
+};
+
+// Every CTA of the (co-resident) grid arrives before any leaves. A wait that gives up (2^22 polls, seconds) raises the
+// fault word, which ends every other wait, and false is returned to every thread.
+__device__ __forceinline__ bool grid_barrier(PcgControl* c, unsigned target) {
+  __syncthreads();
+  bool ok = true;
+  if (threadIdx.x == 0) {
+    __threadfence();
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&c->barrier) : "memory");
+    unsigned v = 0;
+    ok = false;
+    for (int i = 0; i < (1 << 22); ++i) {
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(&c->barrier) : "memory");
+      if ((int)(v - target) >= 0) { ok = true; break; }
+      if ((i & 1023) == 1023 && *reinterpret_cast<volatile unsigned*>(&c->fault)) break;
+    }
+    if (!ok) atomicExch(&c->fault, 1u);
+    __threadfence();
+  }
+  return !__syncthreads_or(!ok);
+}
+
+// PCG to ||g - S x|| <= tol ||g||. Per iteration two phases, each ended by a grid barrier: (A) q += S p, where p = z +
+// beta p_old is formed as it is read (and stored once for the next iteration), with p'q; (B) x, r, z = M r, r'z, r'r, and
+// q cleared. A start forms the explicit residual g - S x the same way; PCG stops on the recursive residual and starts
+// again from x while the explicit one is above the tolerance (at most four runs). In (A) the blocks are dealt evenly to
+// the warps in storage order; a lane takes two rows of a column's stack of blocks, six loads of two entries each. A CTA's
+// columns are neighbours, so the rows they reach make a short window: each warp adds its products up in a window of its
+// own in shared memory, and the CTA adds their sum to q (a window wider than kPcgWindow: every product by an
+// FP64 atomic, 3.6 million a product at 5000 cameras, which takes 45 us). Every scalar is read by all CTAs after a
+// barrier, so their decisions agree. 5000 cameras, FP32 S of 88 MB, 7 iterations: 604 us as graphs of four kernels an
+// iteration with a host read-back per phase of the solve, 385 us now (40 cameras 278 -> 126).
+constexpr int kPcgWindow = 1120;
+// one CTA an SM (a barrier of 444 CTAs of 256 threads took 4 us, two an iteration): 16 warps, in FP64 12, so that nothing spills (the windows leave
+// no L1 to spill to)
+template <class T>
+__host__ __device__ constexpr int pcg_warps() { return sizeof(T) == 4 ? 16 : 12; }
+template <class T>
+__global__ void __launch_bounds__(32 * pcg_warps<T>(), 1) k_pcg_cols(PcgArgs<T> a) {
+  constexpr int NW = pcg_warps<T>(), NT = 32 * NW;
+  __shared__ double red[2][NW];
+  __shared__ int s_row0;
+  extern __shared__ double acc_smem[];   // per warp kPcgWindow sums
+  PcgControl* c = a.ctl;
+  PcgScalars* sum = &c->sum;
+  if (c->failed != LLONG_MAX) return;   // uniform across the grid
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int64_t nwarps = (int64_t)gridDim.x * NW, w = (int64_t)blockIdx.x * NW + warp;
+  // The warps' shares: every column costs as much as kColumnCost blocks (its loads one after another, 1.5 us), so that the
+  // short columns of the first cameras do not gather in one warp (dealt by blocks alone, warp 0 had 21 columns and took 40
+  // us a product where the median took 17). Share v starts at block `at` of column `col`.
+  constexpr int64_t kColumnCost = 16;
+  auto share = [&](int64_t v, int64_t& col) {
+    const int64_t t = (a.nblk + kColumnCost * a.nrb) * v / nwarps;
+    int64_t lo = 0, hi = a.nrb;
+    while (hi - lo > 1) {
+      const int64_t mid = (lo + hi) / 2;
+      if (__ldg(a.c_ptr + mid) + kColumnCost * mid <= t) lo = mid;
+      else hi = mid;
+    }
+    col = lo;
+    const int64_t c0 = __ldg(a.c_ptr + lo), n = __ldg(a.c_ptr + lo + 1) - c0, at = t - c0 - kColumnCost * (lo + 1);
+    return v >= nwarps ? a.nblk : c0 + (at < 0 ? 0 : at < n ? at : n);
+  };
+  int64_t col0 = 0, unused = 0;
+  const int64_t k_begin = share(w, col0), k_end = share(w + 1, unused);
+  // the variables that the CTA's blocks touch: from the first row of its columns to the end of its last column
+  int64_t row0 = 0;
+  int span = 0;
+  {
+    const int64_t kb = share(NW * (int64_t)blockIdx.x, unused), ke = share(NW * ((int64_t)blockIdx.x + 1), unused);
+    if (tid == 0) s_row0 = INT_MAX;
+    __syncthreads();
+    int lo = INT_MAX;
+    for (int64_t k = kb + tid; k < ke; k += NT) lo = min(lo, __ldg(a.c_xo + k));
+    for (int o = 16; o > 0; o >>= 1) lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+    if (lane == 0) atomicMin(&s_row0, lo);
+    __syncthreads();
+    row0 = s_row0;
+    int64_t l = 0, h = a.nrb;   // the column of the CTA's last block
+    while (h - l > 1) {
+      const int64_t mid = (l + h) / 2;
+      if (__ldg(a.c_ptr + mid) < ke) l = mid;
+      else h = mid;
+    }
+    const int64_t n = ke > kb ? 6 * (l + 1) - row0 : 0;
+    span = n <= kPcgWindow ? (int)n : 0;
+  }
+  double* acc = span ? acc_smem + warp * kPcgWindow : nullptr;
+  if (acc)
+    for (int i = lane; i < span; i += 32) acc[i] = 0.0;
+  __syncwarp();
+  unsigned target = 0;
+  auto barrier = [&] { return grid_barrier(c, target += gridDim.x); };
+  // the CTA's two sums, added to global memory
+  auto add = [&](double u, double v, double* to_u, double* to_v) {
+    u = warp_sum_d(u);
+    v = warp_sum_d(v);
+    if (lane == 0) {
+      red[0][warp] = u;
+      red[1][warp] = v;
+    }
+    __syncthreads();
+    if (tid < 2) {
+      double s = 0.0;
+      for (int i = 0; i < NW; ++i) s += red[tid][i];
+      double* to = tid ? to_v : to_u;
+      if (to) atomicAdd(to, s);
+    }
+  };
+  // q += S v for v = in (old == nullptr) or in + beta old; returns this thread's part of v'q
+  auto product = [&](const double* in, const double* old, double beta) {
+    double vq = 0.0;
+    auto get = [&](int64_t i) {
+      double2 v = *reinterpret_cast<const double2*>(in + i);
+      if (old) {
+        const double2 o = *reinterpret_cast<const double2*>(old + i);
+        v.x += beta * o.x;
+        v.y += beta * o.y;
+      }
+      return v;
+    };
+    int64_t col = col0;
+    for (int64_t k = k_begin; k < k_end; ++col) {
+      const int64_t c0 = __ldg(a.c_ptr + col), c1 = __ldg(a.c_ptr + col + 1);
+      if (k >= c1) continue;   // a column without blocks (none in a valid pattern)
+      const int64_t ke = c1 < k_end ? c1 : k_end, j0 = 6 * col;
+      const int64_t stride = __ldg(a.c_stride + col);
+      const T* B = a.S + __ldg(a.c_base + c0);
+      double pj[6], t[6];
+#pragma unroll
+      for (int i = 0; i < 6; i += 2) {
+        const double2 v = get(j0 + i);
+        pj[i] = v.x;
+        pj[i + 1] = v.y;
+        t[i] = t[i + 1] = 0.0;
+      }
+      const int r1 = (int)(6 * (ke - c0));
+      // the next step's entries and row offset are in flight while a step is worked on
+      using V2 = typename std::conditional<sizeof(T) == 4, float2, double2>::type;
+      V2 sn[6];
+      int xn = 0;
+      auto fetch = [&](int rr) {
+#pragma unroll
+        for (int i = 0; i < 6; ++i) sn[i] = __ldg(reinterpret_cast<const V2*>(B + rr + i * stride));
+        xn = __ldg(a.c_xo + c0 + rr / 6);
+      };
+      int rr = (int)(6 * (k - c0)) + 2 * lane;
+      if (rr < r1) fetch(rr);
+      for (; rr < r1; rr += 64) {
+        double s0[6], s1[6];
+#pragma unroll
+        for (int i = 0; i < 6; ++i) {
+          s0[i] = (double)sn[i].x;
+          s1[i] = (double)sn[i].y;
+        }
+        const int ra = rr % 6;
+        const int64_t xo = xn;
+        if (rr + 64 < r1) fetch(rr + 64);
+        const double2 pi = get(xo + ra);
+        const bool off = xo != j0;   // not the diagonal block, which takes its upper triangle both ways
+        double v0 = 0.0, v1 = 0.0;
+#pragma unroll
+        for (int i = 0; i < 6; ++i) {
+          if (off || i >= ra) v0 += s0[i] * pj[i];
+          if (off || i > ra) {
+            v1 += s1[i] * pj[i];
+            t[i] += s0[i] * pi.x;
+          }
+          if (off || i > ra + 1) t[i] += s1[i] * pi.y;
+        }
+        if (acc) {   // a column's rows are distinct: no two lanes meet
+          double2* to = reinterpret_cast<double2*>(acc + (xo + ra - row0));
+          double2 o = *to;
+          o.x += v0;
+          o.y += v1;
+          *to = o;
+        } else {
+          atomicAdd(a.q + xo + ra, v0);
+          atomicAdd(a.q + xo + ra + 1, v1);
+        }
+        vq += v0 * pi.x + v1 * pi.y;
+      }
+      double own = 0.0;
+#pragma unroll
+      for (int i = 0; i < 6; ++i) {
+        vq += t[i] * pj[i];
+        const double s = warp_sum_d(t[i]);
+        if (lane == i) own = s;
+      }
+      __syncwarp();   // the rows' sums, before the column's own and before the next column's
+      if (lane < 6) {
+        if (acc) acc[j0 + lane - row0] += own;
+        else atomicAdd(a.q + j0 + lane, own);
+      }
+      __syncwarp();
+      k = ke;
+    }
+    if (span) {   // the CTA's sums to q, and its windows cleared for the next product
+      __syncthreads();
+      for (int i = tid; i < span; i += NT) {
+        double s = 0.0;
+#pragma unroll 8
+        for (int o = 0; o < NW; ++o) {
+          s += acc_smem[o * kPcgWindow + i];
+          acc_smem[o * kPcgWindow + i] = 0.0;
+        }
+        if (s != 0.0) atomicAdd(a.q + row0 + i, s);
+      }
+    }
+    return vq;
+  };
+  // six lanes per block, five blocks per warp: f(variable, its place in the block, whether it exists) for every variable
+  const int sub = lane / 6, ii = lane - 6 * sub;
+  auto rows = [&](auto&& f) {
+    for (int64_t b0 = w * 5; b0 < a.nrb; b0 += nwarps * 5) {
+      const int64_t b = b0 + sub;
+      f(6 * b + ii, b, sub < 5 && b < a.nrb);
+    }
+  };
+  // z = M r of the lane's variable from its block's six residuals
+  auto precondition6 = [&](int64_t b, bool on, double r) {
+    double z = 0.0;
+#pragma unroll
+    for (int j = 0; j < 6; ++j) {
+      const double rj = __shfl_sync(0xffffffffu, r, (6 * sub + j) & 31);
+      if (on) z += __ldg(a.M + 36 * b + 6 * j + ii) * rj;
+    }
+    return z;
+  };
+  int64_t it = 0;
+  double rr = 0.0, gg = 0.0;
+  for (int run = 0;; ++run) {
+    // the explicit residual of x
+    product(a.x, nullptr, 0.0);
+    if (!barrier()) break;
+    double urz = 0.0, urr = 0.0, ugg = 0.0;
+    rows([&](int64_t i, int64_t b, bool on) {
+      const double g = on ? __ldg(a.g + i) : 0.0, r = on ? g - a.q[i] : 0.0;
+      const double z = precondition6(b, on, r);
+      if (on) {
+        a.q[i] = 0.0;
+        a.r[i] = r;
+        a.z[i] = z;
+      }
+      urz += r * z;
+      urr += r * r;
+      ugg += g * g;
+    });
+    add(urz, urr, &sum->srz[run], &sum->srr[run]);
+    if (run == 0) {
+      __syncthreads();   // red is read
+      add(ugg, 0.0, &sum->gg, nullptr);
+    }
+    if (!barrier()) break;
+    gg = *reinterpret_cast<volatile double*>(&sum->gg);
+    rr = *reinterpret_cast<volatile double*>(&sum->srr[run]);
+    double rz = *reinterpret_cast<volatile double*>(&sum->srz[run]), rz_old = 0.0;
+    const double t2 = a.tol * a.tol * gg;
+    if (!(rr > t2) || run == 4 || it >= a.maxit || (run > 0 && !isfinite(rr))) break;
+    bool first = true, ok = true;
+    double rec = rr;
+    while (it < a.maxit && rec > t2) {   // a NaN stops too
+      const int s0 = (int)(it & 3), s1 = (int)((it + 1) & 3), s2 = (int)((it + 2) & 3);
+      if (blockIdx.x == 0 && tid == 0) sum->pq[s2] = sum->rz[s2] = sum->rr[s2] = 0.0;
+      double* p = it & 1 ? a.p1 : a.p0;
+      const double* old = first ? nullptr : it & 1 ? a.p0 : a.p1;
+      const double beta = first ? 0.0 : rz / rz_old;
+      const double pq_part = product(a.z, old, beta);
+      rows([&](int64_t i, int64_t, bool on) {
+        if (on) p[i] = old ? a.z[i] + beta * old[i] : a.z[i];
+      });
+      add(pq_part, 0.0, &sum->pq[s0], nullptr);
+      if (!(ok = barrier())) break;
+      const double alpha = rz / *reinterpret_cast<volatile double*>(&sum->pq[s0]);
+      double vrz = 0.0, vrr = 0.0;
+      rows([&](int64_t i, int64_t b, bool on) {
+        double r = 0.0;
+        if (on) {
+          a.x[i] += alpha * p[i];
+          r = a.r[i] - alpha * a.q[i];
+          a.q[i] = 0.0;
+          a.r[i] = r;
+        }
+        const double z = precondition6(b, on, r);
+        if (on) a.z[i] = z;
+        vrz += r * z;
+        vrr += r * r;
+      });
+      __syncthreads();   // red is read
+      add(vrz, vrr, &sum->rz[s1], &sum->rr[s1]);
+      if (!(ok = barrier())) break;
+      rz_old = rz;
+      rz = *reinterpret_cast<volatile double*>(&sum->rz[s1]);
+      rec = *reinterpret_cast<volatile double*>(&sum->rr[s1]);
+      first = false;
+      ++it;
+    }
+    if (!ok) break;
+  }
+  if (blockIdx.x == 0 && tid == 0) {
+    c->out[0] = (double)it;
+    c->out[1] = rr;
+    c->out[2] = gg;
+    c->out[3] = (double)*reinterpret_cast<volatile unsigned*>(&c->fault);
+  }
+}
+
+// ---------------------------------------------------------------------------------------------------------------
 // Host side
 // ---------------------------------------------------------------------------------------------------------------
 static PCGPlan* pcg_plan_create(bls_ctx* ctx, int64_t nrb, const int64_t* r_dims, const int64_t* bcolptr, const int64_t* browval,
@@ -492,6 +889,15 @@ static PCGPlan* pcg_plan_create(bls_ctx* ctx, int64_t nrb, const int64_t* r_dims
       upload(P->c_xo, cxo, s);
       upload(P->c_stride, cstr, s);
       P->cols6 = true;
+      P->one_launch = true;
+      for (int64_t r2 = 0; r2 < nrb && P->one_launch; ++r2)
+        for (int64_t k = bcolptr[r2]; k < bcolptr[r2 + 1]; ++k)
+          if (brow_off[k] != 6 * (k - bcolptr[r2]) || ((Scolptr[boff[r2]] | col_h[r2]) & 1)) P->one_launch = false;
+      if (P->one_launch) {
+        P->p2.alloc(sizeof(double) * nr);
+        P->Minv.alloc(sizeof(double) * 36 * nrb);
+        P->ctl.alloc(sizeof(PcgControl));
+      }
     }
   }
   upload(P->r_dims, dims, s);
@@ -506,7 +912,7 @@ static PCGPlan* pcg_plan_create(bls_ctx* ctx, int64_t nrb, const int64_t* r_dims
   P->q.alloc(sizeof(double) * nr);
   P->scal.alloc(sizeof(double) * ((P->K + 1) * PS_W + 8));
   P->flags.alloc(sizeof(int) * 4 + sizeof(long long) * 2);
-  BLS_CUDA(cudaMallocHost(&P->host, sizeof(double) * 8));
+  BLS_CUDA(cudaMallocHost(&P->host, sizeof(PcgControl)));
   BLS_CUDA(cudaStreamSynchronize(s));
   return P.release();
 }
@@ -575,12 +981,83 @@ static void run_block(PCGPlan* P, const T* S, double* x, int n, cudaStream_t s) 
   for (int j = 0; j < n; ++j) iteration<T>(P, S, x, j, s);
 }
 
+// The one-launch solve: the diagonal blocks' inverses, k_pcg_cols, one read-back.
+template <class T>
+static int pcg_solve_cols(PCGPlan* P, const T* S, const double* g, double* x, double tol, int64_t maxit, int64_t* iters_out, double* rel_out,
+                          int64_t* failed_block) {
+  cudaStream_t s = P->ctx->stream;
+  PcgControl* ctl = P->ctl.as<PcgControl>();
+  PcgControl* h = reinterpret_cast<PcgControl*>(P->host);
+  std::memset(h, 0, sizeof(PcgControl));
+  h->failed = LLONG_MAX;
+  BLS_CUDA(cudaMemcpyAsync(ctl, h, sizeof(PcgControl), cudaMemcpyHostToDevice, s));
+  BLS_CUDA(cudaMemsetAsync(P->q.p, 0, sizeof(double) * P->nr, s));
+  k_block_inverse6<T><<<grid_for(P->nrb, 64), 64, 0, s>>>(P->nrb, P->diag_base.as<int64_t>(), P->diag_stride.as<int32_t>(), S,
+                                                          P->Minv.as<double>(), &ctl->failed);
+  int& grid = P->pcg_grid[sizeof(T) == 4 ? 0 : 1];
+  constexpr int NW = pcg_warps<T>();
+  const int smem = NW * kPcgWindow * (int)sizeof(double);
+  if (grid == 0) {
+    int per_sm = 0, nsm = 0, dev = 0;
+    BLS_CUDA(cudaGetDevice(&dev));
+    BLS_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+    BLS_CUDA(cudaFuncSetAttribute(k_pcg_cols<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    BLS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pcg_cols<T>, 32 * NW, smem));
+    // a warp per six blocks at the least: small systems take fewer CTAs, whose barriers are cheaper
+    const int64_t nblk = (int64_t)(P->c_xo.bytes / sizeof(int32_t));
+    grid = (int)std::max<int64_t>(1, std::min<int64_t>((nblk + 6 * NW - 1) / (6 * NW), (int64_t)std::max(1, per_sm) * nsm));
+  }
+  PcgArgs<T> a;
+  a.nrb = P->nrb;
+  a.nr = P->nr;
+  a.nblk = (int64_t)(P->c_xo.bytes / sizeof(int32_t));
+  a.maxit = maxit;
+  a.c_ptr = P->c_ptr.as<int64_t>();
+  a.c_base = P->c_base.as<int64_t>();
+  a.c_xo = P->c_xo.as<int32_t>();
+  a.c_stride = P->c_stride.as<int32_t>();
+  a.S = S;
+  a.g = g;
+  a.M = P->precond ? P->precond : P->Minv.as<double>();
+  a.x = x;
+  a.r = P->r.as<double>();
+  a.z = P->z.as<double>();
+  a.p0 = P->p.as<double>();
+  a.p1 = P->p2.as<double>();
+  a.q = P->q.as<double>();
+  a.ctl = ctl;
+  a.tol = tol;
+  void* args[] = {&a};
+  BLS_CUDA(cudaLaunchCooperativeKernel((const void*)k_pcg_cols<T>, dim3((unsigned)grid), dim3(32 * NW), args, (size_t)smem, s));
+  P->launches += 2;
+  BLS_CUDA(cudaMemcpyAsync(h, ctl, sizeof(PcgControl), cudaMemcpyDeviceToHost, s));
+  BLS_CUDA(cudaStreamSynchronize(s));
+  if (h->failed != LLONG_MAX) {
+    if (failed_block) *failed_block = h->failed + 1;
+    return BLS_NOT_PD;
+  }
+  if (h->out[3] != 0.0) throw Error(BLS_ECUDA, "a grid barrier of the PCG solve did not complete within its wait limit");
+  *iters_out = (int64_t)h->out[0];
+  if (h->out[2] == 0.0) {   // g = 0
+    k_zero_d<<<grid_for(P->nr, 256), 256, 0, s>>>(x, P->nr);
+    P->launches += 1;
+    *iters_out = 0;
+    *rel_out = 0.0;
+    return BLS_OK;
+  }
+  *rel_out = std::sqrt(h->out[1] / h->out[2]);
+  return *rel_out <= tol || h->out[1] <= tol * tol * h->out[2] ? BLS_OK : BLS_NOT_CONVERGED;
+}
+
 // PCG to ||g - S x|| <= tol ||g|| (FP64), block-Jacobi preconditioner in P->D (factored). Returns BLS_OK,
 // BLS_NOT_CONVERGED (maxit reached) or BLS_NOT_PD (a diagonal block of S is not positive definite).
 template <class T>
 static int pcg_solve(PCGPlan* P, const T* S, const double* g, double* x, double tol, int64_t maxit, bool use_graph, int64_t* iters_out,
                      double* rel_out, int64_t* failed_block) {
   if (!(tol > 0) || maxit < 0) throw Error(BLS_EINVAL, "tol must be positive and maxit non-negative");
+  // one launch where every retained block has 6 columns and S and x can be read in pairs of entries
+  if (P->one_launch && reinterpret_cast<uintptr_t>(S) % (2 * sizeof(T)) == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0)
+    return pcg_solve_cols<T>(P, S, g, x, tol, maxit, iters_out, rel_out, failed_block);
   cudaStream_t s = P->ctx->stream;
   int* flags = P->flags.as<int>();
   double* scal = P->scal.as<double>();

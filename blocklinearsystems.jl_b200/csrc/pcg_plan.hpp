@@ -31,6 +31,11 @@ struct PCGPlan {
   // variables' offset; S is read once, the products scattered into q with FP64 atomics
   bool cols6 = false;
   DevBuf c_ptr, c_base, c_xo, c_stride;
+  // the one-launch solve (k_pcg_cols): columns whose blocks are stacked without gaps; its second direction vector, the
+  // inverses of the diagonal blocks, and {grid barrier, failing block, scalars, result} (ctl)
+  bool one_launch = false;
+  DevBuf p2, Minv, ctl;
+  int pcg_grid[2] = {0, 0};
   DevBuf ref_r, ref_d, ref_y;   // refined solve: outer residual, correction, operator product (FP64, allocated at its first call)
   int K = 8;                // iterations per replayed graph
   cudaGraphExec_t graph = nullptr;

@@ -137,7 +137,8 @@ class PCGWorkspace:
               graph: bool = True, preconditioner: torch.Tensor | None = None) -> tuple[torch.Tensor, PCGResult]:
         """PCG from x (zero when None) to ||g - S x|| <= tol ||g|| on an explicit FP64 residual, preconditioned by
         block-Jacobi or, when given, by the dense SPD blocks `preconditioner` (float64, d x d per block, as
-        LearnedPreconditioner.blocks returns them). x is updated in place and returned with the run's PCGResult."""
+        LearnedPreconditioner.blocks returns them). x is updated in place and returned with the run's PCGResult. `graph`
+        (patterns with other than 6-column blocks; those run as one launch): replay the iterations as a CUDA graph."""
         if preconditioner is not None:
             _dev(preconditioner, "preconditioner", self.ndiag, torch.float64)
         check(_lib.gpu().bls_pcg_set_preconditioner(self.handle, dptr(preconditioner)))

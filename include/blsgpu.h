@@ -452,7 +452,8 @@ int bls_spmv_sym(bls_pcg_plan* plan, int dtype, const void* S_nzval_dev, const d
 int bls_extract_diagonal_blocks(bls_pcg_plan* plan, int dtype, const void* S_nzval_dev, double* D_dev);
 /* PCG from the initial x to ||g - S x||_2 <= tol ||g||_2, checked on an explicit FP64 residual (restarted from x while
  * the recursive residual has drifted: iterative refinement), preconditioned by the block-Jacobi factorisation of S's
- * diagonal blocks. use_graph: replay runs of iterations as one CUDA graph. Returns BLS_OK, BLS_NOT_CONVERGED (maxit
+ * diagonal blocks. use_graph: replay runs of iterations as one CUDA graph (patterns
+ * whose retained blocks all have 6 columns run the whole solve as one cooperative launch). Returns BLS_OK, BLS_NOT_CONVERGED (maxit
  * reached; x is the last iterate) or BLS_NOT_PD (failed_block = the lowest diagonal block of S, 1-based, that is not
  * positive definite). iterations and rel_residual report the run. */
 int bls_pcg_solve(bls_pcg_plan* plan, int dtype, const void* S_nzval_dev, const double* g_dev, double* x_dev, double tol,
