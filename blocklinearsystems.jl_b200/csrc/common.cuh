@@ -39,6 +39,27 @@ __device__ __forceinline__ void run_cp16(void* smem, const void* gmem, int bytes
 __device__ __forceinline__ void run_cp_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void run_cp_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
+
+// Add six consecutive entries of a column of S (vector reductions where the address allows: red.global.add.v4/.v2
+// for FP32, scalar for FP64). v[i] goes to col[i].
+__device__ __forceinline__ void red2(float* p, float a, float b) {
+  asm volatile("red.relaxed.gpu.global.add.v2.f32 [%0], {%1, %2};\n" ::"l"(p), "f"(a), "f"(b) : "memory");
+}
+__device__ __forceinline__ void red4(float* p, float a, float b, float c, float d) {
+  asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};\n" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
+}
+__device__ __forceinline__ void red_column6(float* col, const float v[6]) {
+  switch ((reinterpret_cast<uintptr_t>(col) >> 2) & 3) {   // position of col[0] within its 16-byte line
+    case 0: red4(col, v[0], v[1], v[2], v[3]); red2(col + 4, v[4], v[5]); break;
+    case 1: atomicAdd(col, v[0]); red2(col + 1, v[1], v[2]); red2(col + 3, v[3], v[4]); atomicAdd(col + 5, v[5]); break;
+    case 2: red2(col, v[0], v[1]); red4(col + 2, v[2], v[3], v[4], v[5]); break;
+    default: atomicAdd(col, v[0]); red4(col + 1, v[1], v[2], v[3], v[4]); atomicAdd(col + 5, v[5]); break;
+  }
+}
+__device__ __forceinline__ void red_column6(double* col, const double v[6]) {
+#pragma unroll
+  for (int i = 0; i < 6; ++i) atomicAdd(col + i, v[i]);
+}
 #endif
 
 inline int grid_for(int64_t n, int threads) { return (int)((n + threads - 1) / threads); }

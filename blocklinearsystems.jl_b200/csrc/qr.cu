@@ -81,7 +81,9 @@ struct QRPlan {
   // reduced_tmul!'s per-(entry, column) dot products (allocated at its first call), rdmax = the largest retained block
   DevBuf tm_part, red_tab, u_meta;
   int rdmax = 0;
-  DevBuf ls_u, ls_v, ls_h, ls_hbar, ls_t, ls_w, ls_sqd, ls_part, ls_L, ls_acc, ls_flag;
+  DevBuf ls_u, ls_v, ls_h, ls_hbar, ls_t, ls_sqd, ls_part, ls_L, ls_acc, ls_flag;
+  DevBuf ls_chunk;      // the first table of every chunk of k_lsmr_pass, and ntables
+  int64_t ls_nchunks = 0;
   double* ls_host = nullptr;
   DevBuf status;
   long long* host_status = nullptr;
@@ -611,8 +613,10 @@ __global__ void k_qr_free(int64_t t0, int64_t nt, const int32_t* __restrict__ t_
 // accumulate_qr_entry! (src/qr_reduced.jl:375-405) per table. MODE 0: S blocks (upper triangle of diagonal blocks) and
 // J~'r~ into g; MODE 1: the full diagonal blocks D (reduced_diagonal_blocks!, :484-512). from_raw: the same products
 // over the data rows of the raw tables, J'J of the retained columns and J'r (the retained part of the assembly).
-template <class T, int MODE, bool ALL6>
-__global__ void __launch_bounds__(32 * QR_MAX_WARPS) k_qr_gram(int64_t ntab, int warp_bytes, const int32_t* __restrict__ tables,
+// WHOLE: tables with more than 16 pairs take a whole 6 x 6 block per lane; the form without it, for classes of smaller
+// tables, is held to 64 registers in FP32, eight CTAs an SM.
+template <class T, int MODE, bool ALL6, bool WHOLE>
+__global__ void __launch_bounds__(32 * QR_MAX_WARPS, sizeof(T) == 4 && ALL6 && !WHOLE ? 8 : 1) k_qr_gram(int64_t ntab, int warp_bytes, const int32_t* __restrict__ tables,
                                                               const int32_t* __restrict__ t_rows, const int32_t* __restrict__ t_cols,
                                                               const int32_t* __restrict__ t_top, const int64_t* __restrict__ t_raw,
                                                               const int64_t* __restrict__ t_res, const int32_t* __restrict__ t_ptr,
@@ -642,6 +646,47 @@ __global__ void __launch_bounds__(32 * QR_MAX_WARPS) k_qr_gram(int64_t ntab, int
   // rows [row0, row0 + n): the bottom rows J~ of a factored table, or the data rows of a raw one (its damping rows last)
   const int row0 = from_raw ? 0 : top;
   const T* src = F + t_raw[t] + row0;
+  // What the products and sums need besides the table: tables of 6 x 6 blocks look the first of it up while the table is
+  // on its way (each is a chain of two or three loads: 447 us -> 386 on 500 x 100,000 in FP32, and 374 with WHOLE).
+  const int npairs = kt * (kt + 1) / 2;
+  struct Unit { int u1, u2, w0, r2; int64_t base, stride; };   // w0 < 0: none
+  auto unit_of = [&](int q, int G) {
+    Unit v{0, 0, -1, 0, 0, 0};
+    const int upp = (dmax + G - 1) / G;
+    if (q >= npairs * upp) return v;
+    const int p = q / upp;
+    v.w0 = G * (q - p * upp);
+    int u2l = (int)((sqrtf(8.0f * p + 1.0f) - 1.0f) * 0.5f);
+    while ((u2l + 1) * (u2l + 2) / 2 <= p) ++u2l;
+    while (u2l * (u2l + 1) / 2 > p) --u2l;
+    v.u2 = u2l;
+    v.u1 = p - u2l * (u2l + 1) / 2;
+    if (MODE == 0) {
+      const int k = tp_blk[tp_ptr[t] + p];
+      v.stride = blk_stride ? (int64_t)blk_stride[k] : dense_nr;
+      v.base = blk_base[k] + v.w0 * v.stride;
+    } else {
+      v.r2 = u_ret[u0 + v.u2];
+    }
+    return v;
+  };
+  // the variable of column j of the table
+  auto variable = [&](int j) {
+    if (ALL6) {
+      const int u = u0 + j / 6, c0 = u_col[u];
+      if (c0 == j - j % 6) return boff_r[u_ret[u]] + (j - c0);
+    }
+    int gi = 0;
+    for (int u = u0; u < u0 + kt; ++u) {
+      const int c0 = u_col[u], r = u_ret[u];
+      if (j >= c0 && j < c0 + r_dims[r]) gi = boff_r[r] + (j - c0);
+    }
+    return gi;
+  };
+  const bool whole = WHOLE && npairs > 16;   // a whole block per lane
+  Unit first{0, 0, -1, 0, 0, 0};
+  int first_var = 0;
+  bool looked_up = ALL6;
   if (bulk && ce > 0) {
     // rows row0.. of columns 0..ce-1 lie in one contiguous span of (ce - 1) M + n entries: one bulk copy (TMA), the
     // columns then at stride M (the rows above row0 of columns 1.. come along and are not read)
@@ -657,6 +702,10 @@ __global__ void __launch_bounds__(32 * QR_MAX_WARPS) k_qr_gram(int64_t ntab, int
     }
     B = span_first(reinterpret_cast<T*>(bbase), sb);
     rr = span_first(reinterpret_cast<double*>(rbase), sr);
+    if (ALL6) {
+      first = unit_of(lane, whole ? 6 : 3);
+      if (MODE == 0 && lane < ce) first_var = variable(lane);
+    }
     __syncwarp();
     if (!mbar_wait(bar, 0)) {
       if (lane == 0) atomicExch(reinterpret_cast<unsigned long long*>(st + 2), 1ull);   // a copy that did not land: fault
@@ -666,6 +715,7 @@ __global__ void __launch_bounds__(32 * QR_MAX_WARPS) k_qr_gram(int64_t ntab, int
     __syncwarp();
   } else {
     ns = n | 1;
+    looked_up = false;
     rr = reinterpret_cast<double*>(rbase);
     B = reinterpret_cast<T*>(bbase);
     for (int q = lane; q < ce * n; q += 32) {
@@ -678,16 +728,11 @@ __global__ void __launch_bounds__(32 * QR_MAX_WARPS) k_qr_gram(int64_t ntab, int
     __syncwarp();
   }
   if (MODE == 0) {
-    // J~'r~: lane per column, entry found by scanning the table's entries
+    // J~'r~: lane per column
     for (int j = lane; j < ce; j += 32) {
-      int gi = 0;
-      for (int u = u0; u < u0 + kt; ++u) {
-        const int c0 = u_col[u], r = u_ret[u];
-        if (j >= c0 && j < c0 + r_dims[r]) gi = boff_r[r] + (j - c0);
-      }
       double acc = 0.0;
       for (int i = 0; i < n; ++i) acc += (double)B[j * ns + i] * rr[i];
-      atomicAdd(g + gi, acc);
+      atomicAdd(g + (looked_up && j == lane ? first_var : variable(j)), acc);
     }
   }
   // From the raw tables (the assembly), an entry's columns are zero outside its own observations' rows in a
@@ -714,75 +759,82 @@ __global__ void __launch_bounds__(32 * QR_MAX_WARPS) k_qr_gram(int64_t ntab, int
     __syncwarp();
     span = sp;
   }
-  // work units: (pair, a group of three columns of the pair's block); lanes take units in order, so the lanes of one
-  // pair read the same X rows (shared-memory broadcast)
-  const int npairs = kt * (kt + 1) / 2;
-  constexpr int G = 3;   // columns of the pair's block per work unit
-  const int upp = (dmax + G - 1) / G;
-  for (int q = lane; q < npairs * upp; q += 32) {
-    const int p = q / upp, w0 = G * (q - p * upp);
-    int u2l = (int)((sqrtf(8.0f * p + 1.0f) - 1.0f) * 0.5f);
-    while ((u2l + 1) * (u2l + 2) / 2 <= p) ++u2l;
-    while (u2l * (u2l + 1) / 2 > p) --u2l;
-    const int u1l = p - u2l * (u2l + 1) / 2;
-    const bool diag = u1l == u2l;
-    if (MODE == 1 && !diag) continue;
-    const int r1 = u_ret[u0 + u1l], r2 = u_ret[u0 + u2l];
-    const int d1 = r_dims[r1], d2 = r_dims[r2];
-    if (w0 >= d2) continue;
-    const int ilo = span ? max(span[u1l].x, span[u2l].x) : 0, ihi = span ? min(span[u1l].y, span[u2l].y) : n;
-    if (ilo >= ihi) continue;
-    const T* X = B + u_col[u0 + u1l] * ns;
-    const T* Y = B + (u_col[u0 + u2l] + w0) * ns;
-    T* out;
-    int64_t stride;
-    if (MODE == 0) {
-      const int k = tp_blk[tp_ptr[t] + p];
-      stride = blk_stride ? (int64_t)blk_stride[k] : dense_nr;
-      out = S + blk_base[k] + w0 * stride;
-    } else {
-      stride = d2;
-      out = S + doff[r2] + w0 * d2;
-    }
-    if (ALL6 || (d1 == 6 && d2 == 6)) {
-      // products accumulated in the storage type: FP32 in the mixed form (the bulk of the arithmetic), FP64 otherwise
-      T acc[G][6];
-#pragma unroll
-      for (int w = 0; w < G; ++w)
-#pragma unroll
-        for (int a = 0; a < 6; ++a) acc[w][a] = T(0);
-      for (int i = ilo; i < ihi; ++i) {
-        T x[6], y[G];
-#pragma unroll
-        for (int a = 0; a < 6; ++a) x[a] = X[a * ns + i];
-#pragma unroll
-        for (int w = 0; w < G; ++w) y[w] = Y[w * ns + i];
+  // work units: (pair, a group of G columns of the pair's block); lanes take units in order, so the lanes of one pair read
+  // the same X rows (shared-memory broadcast). FP32 tables of 6 x 6 blocks with more than 16 pairs take a whole block per
+  // lane (12 loads per 36 products instead of 9 per 18), the others three columns, which keeps more lanes busy. FP32
+  // columns are added with vector reductions (two or three per column instead of six atomics).
+  auto units = [&](auto g_const) {
+    constexpr int G = decltype(g_const)::value;   // columns of the pair's block per work unit
+    const int upp = (dmax + G - 1) / G;
+    for (int q = lane; q < npairs * upp; q += 32) {
+      const Unit v = looked_up && q == lane ? first : unit_of(q, G);
+      const int u1l = v.u1, u2l = v.u2, w0 = v.w0;
+      const bool diag = u1l == u2l;
+      if (MODE == 1 && !diag) continue;
+      const int d1 = ALL6 ? 6 : r_dims[u_ret[u0 + u1l]], d2 = ALL6 ? 6 : r_dims[u_ret[u0 + u2l]];
+      if (w0 >= d2) continue;
+      const int ilo = span ? max(span[u1l].x, span[u2l].x) : 0, ihi = span ? min(span[u1l].y, span[u2l].y) : n;
+      if (ilo >= ihi) continue;
+      const T* X = B + u_col[u0 + u1l] * ns;
+      const T* Y = B + (u_col[u0 + u2l] + w0) * ns;
+      const int64_t stride = MODE == 0 ? v.stride : d2;
+      T* out = MODE == 0 ? S + v.base : S + doff[v.r2] + w0 * d2;
+      if (ALL6 || (d1 == 6 && d2 == 6)) {
+        // products accumulated in the storage type: FP32 in the mixed form (the bulk of the arithmetic), FP64 otherwise
+        T acc[G][6];
 #pragma unroll
         for (int w = 0; w < G; ++w)
 #pragma unroll
-          for (int a = 0; a < 6; ++a) acc[w][a] += x[a] * y[w];
-      }
-#pragma unroll
-      for (int w = 0; w < G; ++w)
-#pragma unroll
-        for (int a = 0; a < 6; ++a)
-          if (MODE == 1 || !diag || a <= w0 + w) atomicAdd(out + w * stride + a, acc[w][a]);
-    } else if (!ALL6) {
-      for (int w = w0; w < d2 && w < w0 + G; ++w) {
-        double acc[16];
-#pragma unroll
-        for (int a = 0; a < 16; ++a) acc[a] = 0.0;
+          for (int a = 0; a < 6; ++a) acc[w][a] = T(0);
         for (int i = ilo; i < ihi; ++i) {
-          const double y = (double)Y[(w - w0) * ns + i];
+          T x[6], y[G];
+#pragma unroll
+          for (int a = 0; a < 6; ++a) x[a] = X[a * ns + i];
+#pragma unroll
+          for (int w = 0; w < G; ++w) y[w] = Y[w * ns + i];
+#pragma unroll
+          for (int w = 0; w < G; ++w)
+#pragma unroll
+            for (int a = 0; a < 6; ++a) acc[w][a] += x[a] * y[w];
+        }
+        if (MODE == 0 && sizeof(T) == 4) {
+#pragma unroll
+          for (int w = 0; w < G; ++w) {
+            T v[6];   // below the diagonal -0.0, which leaves every value unchanged
+#pragma unroll
+            for (int a = 0; a < 6; ++a) v[a] = !diag || a <= w0 + w ? acc[w][a] : T(-0.0);
+            red_column6(out + w * stride, v);
+          }
+        } else {
+#pragma unroll
+          for (int w = 0; w < G; ++w)
+#pragma unroll
+            for (int a = 0; a < 6; ++a)
+              if (MODE == 1 || !diag || a <= w0 + w) atomicAdd(out + w * stride + a, acc[w][a]);
+        }
+      } else if (!ALL6) {
+        for (int w = w0; w < d2 && w < w0 + G; ++w) {
+          double acc[16];
+#pragma unroll
+          for (int a = 0; a < 16; ++a) acc[a] = 0.0;
+          for (int i = ilo; i < ihi; ++i) {
+            const double y = (double)Y[(w - w0) * ns + i];
+#pragma unroll
+            for (int a = 0; a < 16; ++a)
+              if (a < d1) acc[a] += (double)X[a * ns + i] * y;
+          }
 #pragma unroll
           for (int a = 0; a < 16; ++a)
-            if (a < d1) acc[a] += (double)X[a * ns + i] * y;
+            if (a < d1 && (MODE == 1 || !diag || a <= w)) atomicAdd(out + (w - w0) * stride + a, T(acc[a]));
         }
-#pragma unroll
-        for (int a = 0; a < 16; ++a)
-          if (a < d1 && (MODE == 1 || !diag || a <= w)) atomicAdd(out + (w - w0) * stride + a, T(acc[a]));
       }
     }
+  };
+  if constexpr (WHOLE) {
+    if (whole) units(std::integral_constant<int, 6>{});
+    else units(std::integral_constant<int, 3>{});
+  } else {
+    units(std::integral_constant<int, 3>{});
   }
 }
 
@@ -933,34 +985,78 @@ __global__ void __launch_bounds__(256) k_jtj_quadform(int64_t nt, int64_t neb, i
   if (lane == 0 && part != 0.0) atomicAdd(total, part);
 }
 
-// qr_backsubstitute_group! (src/qr_reduced.jl:24-93): thread per eliminated table, FP64
-template <class T>
-__global__ void k_qr_backsub(int64_t ne_tab, const int32_t* __restrict__ t_rows, const int32_t* __restrict__ t_cols,
+// qr_backsubstitute_group! (src/qr_reduced.jl:24-93), FP64: eight lanes per eliminated table over its entries' columns, the
+// sums added up by shuffles, then U x_e = q - B x_r solved by one lane; MDE rows at a time from the last, so that a table
+// of any size keeps its sums in registers. 31,007 tables, FP64: 129 us with a thread per table, accumulating in x_e in
+// global memory, 41 us now; 3,000 tables: 87 us, 13 now.
+template <class T, int MDE>
+__global__ void __launch_bounds__(256) k_qr_backsub(int64_t ne_tab, const int32_t* __restrict__ t_rows, const int32_t* __restrict__ t_cols,
                              const int64_t* __restrict__ t_raw, const int64_t* __restrict__ t_res, const int32_t* __restrict__ t_ptr,
                              const int32_t* __restrict__ u_col, const int32_t* __restrict__ u_ret, const int32_t* __restrict__ r_dims,
                              const int32_t* __restrict__ boff_r, const int32_t* __restrict__ e_dims, const int32_t* __restrict__ boff_e,
-                             const T* __restrict__ F, const double* __restrict__ Fr, const double* __restrict__ x_r, double* __restrict__ x_e,
+                             const T* __restrict__ F, const double* __restrict__ Fr, const double* __restrict__ x_r, double* x_e,
                              const double* __restrict__ w = nullptr) {
-  const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (e >= ne_tab) return;
-  const int M = t_rows[e], C = t_cols[e], de = e_dims[e], ce = C - de - 1;
+  const int64_t e = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 3;
+  const int l = threadIdx.x & 7;
+  const unsigned group = 0xffu << (threadIdx.x & 24);
+  if (e >= ne_tab) return;   // whole groups
+  const int M = t_rows[e], de = e_dims[e], ce = t_cols[e] - de - 1;
   const int64_t off = t_raw[e];
-  // t = q - B x_r accumulated in x_e's own entries, then U x_e = t solved in place (the same operations in the same order);
-  // q is the factored residual's top rows, or the given w (a refinement step's U^-T d_e)
   double* xe = x_e + boff_e[e];
-  for (int i = 0; i < de; ++i) xe[i] = w ? w[boff_e[e] + i] : Fr[t_res[e] + i];
-  for (int u = t_ptr[e]; u < t_ptr[e + 1]; ++u) {
-    const int r = u_ret[u], ro = boff_r[r];
-    const T* cb = F + off + (int64_t)u_col[u] * M;
-    for (int j = 0; j < r_dims[r]; ++j) {
-      const double xj = x_r[ro + j];
-      for (int i = 0; i < de; ++i) xe[i] -= (double)cb[(int64_t)j * M + i] * xj;
+  constexpr bool ONE = MDE <= 4;   // no table is larger: one step
+  for (int i0 = ONE ? 0 : (de - 1) / MDE * MDE; i0 >= 0; i0 -= MDE) {
+    const int n = ONE ? de : (de - i0 < MDE ? de - i0 : MDE);
+    double t[MDE], U[MDE <= 4 ? MDE : 1][MDE <= 4 ? MDE : 1];
+    const T* Uc = F + off + (int64_t)(ce + i0) * M + i0;
+#pragma unroll
+    for (int i = 0; i < MDE; ++i) t[i] = 0.0;
+    if constexpr (MDE <= 4) {   // U's columns in flight with the rest
+#pragma unroll
+      for (int j = 0; j < MDE; ++j)
+#pragma unroll
+        for (int i = 0; i <= j; ++i) U[j][i] = j < n ? (double)Uc[(int64_t)j * M + i] : 1.0;
     }
-  }
-  for (int i = de - 1; i >= 0; --i) {
-    double acc = xe[i];
-    for (int j = i + 1; j < de; ++j) acc -= (double)F[off + (int64_t)(ce + j) * M + i] * xe[j];
-    xe[i] = acc / (double)F[off + (int64_t)(ce + i) * M + i];
+    for (int u = t_ptr[e]; u < t_ptr[e + 1]; ++u) {
+      const int r = u_ret[u], dr = r_dims[r], ro = boff_r[r];
+      const T* cb = F + off + (int64_t)u_col[u] * M + i0;
+      for (int j = l; j < dr; j += 8) {
+        const double xj = x_r[ro + j];
+#pragma unroll
+        for (int i = 0; i < MDE; ++i)
+          if (i < n) t[i] += (double)cb[(int64_t)j * M + i] * xj;
+      }
+    }
+    for (int j = n + l; !ONE && j < de - i0; j += 8) {   // the rows already solved
+      const double xj = xe[i0 + j];
+#pragma unroll
+      for (int i = 0; i < MDE; ++i)
+        if (i < n) t[i] += (double)Uc[(int64_t)j * M + i] * xj;
+    }
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1)
+#pragma unroll
+      for (int i = 0; i < MDE; ++i) t[i] += __shfl_xor_sync(group, t[i], o);
+    if (l == 0) {
+      // q is the factored residual's top rows, or the given w (a refinement step's U^-T d_e)
+#pragma unroll
+      for (int i = 0; i < MDE; ++i)
+        if (i < n) t[i] = (w ? w[boff_e[e] + i0 + i] : Fr[t_res[e] + i0 + i]) - t[i];
+#pragma unroll
+      for (int i = MDE - 1; i >= 0; --i)
+        if (i < n) {
+          double acc = t[i];
+#pragma unroll
+          for (int j = i + 1; j < MDE; ++j)
+            if (j < n) {
+              if constexpr (MDE <= 4) acc -= U[j][i] * t[j];
+              else acc -= (double)Uc[(int64_t)j * M + i] * t[j];
+            }
+          if constexpr (MDE <= 4) t[i] = acc / U[i][i];
+          else t[i] = acc / (double)Uc[(int64_t)i * M + i];
+          xe[i0 + i] = t[i];
+        }
+    }
+    if (!ONE) __syncwarp(group);   // the rows solved, for the next ones
   }
 }
 
@@ -1261,6 +1357,8 @@ static void check_jt_pattern(const QRPlan* P, int64_t nrows, int64_t ncols, cons
     }
 }
 
+constexpr int kLsmrChunk = 64 * 1024;   // bytes of tables (in FP64) that a CTA of k_lsmr_pass takes
+
 static QRPlan* qr_plan_create(bls_ctx* ctx, const bls_qr_plan_desc* d) {
   if (!d || d->nrblocks < 1 || d->neblocks < 1 || d->ntables < d->neblocks) throw Error(BLS_EINVAL, "a QR plan needs retained blocks, eliminated blocks and their tables");
   std::unique_ptr<QRPlan> P(new QRPlan());
@@ -1495,6 +1593,18 @@ static QRPlan* qr_plan_create(bls_ctx* ctx, const bls_qr_plan_desc* d) {
     upload(P->u_runpos, runpos, s);
     P->q_total.alloc(sizeof(double));
   }
+  {   // k_lsmr_pass's chunks: consecutive tables of at most kLsmrChunk bytes in FP64 (a larger table is a chunk of its own)
+    std::vector<int32_t> chunk;
+    int64_t lo = 0;
+    for (int64_t t = 0; t < nt; ++t)
+      if (t == 0 || 8 * (d->raw_offsets[t + 1] - lo) > kLsmrChunk) {
+        chunk.push_back((int32_t)t);
+        lo = d->raw_offsets[t];
+      }
+    P->ls_nchunks = (int64_t)chunk.size();
+    chunk.push_back((int32_t)nt);
+    upload(P->ls_chunk, chunk, s);
+  }
   upload(P->blk_stride, b_stride, s);
   upload(P->blk_base_sparse, b_base, s);
   upload(P->blk_base_dense, b_base_dense, s);
@@ -1592,7 +1702,10 @@ static void gram(QRPlan* P, T* S, bool dense, double* g, const T* F, const doubl
     if (k.n == 0) continue;
     cudaStream_t cs = class_stream(P, s, q++);
     const int64_t wb = ((std::is_same<T, double>::value ? k.bytes_f64 : k.bytes_f32) + 15) & ~int64_t(15);
-    auto kern = P->all6 ? k_qr_gram<T, MODE, true> : k_qr_gram<T, MODE, false>;
+    auto kern = P->all6 ? k_qr_gram<T, MODE, true, false> : k_qr_gram<T, MODE, false, false>;
+    // a table of 3 KB or more can have 16 pairs (5 entries of 6 columns by 10 rows)
+    if constexpr (std::is_same<T, float>::value && MODE == 0)
+      if (P->all6 && wb >= 3072) kern = k_qr_gram<T, MODE, true, true>;
     const int wpc = std::max(1, tables_per_cta(wb, 32, warp_cap(reinterpret_cast<const void*>(kern))));
     const size_t smem = (size_t)(wb * wpc);
     set_smem(reinterpret_cast<const void*>(kern), smem);
@@ -1686,34 +1799,9 @@ static void diagonal_blocks(QRPlan* P, T* D, const T* F) {
 // and the h update need). The vectors are FP64 on the device; the scalar recurrences of Fong & Saunders (SIAM J. Sci.
 // Comput. 33 (2011), LSMR with its estimates of ||r||, ||A'r||, ||A|| and cond(A)) run on the host.
 
-// The diagonal blocks of J~'J~ in FP64, straight from the factored tables, in two passes as reduced_tmul!: a thread
-// per (entry, column pair a <= b) forms the pair's dot product over the entry's reduced rows into
-// part[u * npair + b (b + 1) / 2 + a]; a warp per (retained block, pair) sums its entries in order into both triangles
-// of L's block (column-major, at doff).
-template <class T>
-__global__ void __launch_bounds__(256) k_lsmr_diag_entries(int64_t nent, int npair, const int4* __restrict__ meta,
-                                                           const int32_t* __restrict__ t_rows, const int32_t* __restrict__ t_top,
-                                                           const int64_t* __restrict__ t_raw, const T* __restrict__ F,
-                                                           double* __restrict__ part) {
-  const int64_t gid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (gid >= nent * npair) return;
-  const int64_t u = gid / npair;
-  const int p = (int)(gid - u * npair);
-  int b = (int)((sqrtf(8.0f * p + 1.0f) - 1.0f) * 0.5f);
-  while ((b + 1) * (b + 2) / 2 <= p) ++b;
-  while (b * (b + 1) / 2 > p) --b;
-  const int a = p - b * (b + 1) / 2;
-  const int4 q = meta[u];   // column, retained offset, retained size, table
-  if (b >= q.z) return;
-  const int t = q.w, M = t_rows[t], top = t_top[t], n = M - top;
-  const T* ca = F + t_raw[t] + (int64_t)(q.x + a) * M + top;
-  const T* cb = F + t_raw[t] + (int64_t)(q.x + b) * M + top;
-  double acc = 0.0;
-#pragma unroll 4
-  for (int i = 0; i < n; ++i) acc += (double)ca[i] * (double)cb[i];
-  part[gid] = acc;
-}
-
+// The diagonal blocks of J~'J~ in FP64: a warp per (retained block, pair of columns a <= b) sums its entries' parts
+// (part[entry * npair + b (b + 1) / 2 + a], formed by k_lsmr_pass) in order into both triangles of L's block (column-major,
+// at doff).
 __global__ void __launch_bounds__(256) k_lsmr_diag_reduce(int64_t nrb, int npair, const int32_t* __restrict__ rptr,
                                                           const int32_t* __restrict__ rent, const int32_t* __restrict__ r_dims,
                                                           const int64_t* __restrict__ doff, const double* __restrict__ part,
@@ -1736,7 +1824,8 @@ __global__ void __launch_bounds__(256) k_lsmr_diag_reduce(int64_t nrb, int npair
   }
 }
 
-// D_b + sqd^2 on its diagonal, then its Cholesky factor (lower, column-major) in place in L; a thread per block. A
+// D_b + sqd^2 on its diagonal, then the inverse of its Cholesky factor (lower, column-major) in place in L; a thread per
+// block. A
 // block that is not positive definite (or not finite) records the lowest such block in *bad.
 __global__ void k_lsmr_factor(int64_t nrb, const int32_t* __restrict__ r_dims, const int32_t* __restrict__ boff_r,
                               const int64_t* __restrict__ doff, const double* __restrict__ sqd, double* __restrict__ L,
@@ -1761,6 +1850,14 @@ __global__ void k_lsmr_factor(int64_t nrb, const int32_t* __restrict__ r_dims, c
       a[i + d * j] = q / ljj;
     }
   }
+  for (int j = 0; j < d; ++j) {   // column j of the inverse reads L's columns j and after only
+    a[j + d * j] = 1.0 / a[j + d * j];
+    for (int i = j + 1; i < d; ++i) {
+      double q = 0.0;
+      for (int k = j; k < i; ++k) q += a[i + d * k] * a[k + d * j];
+      a[i + d * j] = -q / a[i + d * i];
+    }
+  }
 }
 
 __device__ __forceinline__ void warp_sum_add(double v, double* out) {
@@ -1768,115 +1865,233 @@ __device__ __forceinline__ void warp_sum_add(double v, double* out) {
   if ((threadIdx.x & 31) == 0 && v != 0.0) atomicAdd(out, v);
 }
 
-// v = L^-1 (sc (w + sqd .* ub)) + gamma v, block by block (w is overwritten), and acc += |v|^2; a thread per block.
-// This is B' u - beta v with u = sc ub_raw: w = J~' u_top(raw), ub = the raw bottom of u.
-__global__ void k_lsmr_fwd(int64_t nrb, const int32_t* __restrict__ r_dims, const int32_t* __restrict__ boff_r,
-                           const int64_t* __restrict__ doff, const double* __restrict__ L, double* __restrict__ w,
-                           const double* __restrict__ sqd, const double* __restrict__ ub, double sc, double gamma,
-                           double* __restrict__ v, double* __restrict__ acc) {
-  const int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  double nn = 0.0;
-  if (b < nrb) {
-    const int d = r_dims[b], ro = boff_r[b];
-    const double* a = L + doff[b];
-    for (int i = 0; i < d; ++i) {
-      double q = sc * (w[ro + i] + sqd[ro + i] * ub[ro + i]);
-      for (int k = 0; k < i; ++k) q -= a[i + d * k] * w[ro + k];
-      w[ro + i] = q / a[i + d * i];
-    }
-    for (int i = 0; i < d; ++i) {
-      const double z = w[ro + i] + gamma * v[ro + i];
-      v[ro + i] = z;
-      nn += z * z;
-    }
+// *out += the block's sum, one atomic per CTA: atomics to one address complete about 1.8 ns apart here, so a norm's 24,000
+// warps alone would hold a pass over J~ for 43 us. Every thread of the block calls it.
+__device__ __forceinline__ void block_sum_add(double v, double* out) {
+  __shared__ double warps[16];
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if ((threadIdx.x & 31) == 0) warps[threadIdx.x >> 5] = v;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < (int)(blockDim.x >> 5); ++w) v += warps[w];
+    if (v != 0.0) atomicAdd(out, v);
   }
-  warp_sum_add(nn, acc);
 }
 
-// v *= sc, then t = L^-T v, block by block; a thread per block
-__global__ void k_lsmr_bwd(int64_t nrb, const int32_t* __restrict__ r_dims, const int32_t* __restrict__ boff_r,
-                           const int64_t* __restrict__ doff, const double* __restrict__ L, double sc, double* __restrict__ v,
+// v = L^-1 (w + sqd .* ub) / beta - beta vsc v with w = J~' u (the entries' parts, summed here) and ub the raw bottom of u:
+// B' u - beta v for u = u_raw / beta and v = vsc v_raw, where beta = |u_raw| is read from norms[0] (not positive or not
+// finite: nothing is written); norms[1] += |v|^2. A CTA per retained block: warp j sums the block's entries' parts in
+// column j, then a thread per variable applies L^-1 (kept in L's place).
+__global__ void __launch_bounds__(512) k_lsmr_reduce_fwd(int dmax, const int32_t* __restrict__ rptr, const int32_t* __restrict__ rent,
+                                                         const int32_t* __restrict__ r_dims, const int32_t* __restrict__ boff_r,
+                                                         const int64_t* __restrict__ doff, const double* __restrict__ Linv,
+                                                         const double* __restrict__ part, const double* __restrict__ sqd,
+                                                         const double* __restrict__ ub, double vsc, double* __restrict__ v,
+                                                         double* __restrict__ norms) {
+  __shared__ double q[16];
+  const double beta2 = norms[0];
+  if (!(beta2 > 0.0) || !isfinite(beta2)) return;   // uniform
+  const double beta = sqrt(beta2);
+  const int64_t r = blockIdx.x;
+  const int d = r_dims[r], ro = boff_r[r], lane = threadIdx.x & 31, j = threadIdx.x >> 5;
+  if (j < d) {
+    double s0 = 0.0, s1 = 0.0;
+    int k = rptr[r] + lane;
+    const int ke = rptr[r + 1];
+    for (; k + 32 < ke; k += 64) {
+      s0 += part[(int64_t)rent[k] * dmax + j];
+      s1 += part[(int64_t)rent[k + 32] * dmax + j];
+    }
+    if (k < ke) s0 += part[(int64_t)rent[k] * dmax + j];
+    s0 += s1;
+    for (int o = 16; o > 0; o >>= 1) s0 += __shfl_xor_sync(0xffffffffu, s0, o);
+    if (lane == 0) q[j] = (s0 + sqd[ro + j] * ub[ro + j]) / beta;
+  }
+  __syncthreads();
+  if (j > 0) return;
+  double nn = 0.0;
+  if (lane < d) {
+    const double* a = Linv + doff[r];
+    double z = 0.0;
+    for (int k = 0; k <= lane; ++k) z += a[lane + d * k] * q[k];
+    z -= beta * vsc * v[ro + lane];
+    v[ro + lane] = z;
+    nn = z * z;
+  }
+  warp_sum_add(nn, norms + 1);
+}
+
+// t = L^-T (sc v), a thread per variable (block, i < dmax)
+__device__ __forceinline__ double lsmr_bwd(const double* a, int d, int i, const double* v, double sc) {
+  double t = 0.0;
+  for (int k = i; k < d; ++k) t += a[k + d * i] * v[k];
+  return sc * t;
+}
+__global__ void k_lsmr_bwd(int64_t nrb, int dmax, const int32_t* __restrict__ r_dims, const int32_t* __restrict__ boff_r,
+                           const int64_t* __restrict__ doff, const double* __restrict__ Linv, double sc, const double* __restrict__ v,
                            double* __restrict__ t) {
-  const int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (b >= nrb) return;
-  const int d = r_dims[b], ro = boff_r[b];
-  const double* a = L + doff[b];
-  for (int i = 0; i < d; ++i) v[ro + i] *= sc;
-  for (int i = d - 1; i >= 0; --i) {
-    double q = v[ro + i];
-    for (int k = i + 1; k < d; ++k) q -= a[k + d * i] * t[ro + k];
-    t[ro + i] = q / a[i + d * i];
-  }
+  const int64_t id = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, b = id / dmax;
+  const int i = (int)(id - b * dmax);
+  if (b >= nrb || i >= r_dims[b]) return;
+  t[boff_r[b] + i] = lsmr_bwd(Linv + doff[b], r_dims[b], i, v + boff_r[b], sc);
 }
 
-// u = B t - a u with B t = [J~ t; sqd .* t] (a thread per row of u: a reduced row's product as reduced_mul! forms it,
-// then the damping rows), acc += |u|^2
-template <class T>
-__global__ void __launch_bounds__(256) k_lsmr_bv(int64_t mt, int64_t nr, const int32_t* __restrict__ red_tab,
-                                                 const int32_t* __restrict__ t_rows, const int32_t* __restrict__ t_top,
-                                                 const int64_t* __restrict__ t_raw, const int64_t* __restrict__ t_red,
-                                                 const int32_t* __restrict__ t_ptr, const int4* __restrict__ meta,
-                                                 const T* __restrict__ F, const double* __restrict__ sqd,
-                                                 const double* __restrict__ t, double a,
-                                                 double* __restrict__ u, double* __restrict__ acc) {
-  const int64_t row = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+// One pass over J~ for a solve's two products with it. A CTA takes a chunk of consecutive tables (QRPlan::ls_chunk: as many
+// as fit kLsmrChunk bytes), brings them into shared memory with one bulk copy (a table that does not fit, or an F off a
+// 16-byte boundary, is read where it is), and then
+//   INIT: forms per (entry, pair of columns) the parts of the diagonal blocks of J~'J~ (diag[entry * np + pair]);
+//   else: a thread per reduced row, u = J~ t - a u, acc += |u|^2; the CTAs past the chunks take the damping rows,
+//         u = sqd .* t - a u;
+// and a thread per (entry, column) forms the parts of J~' u (part[entry * dmax + column]). Every sum is FP64.
+// 31,007 tables (178 MB) in FP64: an iteration's two products 47 + 44 us and the start's 90 + 45 as kernels of their own
+// that read J~ from memory, 79 and 98 now; what is left are the chains of lookups from a row to its table, its entries and
+// their variables, several per CTA and only partly hidden by the other two CTAs of an SM. Chunks of 24, 32 and 48 KB, four
+// lanes per row and the first lookups before the wait are within 3% of this.
+template <class T, bool INIT>
+__global__ void __launch_bounds__(256) k_lsmr_pass(int nchunks, int64_t mt, int64_t nr, int dmax, const int32_t* __restrict__ chunk,
+                                                   const int32_t* __restrict__ red_tab, const int32_t* __restrict__ t_rows,
+                                                   const int32_t* __restrict__ t_cols, const int32_t* __restrict__ t_top,
+                                                   const int64_t* __restrict__ t_raw, const int64_t* __restrict__ t_red,
+                                                   const int32_t* __restrict__ t_ptr, const int4* __restrict__ meta,
+                                                   const T* __restrict__ F, const T* __restrict__ F_end, int room,
+                                                   const double* __restrict__ sqd, const double* __restrict__ t, double a, double* u,
+                                                   double* __restrict__ part, int np, double* __restrict__ diag, double* __restrict__ acc,
+                                                   long long* st) {
+  extern __shared__ __align__(16) unsigned char lsm[];
+  __shared__ __align__(8) uint64_t bar;
+  const int tid = threadIdx.x;
   double nn = 0.0;
-  if (row < mt) {
-    const int tb = red_tab[row];
-    const int M = t_rows[tb], top = t_top[tb];
-    const int64_t raw = t_raw[tb] + top + (row - t_red[tb]);
-    double y = 0.0;
-    for (int e = t_ptr[tb]; e < t_ptr[tb + 1]; ++e) {
-      const int4 q = meta[e];   // column, retained offset, retained size
-      const T* col = F + raw + (int64_t)q.x * M;
-      if (q.z == 6) {           // the common camera block: six independent loads in flight
-        T f[6];
-#pragma unroll
-        for (int j = 0; j < 6; ++j) f[j] = col[(int64_t)j * M];
-#pragma unroll
-        for (int j = 0; j < 6; ++j) y += (double)f[j] * t[q.y + j];
-      } else {
-        for (int j = 0; j < q.z; ++j) y += (double)col[(int64_t)j * M] * t[q.y + j];
-      }
+  if ((int)blockIdx.x >= nchunks) {
+    const int64_t i = ((int64_t)blockIdx.x - nchunks) * 256 + tid;
+    if (i < nr) {
+      const double z = sqd[i] * t[i] - a * u[mt + i];
+      u[mt + i] = z;
+      nn = z * z;
     }
-    const double z = y - a * u[row];
-    u[row] = z;
-    nn = z * z;
-  } else if (row < mt + nr) {
-    const double z = sqd[row - mt] * t[row - mt] - a * u[row];
-    u[row] = z;
-    nn = z * z;
+    block_sum_add(nn, acc);
+    return;
   }
-  warp_sum_add(nn, acc);
+  const int ta = chunk[blockIdx.x], tl = chunk[blockIdx.x + 1] - 1;
+  const int64_t raw0 = t_raw[ta], len = t_raw[tl] + (int64_t)t_rows[tl] * (t_cols[tl] - 1) - raw0;
+  const T* base = F + raw0;   // the chunk's first entry, in shared memory when it was staged
+  const int64_t e0 = t_ptr[ta], ne = t_ptr[tl + 1] - e0;
+  int64_t row = 0, r1 = 0, x_off = 0;   // the thread's row, the chunk's end, the row's place in it
+  int M_row = 0, e_lo = 0, e_hi = 0;
+  int4 q_row = make_int4(0, 0, 0, 0);
+  auto find_row = [&] {
+    const int tb = red_tab[row];
+    M_row = t_rows[tb];
+    x_off = (t_raw[tb] - raw0) + t_top[tb] + (row - t_red[tb]);
+    e_lo = t_ptr[tb];
+    e_hi = t_ptr[tb + 1];
+    if (e_lo < e_hi) q_row = meta[e_lo];
+  };
+  const bool staged = len * (int64_t)sizeof(T) + 32 <= room;
+  if (staged) {
+    const Span sp = span_of(F + raw0, len, F_end);
+    base = span_first(reinterpret_cast<T*>(lsm), sp);
+    if (tid == 0) {
+      mbar_init(&bar, 1);
+      mbar_fence_init();
+      mbar_arrive_expect_tx(&bar, span_bytes(sp));
+      span_issue(reinterpret_cast<T*>(lsm), sp, &bar);
+    }
+  }
+  if (!INIT) {   // the first row's lookups run while the tables are in flight
+    row = t_red[ta] + tid;
+    r1 = t_red[tl] + (t_rows[tl] - t_top[tl]);
+    if (row < r1) find_row();
+  }
+  if (staged) {
+    __syncthreads();   // the barrier is initialised
+    const bool ok = mbar_wait(&bar, 0);
+    if (__syncthreads_or(!ok)) {   // a copy that did not land: a fault, as in the table kernels; the host sees a norm that is not finite
+      if (tid == 0) {
+        atomicExch(reinterpret_cast<unsigned long long*>(st + 2), 1ull);
+        atomicAdd(acc, (double)NAN);
+      }
+      mbar_wait(&bar, 0);
+      return;
+    }
+  }
+  if (INIT) {
+    for (int64_t id = tid; id < ne * np; id += 256) {
+      const int64_t e = e0 + id / np;
+      const int p = (int)(id % np);
+      int cb = (int)((sqrtf(8.0f * p + 1.0f) - 1.0f) * 0.5f);
+      while ((cb + 1) * (cb + 2) / 2 <= p) ++cb;
+      while (cb * (cb + 1) / 2 > p) --cb;
+      const int ca = p - cb * (cb + 1) / 2;
+      const int4 q = meta[e];   // column, retained offset, retained size, table
+      if (cb >= q.z) continue;
+      const int tb = q.w, M = t_rows[tb], top = t_top[tb], rows = M - top;
+      const T* x = base + (t_raw[tb] - raw0) + (int64_t)(q.x + ca) * M + top;
+      const T* y = x + (int64_t)(cb - ca) * M;
+      double s = 0.0;
+#pragma unroll 4
+      for (int i = 0; i < rows; ++i) s += (double)x[i] * (double)y[i];
+      diag[e * np + p] = s;
+    }
+  } else {
+    while (row < r1) {
+      const T* x = base + x_off;
+      double y = 0.0;
+      for (int e = e_lo; e < e_hi; ++e) {
+        const int4 q = e == e_lo ? q_row : meta[e];
+        const T* col = x + (int64_t)q.x * M_row;
+        if (q.z == 6) {   // the common camera block: six independent loads in flight
+          T f[6];
+#pragma unroll
+          for (int j = 0; j < 6; ++j) f[j] = col[(int64_t)j * M_row];
+#pragma unroll
+          for (int j = 0; j < 6; ++j) y += (double)f[j] * t[q.y + j];
+        } else {
+          for (int j = 0; j < q.z; ++j) y += (double)col[(int64_t)j * M_row] * t[q.y + j];
+        }
+      }
+      const double z = y - a * u[row];
+      u[row] = z;
+      nn += z * z;
+      row += 256;
+      if (row < r1) find_row();
+    }
+    block_sum_add(nn, acc);   // its barrier also orders the chunk's u
+  }
+  for (int64_t id = tid; id < ne * dmax; id += 256) {
+    const int64_t e = e0 + id / dmax;
+    const int j = (int)(id % dmax);
+    const int4 q = meta[e];
+    if (j >= q.z) continue;
+    const int tb = q.w, M = t_rows[tb], top = t_top[tb], rows = M - top;
+    const T* col = base + (t_raw[tb] - raw0) + (int64_t)(q.x + j) * M + top;
+    const double* ur = u + t_red[tb];
+    double s = 0.0;
+#pragma unroll 4
+    for (int i = 0; i < rows; ++i) s += (double)col[i] * ur[i];
+    part[e * dmax + j] = s;
+  }
 }
 
-// One iteration's end, a thread per block: v *= sc, t = L^-T v, then for the block's entries hbar = h - c1 hbar,
-// x += c2 hbar, h = t - c3 h; acc += |x|^2
-__global__ void k_lsmr_bwd_update(int64_t nrb, const int32_t* __restrict__ r_dims, const int32_t* __restrict__ boff_r,
-                                  const int64_t* __restrict__ doff, const double* __restrict__ L, double sc, double* __restrict__ v,
+// One iteration's end, a thread per variable: t = L^-T (sc v), hbar = h - c1 hbar, x += c2 hbar, h = t - c3 h; acc += |x|^2
+__global__ void k_lsmr_bwd_update(int64_t nrb, int dmax, const int32_t* __restrict__ r_dims, const int32_t* __restrict__ boff_r,
+                                  const int64_t* __restrict__ doff, const double* __restrict__ Linv, double sc, const double* __restrict__ v,
                                   double* __restrict__ t, double* __restrict__ h, double* __restrict__ hbar, double* __restrict__ x,
                                   double c1, double c2, double c3, double* __restrict__ acc) {
-  const int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const int64_t id = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, b = id / dmax;
+  const int k = (int)(id - b * dmax);
   double nn = 0.0;
-  if (b < nrb) {
-    const int d = r_dims[b], ro = boff_r[b];
-    const double* a = L + doff[b];
-    for (int i = 0; i < d; ++i) v[ro + i] *= sc;
-    for (int i = d - 1; i >= 0; --i) {
-      double q = v[ro + i];
-      for (int k = i + 1; k < d; ++k) q -= a[k + d * i] * t[ro + k];
-      t[ro + i] = q / a[i + d * i];
-    }
-    for (int i = ro; i < ro + d; ++i) {
-      const double hb = h[i] - c1 * hbar[i];
-      hbar[i] = hb;
-      const double xi = x[i] + c2 * hb;
-      x[i] = xi;
-      h[i] = t[i] - c3 * h[i];
-      nn += xi * xi;
-    }
+  if (b < nrb && k < r_dims[b]) {
+    const int i = boff_r[b] + k;
+    const double ti = lsmr_bwd(Linv + doff[b], r_dims[b], k, v + boff_r[b], sc);
+    t[i] = ti;
+    const double hb = h[i] - c1 * hbar[i];
+    hbar[i] = hb;
+    const double xi = x[i] + c2 * hb;
+    x[i] = xi;
+    h[i] = ti - c3 * h[i];
+    nn = xi * xi;
   }
-  warp_sum_add(nn, acc);
+  block_sum_add(nn, acc);
 }
 
 // sqd = sqrt(lambda s_r) (s_r NULL: sqrt(lambda)); u's bottom rows zero; acc[0] += |r~|^2 (u's top, already written)
@@ -1891,7 +2106,17 @@ __global__ void k_lsmr_init(int64_t mt, int64_t nr, double lambda, const double*
       u[i] = 0.0;
     }
   }
-  warp_sum_add(nn, acc);
+  block_sum_add(nn, acc);
+}
+
+template <class T>
+static void launch_qr_backsub(QRPlan* P, const T* F, const double* Fr, const double* x_r, double* x_e, const double* w) {
+  if (P->neblocks == 0) return;
+  auto kern = P->max_de <= 4 ? k_qr_backsub<T, 4> : k_qr_backsub<T, 16>;
+  kern<<<(unsigned)grid_for(8 * P->neblocks, 256), 256, 0, P->ctx->stream>>>(
+      P->neblocks, P->t_rows.as<int32_t>(), P->t_cols.as<int32_t>(), P->t_raw.as<int64_t>(), P->t_res.as<int64_t>(), P->t_ptr.as<int32_t>(),
+      P->u_col.as<int32_t>(), P->u_ret.as<int32_t>(), P->r_dims.as<int32_t>(), P->boff_r.as<int32_t>(), P->e_dims.as<int32_t>(),
+      P->boff_e.as<int32_t>(), F, Fr, x_r, x_e, w);
 }
 
 struct LsmrOut {
@@ -1909,7 +2134,7 @@ static int lsmr_reduced(QRPlan* P, const T* F, const double* Fr, double lambda, 
   const int64_t mt = P->red_nrows, nr = P->nr, nrb = P->nrblocks, m = mt + nr;
   if (!P->ls_u.p) {
     P->ls_u.alloc(sizeof(double) * (size_t)std::max<int64_t>(m, 1));
-    for (DevBuf* b : {&P->ls_v, &P->ls_h, &P->ls_hbar, &P->ls_t, &P->ls_w, &P->ls_sqd})
+    for (DevBuf* b : {&P->ls_v, &P->ls_h, &P->ls_hbar, &P->ls_t, &P->ls_sqd})
       b->alloc(sizeof(double) * (size_t)std::max<int64_t>(nr, 1));
     P->ls_L.alloc(sizeof(double) * (size_t)std::max<int64_t>(P->ndiag, 1));
     P->ls_acc.alloc(sizeof(double) * 4);
@@ -1917,7 +2142,7 @@ static int lsmr_reduced(QRPlan* P, const T* F, const double* Fr, double lambda, 
     BLS_CUDA(cudaMallocHost(reinterpret_cast<void**>(&P->ls_host), sizeof(double) * 4));
   }
   double *u = P->ls_u.as<double>(), *v = P->ls_v.as<double>(), *h = P->ls_h.as<double>();
-  double *hbar = P->ls_hbar.as<double>(), *t = P->ls_t.as<double>(), *w = P->ls_w.as<double>(), *sqd = P->ls_sqd.as<double>();
+  double *hbar = P->ls_hbar.as<double>(), *t = P->ls_t.as<double>(), *sqd = P->ls_sqd.as<double>();
   double *L = P->ls_L.as<double>(), *acc = P->ls_acc.as<double>(), *hv = P->ls_host;
   int* flag = P->ls_flag.as<int>();
   const int32_t *rd = P->r_dims.as<int32_t>(), *bo = P->boff_r.as<int32_t>();
@@ -1937,44 +2162,69 @@ static int lsmr_reduced(QRPlan* P, const T* F, const double* Fr, double lambda, 
     k_reduced_residual<<<(unsigned)std::max(1, grid_for(P->ntables * 32, 256)), 256, 0, s>>>(
         P->ntables, P->t_rows.as<int32_t>(), P->t_top.as<int32_t>(), P->t_res.as<int64_t>(), P->t_red.as<int64_t>(), Fr, u);
   k_lsmr_init<<<gm, 256, 0, s>>>(mt, nr, lambda, s_r, sqd, u, acc);
+  if (P->rdmax == 0)
+    for (int64_t d : P->h_rdims) P->rdmax = std::max<int>(P->rdmax, (int)d);
+  const int dm = std::max(P->rdmax, 1), np = dm * (dm + 1) / 2;
+  const size_t need = sizeof(double) * (size_t)std::max<int64_t>(P->nentries * np, 1);
+  if (P->ls_part.bytes < need) P->ls_part.alloc(need);
+  const size_t part_bytes = sizeof(double) * (size_t)std::max<int64_t>(P->nentries * dm, 1);
+  if (P->tm_part.bytes < part_bytes) P->tm_part.alloc(part_bytes);
+  double* part = P->tm_part.as<double>();
+  // the start's pass (diagonal blocks and J~' r~) and an iteration's
+  auto pass = [&](auto init, double a) {
+    constexpr bool INIT = decltype(init)::value;
+    const int room = P->bulk && (reinterpret_cast<uintptr_t>(F) & 15) == 0 ? kLsmrChunk / 8 * (int)sizeof(T) + 32 : 0;
+    auto kern = k_lsmr_pass<T, INIT>;
+    if (room > 48 * 1024) BLS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, room));
+    kern<<<(unsigned)(P->ls_nchunks + (INIT ? 0 : (nr + 255) / 256)), 256, room, s>>>(
+        (int)P->ls_nchunks, mt, nr, dm, P->ls_chunk.as<int32_t>(), P->red_tab.as<int32_t>(), P->t_rows.as<int32_t>(),
+        P->t_cols.as<int32_t>(), P->t_top.as<int32_t>(), P->t_raw.as<int64_t>(), P->t_red.as<int64_t>(), P->t_ptr.as<int32_t>(),
+        P->u_meta.as<int4>(), F, F + P->raw_len, room, sqd, t, a, u, part, np, P->ls_part.as<double>(), acc,
+        P->status.as<long long>());
+    P->launches += 1;
+  };
+  auto not_finite = [&]() -> int {   // a bulk copy that did not land poisons the norms: an error of its own
+    long long st = QNONE;
+    BLS_CUDA(cudaMemcpyAsync(&st, P->status.as<long long>() + 2, sizeof(st), cudaMemcpyDeviceToHost, s));
+    BLS_CUDA(cudaStreamSynchronize(s));
+    if (st != QNONE) throw Error(BLS_ECUDA, "a bulk copy of a table did not complete within its wait limit");
+    return BLS_NOT_PD;
+  };
   {
-    if (P->rdmax == 0)
-      for (int64_t d : P->h_rdims) P->rdmax = std::max<int>(P->rdmax, (int)d);
-    const int np = std::max(P->rdmax, 1) * (std::max(P->rdmax, 1) + 1) / 2;
-    const size_t need = sizeof(double) * (size_t)std::max<int64_t>(P->nentries * np, 1);
-    if (P->ls_part.bytes < need) P->ls_part.alloc(need);
     BLS_CUDA(cudaMemsetAsync(L, 0, sizeof(double) * (size_t)P->ndiag, s));   // blocks without entries stay zero
-    if (P->nentries > 0)
-      k_lsmr_diag_entries<T><<<(unsigned)grid_for(P->nentries * np, 256), 256, 0, s>>>(
-          P->nentries, np, P->u_meta.as<int4>(), P->t_rows.as<int32_t>(), P->t_top.as<int32_t>(), P->t_raw.as<int64_t>(), F,
-          P->ls_part.as<double>());
+    if (P->nentries > 0) pass(std::true_type(), (double)0);
     k_lsmr_diag_reduce<<<(unsigned)std::max(1, grid_for(nrb * np * 32, 256)), 256, 0, s>>>(
         nrb, np, P->q_rptr.as<int32_t>(), P->q_rent.as<int32_t>(), rd, doff, P->ls_part.as<double>(), L);
   }
   k_lsmr_factor<<<gb, 128, 0, s>>>(nrb, rd, bo, doff, sqd, L, flag);
-  P->launches += 4 + (mt > 0);
+  P->launches += 3 + (mt > 0);
   BLS_CUDA(cudaGetLastError());
   BLS_CUDA(cudaMemcpyAsync(hv, acc, sizeof(double), cudaMemcpyDeviceToHost, s));
   int bad = 0;
   BLS_CUDA(cudaMemcpyAsync(&bad, flag, sizeof(int), cudaMemcpyDeviceToHost, s));
   BLS_CUDA(cudaStreamSynchronize(s));
   const double bb = hv[0];
-  if (!std::isfinite(bb)) return BLS_NOT_PD;          // a non-finite reduced residual
+  if (!std::isfinite(bb)) return not_finite();        // a non-finite reduced residual
   if (lambda == 0 && mt < nr) return BLS_NOT_PD;      // undamped with fewer reduced rows than variables: rank deficient
   if (bad != 0x7f7f7f7f) return BLS_NOT_PD;           // a diagonal block of A'A is not positive definite
   double beta = std::sqrt(bb);
   out->normr = beta;
   if (nr == 0 || beta == 0) return BLS_OK;            // x = 0 solves it
-  // alpha v = B' u with u = u_raw / beta; t = L^-T v; h = t
-  BLS_CUDA(cudaMemsetAsync(acc, 0, sizeof(double) * 4, s));
+  // alpha v = B' u with u = u_raw / beta (|u_raw|^2 is in acc[0]); t = L^-T v; h = t
+  const unsigned gv = (unsigned)std::max<int64_t>(1, grid_for(nrb * dm, 128));
+  double vsc = 0.0;   // v = vsc v_raw
+  auto forward = [&] {
+    k_lsmr_reduce_fwd<<<(unsigned)nrb, 32 * dm, 0, s>>>(dm, P->q_rptr.as<int32_t>(), P->q_rent.as<int32_t>(), rd, bo, doff, L, part, sqd, u + mt,
+                                                        vsc, v, acc);
+    P->launches += 1;
+  };
   BLS_CUDA(cudaMemsetAsync(v, 0, sizeof(double) * (size_t)nr, s));
   BLS_CUDA(cudaMemsetAsync(hbar, 0, sizeof(double) * (size_t)nr, s));
-  launch_reduced_tmul<T>(P, F, u, w);
-  k_lsmr_fwd<<<gb, 128, 0, s>>>(nrb, rd, bo, doff, L, w, sqd, u + mt, 1.0 / beta, 0.0, v, acc + 1);
-  P->launches += 1;
+  forward();
   read(2);
   double alpha = std::sqrt(hv[1]);
-  k_lsmr_bwd<<<gb, 128, 0, s>>>(nrb, rd, bo, doff, L, alpha > 0 ? 1.0 / alpha : 1.0, v, t);
+  vsc = alpha > 0 ? 1.0 / alpha : 1.0;
+  k_lsmr_bwd<<<gv, 128, 0, s>>>(nrb, dm, rd, bo, doff, L, vsc, v, t);
   P->launches += 1;
   BLS_CUDA(cudaMemcpyAsync(h, t, sizeof(double) * (size_t)nr, cudaMemcpyDeviceToDevice, s));
   double uscale = 1.0 / beta;   // u = uscale * u_raw
@@ -2018,13 +2268,12 @@ static int lsmr_reduced(QRPlan* P, const T* F, const double* Fr, double lambda, 
   };
   bool pending = false;
   for (;;) {
-    // u_raw = B v - alpha u
+    // u_raw = B v - alpha u and J~' u_raw, then v_raw = B' u - beta v for u = u_raw / |u_raw|: the host reads |u_raw|,
+    // |v_raw| and the last iteration's |x| together
     if (itn < itmax) {
       BLS_CUDA(cudaMemsetAsync(acc, 0, sizeof(double) * 2, s));
-      k_lsmr_bv<T><<<(unsigned)grid_for(m, 256), 256, 0, s>>>(
-          mt, nr, P->red_tab.as<int32_t>(), P->t_rows.as<int32_t>(), P->t_top.as<int32_t>(), P->t_raw.as<int64_t>(),
-          P->t_red.as<int64_t>(), P->t_ptr.as<int32_t>(), P->u_meta.as<int4>(), F, sqd, t, alpha * uscale, u, acc);
-      P->launches += 1;
+      pass(std::false_type(), alpha * uscale);
+      forward();
     }
     read(3);
     if (pending) {
@@ -2034,20 +2283,15 @@ static int lsmr_reduced(QRPlan* P, const T* F, const double* Fr, double lambda, 
     }
     ++itn;
     beta = std::sqrt(hv[0]);
-    if (!std::isfinite(beta)) return BLS_NOT_PD;
+    if (!std::isfinite(beta)) return not_finite();
     if (beta > 0) {
       uscale = 1.0 / beta;
-      // v_raw = B' u - beta v, alpha = |v_raw|, v = v_raw / alpha, t = L^-T v
-      launch_reduced_tmul<T>(P, F, u, w);
-      k_lsmr_fwd<<<gb, 128, 0, s>>>(nrb, rd, bo, doff, L, w, sqd, u + mt, uscale, -beta, v, acc + 1);
-      P->launches += 1;
-      read(2);
       alpha = std::sqrt(hv[1]);
       if (!std::isfinite(alpha)) return BLS_NOT_PD;
+      vsc = alpha > 0 ? 1.0 / alpha : 1.0;
     } else {
-      uscale = 0.0;
+      uscale = 0.0;   // v unchanged: t is recomputed as it is
     }
-    const double vscale = beta > 0 && alpha > 0 ? 1.0 / alpha : 1.0;   // v unchanged when beta = 0: t is recomputed as is
     // the plane rotations (no regularisation in LSMR itself: the damping rows are part of A)
     const double alphahat = alphabar;
     const double rhoold = rho;
@@ -2063,7 +2307,7 @@ static int lsmr_reduced(QRPlan* P, const T* F, const double* Fr, double lambda, 
     zetabar = -sbar * zetabar;
     // hbar = h - (thetabar rho / (rhoold rhobarold)) hbar; x += (zeta / (rho rhobar)) hbar; h = t - (thetanew / rho) h
     BLS_CUDA(cudaMemsetAsync(acc + 2, 0, sizeof(double), s));
-    k_lsmr_bwd_update<<<gb, 128, 0, s>>>(nrb, rd, bo, doff, L, vscale, v, t, h, hbar, x, thetabar * rho / (rhoold * rhobarold),
+    k_lsmr_bwd_update<<<gv, 128, 0, s>>>(nrb, dm, rd, bo, doff, L, vsc, v, t, h, hbar, x, thetabar * rho / (rhoold * rhobarold),
                                          zeta / (rho * rhobar), thetanew / rho, acc + 2);
     P->launches += 1;
     // ||r||: the rotations applied to (betadd, betad) and the running tau
@@ -2194,19 +2438,9 @@ int bls_qr_backsubstitute_rhs(bls_qr_plan* P, int dtype, const void* F, const do
   QR_GUARD({
     if (!P || !F || !w || !x_r || !x_e) throw Error(BLS_EINVAL, "a device pointer is NULL");
     cudaStream_t s = P->ctx->stream;
-    const unsigned grid = (unsigned)std::max<int64_t>(1, grid_for(P->neblocks, 128));
-    if (dtype == BLS_F64)
-      k_qr_backsub<double><<<grid, 128, 0, s>>>(P->neblocks, P->t_rows.as<int32_t>(), P->t_cols.as<int32_t>(), P->t_raw.as<int64_t>(),
-                                               P->t_res.as<int64_t>(), P->t_ptr.as<int32_t>(), P->u_col.as<int32_t>(), P->u_ret.as<int32_t>(),
-                                               P->r_dims.as<int32_t>(), P->boff_r.as<int32_t>(), P->e_dims.as<int32_t>(), P->boff_e.as<int32_t>(),
-                                               (const double*)F, nullptr, x_r, x_e, w);
-    else if (dtype == BLS_F32)
-      k_qr_backsub<float><<<grid, 128, 0, s>>>(P->neblocks, P->t_rows.as<int32_t>(), P->t_cols.as<int32_t>(), P->t_raw.as<int64_t>(),
-                                              P->t_res.as<int64_t>(), P->t_ptr.as<int32_t>(), P->u_col.as<int32_t>(), P->u_ret.as<int32_t>(),
-                                              P->r_dims.as<int32_t>(), P->boff_r.as<int32_t>(), P->e_dims.as<int32_t>(), P->boff_e.as<int32_t>(),
-                                              (const float*)F, nullptr, x_r, x_e, w);
-    else
-      throw Error(BLS_EINVAL, "unknown dtype");
+    if (dtype == BLS_F64) launch_qr_backsub<double>(P, (const double*)F, nullptr, x_r, x_e, w);
+    else if (dtype == BLS_F32) launch_qr_backsub<float>(P, (const float*)F, nullptr, x_r, x_e, w);
+    else throw Error(BLS_EINVAL, "unknown dtype");
     P->launches += 1;
     BLS_CUDA(cudaGetLastError());
     return BLS_OK;
@@ -2245,18 +2479,8 @@ int64_t bls_qr_plan_counters(bls_qr_plan* P) {
 int bls_qr_backsubstitute(bls_qr_plan* P, int dtype, double* x_e, const double* x_r, const void* F, const double* Fr) {
   QR_GUARD({
     cudaStream_t s = P->ctx->stream;
-    if (dtype == BLS_F64)
-      k_qr_backsub<double><<<grid_for(P->neblocks, 128), 128, 0, s>>>(P->neblocks, P->t_rows.as<int32_t>(), P->t_cols.as<int32_t>(),
-                                                                     P->t_raw.as<int64_t>(), P->t_res.as<int64_t>(), P->t_ptr.as<int32_t>(),
-                                                                     P->u_col.as<int32_t>(), P->u_ret.as<int32_t>(), P->r_dims.as<int32_t>(),
-                                                                     P->boff_r.as<int32_t>(), P->e_dims.as<int32_t>(), P->boff_e.as<int32_t>(),
-                                                                     (const double*)F, Fr, x_r, x_e);
-    else if (dtype == BLS_F32)
-      k_qr_backsub<float><<<grid_for(P->neblocks, 128), 128, 0, s>>>(P->neblocks, P->t_rows.as<int32_t>(), P->t_cols.as<int32_t>(),
-                                                                    P->t_raw.as<int64_t>(), P->t_res.as<int64_t>(), P->t_ptr.as<int32_t>(),
-                                                                    P->u_col.as<int32_t>(), P->u_ret.as<int32_t>(), P->r_dims.as<int32_t>(),
-                                                                    P->boff_r.as<int32_t>(), P->e_dims.as<int32_t>(), P->boff_e.as<int32_t>(),
-                                                                    (const float*)F, Fr, x_r, x_e);
+    if (dtype == BLS_F64) launch_qr_backsub<double>(P, (const double*)F, Fr, x_r, x_e, nullptr);
+    else if (dtype == BLS_F32) launch_qr_backsub<float>(P, (const float*)F, Fr, x_r, x_e, nullptr);
     else throw Error(BLS_EINVAL, "unknown dtype");
     P->launches += 1;
     BLS_CUDA(cudaGetLastError());
