@@ -23,11 +23,12 @@ constexpr int TS = NB + 2;  // row stride of a tile in shared memory (16-byte ro
 struct DenseSolver {
   bls_ctx* ctx = nullptr;
   int64_t n = 0, ld = 0;   // ld: n rounded up to whole tiles, the order and leading dimension of W
-  DevBuf W;        // ld x ld FP64, column-major; L in its lower triangle after a successful factorisation
-  DevBuf rows;     // the 64 rows below the next diagonal tile, two buffers
-  DevBuf inv16;    // per panel the inverses of its diagonal tile's four 16 x 16 diagonal blocks (column-major)
-  DevBuf inv;      // per panel the inverse of its 64 x 64 diagonal tile (column-major), for the solve
-  DevBuf status;   // [0]: first failing column (0-based) or -1
+  DevBuf mem;      // what follows, in one allocation (a solver's creation and destruction cost what its allocations do)
+  double* W = nullptr;        // ld x ld FP64, column-major; L in its lower triangle after a successful factorisation
+  double* rows = nullptr;     // the 64 rows below the next diagonal tile, two buffers
+  double* inv16 = nullptr;    // per panel the inverses of its diagonal tile's four 16 x 16 diagonal blocks (column-major)
+  double* inv = nullptr;      // per panel the inverse of its 64 x 64 diagonal tile (column-major), for the solve
+  long long* status = nullptr;   // [0]: first failing column (0-based) or -1
   bool factored = false;
   // The diagonal tiles run on one high-priority stream, the panels below them and the updates they wait for on another,
   // while the rest of a group's update runs on the caller's stream (created at the first factorisation).
@@ -39,7 +40,7 @@ struct DenseSolver {
   // factorisation; the panel kernels carry the high priority as a launch attribute, so the graph keeps it.
   cudaStream_t cap_stream = nullptr;
   cudaGraphExec_t factor_graph = nullptr;
-  DevBuf y;               // the solve's exchange: ld forward and ld backward values, all bits set until written
+  double* y = nullptr;    // the solve's exchange: ld forward and ld backward values, all bits set until written
   int solve_grid = 0;     // resident CTAs of k_solve (set at the first solve)
   ~DenseSolver() {
     if (factor_graph) cudaGraphExecDestroy(factor_graph);
@@ -601,14 +602,14 @@ static void launch_prio(void (*kernel)(Args...), dim3 grid, unsigned block, size
 // updates that the next panels wait for on u, the rest of each group's update on s, joined on s.
 static void launch_factor_body(DenseSolver* D, cudaStream_t s, cudaStream_t p) {
   const int64_t ld = D->ld, nt = ld / NB;
-  double* W = D->W.as<double>();
-  double* v16 = D->inv16.as<double>();
-  double* inv = D->inv.as<double>();
-  long long* st = D->status.as<long long>();
+  double* W = D->W;
+  double* v16 = D->inv16;
+  double* inv = D->inv;
+  long long* st = D->status;
   const long long* cst = st;
   const int prio = D->panel_priority;
   cudaStream_t u = D->update_stream;
-  double* rows = D->rows.as<double>();   // two buffers, by the parity of the panel
+  double* rows = D->rows;   // two buffers, by the parity of the panel
   double* none = nullptr;
   auto then = [](cudaStream_t from, cudaEvent_t ev, cudaStream_t to) {
     BLS_CUDA(cudaEventRecord(ev, from));
@@ -662,8 +663,8 @@ static int factor(DenseSolver* D, const T* S, double lambda, const double* s_r, 
   if (!S) throw Error(BLS_EINVAL, "S is NULL");
   cudaStream_t s = D->ctx->stream;
   const int64_t n = D->n;
-  double* W = D->W.as<double>();
-  long long* st = D->status.as<long long>();
+  double* W = D->W;
+  long long* st = D->status;
   if (!D->panel_stream) {
     int lo = 0, hi = 0;
     BLS_CUDA(cudaDeviceGetStreamPriorityRange(&lo, &hi));
@@ -737,11 +738,14 @@ int bls_dense_solver_create(bls_ctx* ctx, int64_t n, bls_dense_solver** out) {
     D->ctx = ctx;
     D->n = n;
     D->ld = (n + NB - 1) / NB * NB;
-    D->W.alloc(sizeof(double) * (size_t)(D->ld * D->ld));
-    D->rows.alloc(sizeof(double) * 2 * NB * NB);
-    D->inv16.alloc(sizeof(double) * 16 * (size_t)D->ld);
-    D->inv.alloc(sizeof(double) * NB * (size_t)D->ld);
-    D->status.alloc(sizeof(long long));
+    const size_t w = (size_t)(D->ld * D->ld), r = 2 * NB * NB, v16 = 16 * (size_t)D->ld, v = NB * (size_t)D->ld, y = 2 * (size_t)D->ld;
+    D->mem.alloc(sizeof(double) * (w + r + v16 + v + y) + sizeof(long long));   // every part a multiple of 128 doubles
+    D->W = D->mem.as<double>();
+    D->rows = D->W + w;
+    D->inv16 = D->rows + r;
+    D->inv = D->inv16 + v16;
+    D->y = D->inv + v;
+    D->status = reinterpret_cast<long long*>(D->y + y);
     *out = D.release();
     return BLS_OK;
   })
@@ -777,7 +781,7 @@ int bls_dense_cholesky_solve(bls_dense_solver* D, const double* g, double* x) {
     if (!D || !g || !x) throw Error(BLS_EINVAL, "null argument");
     if (!D->factored) throw Error(BLS_EINVAL, "the solver holds no factorisation (bls_dense_cholesky first, and it must succeed)");
     const int64_t n = D->n;
-    const double* W = D->W.as<double>();
+    const double* W = D->W;
     cudaStream_t s = D->ctx->stream;
     // the tiles' CTAs must be resident at once (256 at the largest n)
     const int64_t nt = D->ld / NB;
@@ -787,13 +791,12 @@ int bls_dense_cholesky_solve(bls_dense_solver* D, const double* g, double* x) {
       BLS_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
       BLS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_solve, 256, 0));
       if (nt > (int64_t)nsm * per_sm) throw Error(BLS_EUNSUPPORTED, "the device is too small for this system's solve");
-      D->y.alloc(sizeof(double) * 2 * (size_t)D->ld);
       D->solve_grid = (int)nt;
     }
-    double* y = D->y.as<double>();
+    double* y = D->y;
     BLS_CUDA(cudaMemsetAsync(y, 0xff, sizeof(double) * 2 * (size_t)D->ld, s));
     int64_t n_arg = n, ld_arg = D->ld;
-    const double* inv = D->inv.as<double>();
+    const double* inv = D->inv;
     void* args[] = {&n_arg, &ld_arg, &W, &inv, &g, &x, &y};
     BLS_CUDA(cudaLaunchCooperativeKernel((const void*)k_solve, dim3((unsigned)D->solve_grid), dim3(256), args, 0, s));
     BLS_CUDA(cudaGetLastError());
