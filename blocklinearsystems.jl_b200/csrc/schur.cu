@@ -14,7 +14,10 @@
 // A call then runs:
 //   phase 1  k_factor   one thread per point: the damped d_e x d_e inverse in FP64 (closed forms of
 //                        src/kernels.jl:14-67, same pivot tests), z = E^-1 (s_e .* b_e) in FP64;
-//   phase 2  k_pairs    one thread per work item: sum over its pairs of C_c1' (E^-1 C_c2), the 6x6 block in
+//   phase 2  column-owned, the default: k_runs / k_runs_any (column_runs.cuh) or k_stage36 form a block column of S and its
+//                        part of g_S per CTA; the block-owned lists serve the host-buffer call, C off a 16-byte
+//                        boundary and plans without a column-owned schedule:
+//            k_pairs    one thread per work item: sum over its pairs of C_c1' (E^-1 C_c2), the 6x6 block in
 //                        registers, then one plain read-modify-write of S when the block has a single item, else
 //                        atomic adds (one per block entry per item, not per pair);
 //            k_gradient one warp per retained block: g_S = s_r .* b_r - sum C' z over its couplings.
@@ -107,7 +110,7 @@ struct SchurPlan {
   int64_t nprob = 0;
   std::vector<int64_t> prob_point_off, prob_row_off, prob_nnz_off;
   DevBuf prob_fail, prob_of_point, prob_of_cam;
-  int kernel = 1;   // 0: column-owned (k_columns36), 1: block-owned pairs (k_pairs36, the default: faster on sparse scenes)
+  int kernel = 1;   // bls_schur_plan_set_kernel's number; 5 where the plan has a column-owned schedule
   // reset
   DevBuf r_to_s, diag_inds, S_rowval, S_col;
   // one-pass reset (k_reset_columns): per S entry the R entry it takes or -1, and S's column pointers; used when

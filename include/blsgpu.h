@@ -190,11 +190,15 @@ int bls_reset_reduce_schur_sparse_host(bls_schur_plan* plan, int dtype, void* S_
  * reduction on the plan's stream. bls_schur_plan_counters synchronises on the last event, reports the device kernel
  * launches issued since the previous read, the summed pair-kernel time and its number of launches, and resets them. */
 int bls_schur_plan_instrument(bls_schur_plan* plan, int timing);
-/* Phase-2 kernel of the d_r = 6 / d_e = 3 fast path (no counterpart in the reference): 0 = block-column owned,
- * 1 = block owned, six lanes per pair list (the default), 2 = block owned, a lane per pair and a warp per pair list,
- * 3 = block-column owned with visits staged in chunks (sparse S without conditioning scales; otherwise as 1),
- * 4 = point-major, six lanes per pair, entries added into S with vector reductions (as 1 when S has 2^25 or more
- * blocks). All compute the same reduction; the choice is kept for comparisons and for autotuning. */
+/* Phase-2 kernel (no counterpart in the reference) of plans of 6-variable retained and 3-variable eliminated blocks (any
+ * other plan takes the runs, 6, where it has them, whatever is chosen): 0 = block-column owned, 1 = block owned, six lanes
+ * per pair list (the default of a plan with neither 6 nor 7), 2 = block owned, a lane per pair and a warp per pair list, 3 = block-column owned with
+ * visits staged in chunks (sparse S without conditioning scales; otherwise as 1), 4 = point-major, six lanes per pair,
+ * entries added into S with vector reductions (as 1 when S has 2^25 or more blocks), 5 = block-column owned, the faster
+ * of 6 and 7 for the plan's columns and storage type (6 for a dense S; the default), 6 = block-column owned with the couplings of a
+ * column's points staged as contiguous runs, 7 = block-column owned with the point operands of a column staged and the
+ * couplings gathered (sparse S; otherwise as 1). All compute the same reduction; the choice is kept for comparisons and
+ * for autotuning. */
 int bls_schur_plan_set_kernel(bls_schur_plan* plan, int which);
 /* No counterpart in the reference (a tuning knob of this build's schedule): rebuild the column-owned schedule (which = 5)
  * with units of at most `unit` pairs for both storage types (1..4096; at plan creation 20 for FP32 storage and 16 for
