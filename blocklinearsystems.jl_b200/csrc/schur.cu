@@ -2302,16 +2302,25 @@ static SchurPlan* plan_create(bls_ctx* ctx, const bls_schur_plan_desc* d) {
     if (gather) {
       // k_runs against k_stage36 for a sparse S of 6 x 6 blocks (against the block-owned pairs it is ahead everywhere).
       // k_stage36 keeps a column's point operands in shared memory for the whole column and adds a block to its tile
-      // once, so it is ahead where columns are long and there are enough of them; k_runs, whose items are parts of
-      // columns, is ahead on short or few columns and, in FP32, on long ones of few blocks. us, k_stage36 / k_runs, FP32 and FP64: 1000 cameras of 1200 visits and 61 blocks 320 / 250 and 401 /
-      // 461; 10,000 of 766 and 121 1553 / 1760; 3000 of 766 and 121 483 / 590 and 933 / 1165; 300 of 583 and 57 44 / 51
-      // and 79 / 86; 200 of 345 and 31 34 / 28 and 38 / 40; 1500 of 200 and 121 127 / 87 and 160 / 150; 3000 of 200 and
-      // 41 303 / 131 and 325 / 219; 40 of 1100 and 40 54 / 25 and 48 / 34.
+      // once; k_runs brings in every coupling of a point before the visit's, and adds a block once per segment. So the
+      // number of couplings per point times the number of blocks per column decides, with the visits per column (few: a
+      // column is no work for a CTA of k_stage36; above ~1000 in FP32, its items are cut) and the number of columns (few
+      // do not fill k_stage36's CTAs; in FP64 some hundreds fill those better than k_runs's). us, k_stage36 / k_runs, by
+      // visits, blocks and couplings per point; 1,000 to 1,500 cameras where nothing is said:
+      //   FP32  350, 127, 5: 169 / 131      450, 31, 8: 142 / 126      450, 112, 8: 138 / 151     450, 113, 12: 156 / 197
+      //         600, 31, 5: 210 / 167       600, 118, 8 (6,000): 820 / 933      600, 38, 8 (300): 50 / 62
+      //         700, 40, 8: 181 / 187       766, 121, 7.7 (10,000): 1553 / 1760         850, 40, 5: 236 / 224
+      //         850, 87, 5: 229 / 236       1200, 61, 6: 320 / 250      1300, 113, 8: 372 / 367 1300, 114, 12: 487 / 489
+      //   FP64  200, 121, 5: 160 / 150      350, 40, 5: 194 / 170       350, 85, 5: 192 / 208   450, 31, 8: 248 / 216
+      //         600, 31, 5: 332 / 255       600, 31, 8 (6,000): 1467 / 1390     600, 38, 8 (300): 94 / 108
+      //         700, 40, 8: 345 / 343       1200, 61, 6: 401 / 461      1300, 31, 8: 626 / 565  1300, 113, 8: 561 / 652
       int64_t cols = 0;
       for (int64_t r = 0; r < nrb; ++r) cols += rptr[r + 1] > rptr[r];
-      const double visits = cols ? (double)nc / cols : 0.0, blocks = (double)nb / nrb;
-      P->runs_first[0] = !(visits >= 512 && cols >= 148 && (blocks >= 90 || visits < 900));
-      P->runs_first[1] = !(visits >= 300 && cols >= 148);
+      const double visits = cols ? (double)nc / cols : 0.0;
+      const double kb = neb ? (double)nc / neb * ((double)nb / nrb) : 0.0;   // couplings per point x blocks per column
+      const bool filled = cols >= 148, wide = filled && visits >= 200 && kb >= 800;
+      P->runs_first[0] = !(wide || (filled && visits >= 400 && visits < 1000 && kb >= 300));
+      P->runs_first[1] = !(wide || (filled && visits >= 300 && (kb >= 250 || cols < 400)));
     }
     // a plan of 6 x 6 blocks for a sparse S builds per storage type the schedule that "stage" takes (the other one when it
     // cannot be built, or when it is chosen by name: ensure_gather, ensure_runs); every other plan has the runs only
