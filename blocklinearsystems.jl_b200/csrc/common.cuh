@@ -2,7 +2,11 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <cstdint>
+#include <mutex>
+#include <set>
 #include <string>
+#include <utility>
+#include <vector>
 
 #include "host_layout.hpp"
 
@@ -61,6 +65,24 @@ __device__ __forceinline__ void red_column6(double* col, const double v[6]) {
   for (int i = 0; i < 6; ++i) atomicAdd(col + i, v[i]);
 }
 #endif
+
+// Allows the launches of `kernel` all the dynamic shared memory that a CTA can have beside the kernel's static part. The
+// limit is an attribute of the kernel, process-wide: set to one launch's own size, it could be lowered by another host
+// thread's smaller launch before this one's larger launch, which is then refused. So it is set once per device, to the
+// most that any launch may ask for.
+inline void allow_smem(const void* kernel) {
+  static std::mutex mu;
+  static std::set<std::pair<const void*, int>> done;
+  int dev = 0, most = 0;
+  BLS_CUDA(cudaGetDevice(&dev));
+  std::lock_guard<std::mutex> lock(mu);
+  if (done.count({kernel, dev})) return;
+  cudaFuncAttributes a;
+  BLS_CUDA(cudaFuncGetAttributes(&a, kernel));
+  BLS_CUDA(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+  BLS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)a.sharedSizeBytes));
+  done.insert({kernel, dev});
+}
 
 inline int grid_for(int64_t n, int threads) { return (int)((n + threads - 1) / threads); }
 

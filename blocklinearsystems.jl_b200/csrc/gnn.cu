@@ -563,7 +563,7 @@ static void lin_fwd(GNNPlan* G, int K1, const IN1* in1, int K2, const A* in2, co
     }
   }
   const size_t smem = sizeof(float) * O * (K1 + K2);
-  if (smem > 48 * 1024) BLS_CUDA(cudaFuncSetAttribute(k_lin_fwd<A, IN1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (smem > 48 * 1024) allow_smem(reinterpret_cast<const void*>(k_lin_fwd<A, IN1>));
   k_lin_fwd<A, IN1><<<grid_for(G->n * O, 256), 256, smem, s>>>(G->n, K1, in1, K2, in2, W1, W2, b, O, relu, outA, outF);
   G->pcg->launches += 1;
 }

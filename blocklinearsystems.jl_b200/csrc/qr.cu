@@ -149,7 +149,7 @@ static int tables_per_cta(int64_t table_bytes, int G, int max_warps) {
 }
 
 static void set_smem(const void* kernel, size_t bytes) {
-  if (bytes > 48 * 1024) BLS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+  if (bytes > 48 * 1024) allow_smem(kernel);
 }
 
 // Fork the plan's side streams off s (they wait for all work issued on s so far); class q of a run of per-class

@@ -2641,7 +2641,7 @@ static void launch_runs(SchurPlan* P, T* S, bool dense, double* g, const T* C, c
     case 9: kern = k_runs<T, 9, F32 ? 9 : 3>; break;
     default: kern = R.mdr <= 9 ? k_runs_any<T, 9, F32 ? 9 : 5> : k_runs_any<T, 16, F32 ? 8 : 4>;
   }
-  BLS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, R.smem));
+  allow_smem(reinterpret_cast<const void*>(kern));
   if (R.grid == 0) {
     int per_sm = 0, nsm = 0, dev = 0;
     BLS_CUDA(cudaGetDevice(&dev));
@@ -2814,7 +2814,7 @@ static int reduce(SchurPlan* P, T* S, bool dense, double* g, const double* b_r, 
     const SchurPlan::StageSchedule& SS = P->stage[sizeof(T) == 4 ? 0 : 1];
     if (SS.items > 0) {
       const size_t smem = stage_smem<T>(P->max_col_h, SS.max_nv);
-      BLS_CUDA(cudaFuncSetAttribute(k_stage36<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      allow_smem(reinterpret_cast<const void*>(k_stage36<T>));
       if (ev0) BLS_CUDA(cudaEventRecord(ev0, s));
       P->launches += 1;
       if (P->stage_grid[sizeof(T) == 4 ? 0 : 1] == 0) {
@@ -2839,7 +2839,7 @@ static int reduce(SchurPlan* P, T* S, bool dense, double* g, const double* b_r, 
     const size_t smem = sizeof(StageSz) * 8 + sizeof(T) * 6 * hmax;
     if (smem > 200 * 1024) throw Error(BLS_EUNSUPPORTED, "a block column of S exceeds the shared-memory tile of this build");
     auto kern = dense ? k_columns36<T, true> : k_columns36<T, false>;
-    BLS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allow_smem(reinterpret_cast<const void*>(kern));
     if (ev0) BLS_CUDA(cudaEventRecord(ev0, s));
     P->launches += 1;
     kern<<<(int)P->nrblocks, 256, smem, s>>>(P->retained_ptr.as<int32_t>(), P->vis_rec.as<int2>(), P->vis_base.as<int32_t>(),
@@ -2852,7 +2852,7 @@ static int reduce(SchurPlan* P, T* S, bool dense, double* g, const double* b_r, 
     const size_t fixed = sizeof(double) * 32 * 3 + sizeof(double) * 8 * 6 + sizeof(TE) * 32 * 12 + sizeof(T) * 8 * 20 + sizeof(int) * (32 * 5 + 4) + 16;
     const size_t smem = fixed + sizeof(T) * cap + sizeof(T) * 6 * P->max_col_h;
     if (smem > 200 * 1024) throw Error(BLS_EUNSUPPORTED, "a block column of S exceeds the shared-memory tile of this build");
-    BLS_CUDA(cudaFuncSetAttribute(k_tiles36<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allow_smem(reinterpret_cast<const void*>(k_tiles36<T>));
     if (ev0) BLS_CUDA(cudaEventRecord(ev0, s));
     P->launches += 1;
     k_tiles36<T><<<(int)P->nrblocks, 256, smem, s>>>(P->retained_ptr.as<int32_t>(), P->vis_rec.as<int2>(), P->vis_base.as<int32_t>(),
