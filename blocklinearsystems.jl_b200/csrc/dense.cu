@@ -337,6 +337,13 @@ __global__ void __launch_bounds__(256, 1) k_step(int64_t ld, double* __restrict_
   for (int k = 0; k < 4; ++k) inv16[d0 * 16 + tid + 256 * k] = (&s.p.V[0][0][0])[tid + 256 * k];
 }
 
+// Whether a pivot has failed, as thread 0 sees it (false in every other thread). k_step runs beside the kernels that ask
+// and may record its failure at any time: threads that each read the word could disagree, and some would leave before a
+// barrier that the others wait at. A kernel asks once and decides for the whole CTA by __syncthreads_or.
+__device__ __forceinline__ bool stopped(const long long* status) {
+  return threadIdx.x == 0 && *reinterpret_cast<const volatile long long*>(status) >= 0;
+}
+
 // Copies the 64 rows below tile 0 for the first k_step.
 __global__ void __launch_bounds__(256) k_first_rows(int64_t ld, const double* __restrict__ W, double* __restrict__ rows) {
 #pragma unroll
@@ -351,8 +358,8 @@ __global__ void __launch_bounds__(256) k_trsm_panel(int64_t ld, double* __restri
                                                     double* __restrict__ inv, int64_t k0, const long long* __restrict__ status) {
   extern __shared__ __align__(16) unsigned char dense_smem[];
   PanelSmem& s = *reinterpret_cast<PanelSmem*>(dense_smem);
-  if (status[0] >= 0) return;
   const int tid = threadIdx.x;
+  const bool stop = stopped(status);
   const bool rows = blockIdx.x + 1 < gridDim.x;
   const int64_t row0 = k0 + NB + (int64_t)blockIdx.x * NB;
 #pragma unroll
@@ -365,7 +372,7 @@ __global__ void __launch_bounds__(256) k_trsm_panel(int64_t ld, double* __restri
   for (int k = 0; k < 4; ++k) cp_async8(&s.V[0][0][0] + tid + 256 * k, inv16 + k0 * 16 + tid + 256 * k);
   run_cp_commit();
   run_cp_wait<0>();
-  __syncthreads();
+  if (__syncthreads_or(stop)) return;
   if (!rows) {
     tile_inverse(s, inv, k0, tid);
     return;
@@ -394,11 +401,11 @@ __global__ void __launch_bounds__(256, AHEAD ? 3 : MT == 128 ? 2 : 4) k_syrk(int
   constexpr int KC = 16, RM = MT / 16, ST = AHEAD ? 4 : 3;   // RM: rows a thread holds
   extern __shared__ __align__(16) unsigned char dense_smem[];
   double* ring = reinterpret_cast<double*>(dense_smem);
-  if (status[0] >= 0) return;
   const int64_t bj = j0 + NB * (int64_t)blockIdx.y, bi = j0 + MT * (int64_t)blockIdx.x;
   if (bi + MT <= bj) return;   // above the diagonal
   if (AHEAD && blockIdx.x == 0 && blockIdx.y == 0) return;   // the next diagonal tile is k_step's
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  const bool stop = stopped(status);
   const int nch = K / KC;
   auto A = [&](int ch) { return reinterpret_cast<double (*)[MT]>(ring + (ch % ST) * KC * (MT + NB)); };
   auto B = [&](int ch) { return reinterpret_cast<double (*)[NB]>(ring + (ch % ST) * KC * (MT + NB) + KC * MT); };
@@ -439,6 +446,10 @@ __global__ void __launch_bounds__(256, AHEAD ? 3 : MT == 128 ? 2 : 4) k_syrk(int
     for (int p = 0; p < RM; ++p)
 #pragma unroll
       for (int q = 0; q < 4; ++q) out[p][q] = is_out(p, q) ? W[out_row(p) + ld * out_col(q)] : 0.0;
+  }
+  if (__syncthreads_or(stop)) {   // the panels are useless from the failing column on
+    run_cp_wait<0>();
+    return;
   }
   for (int ch = 0; ch < nch; ++ch) {
     run_cp_wait<ST - 2 + (AHEAD ? 1 : 0)>();

@@ -1,0 +1,28 @@
+"""A pivot that fails while panels and updates of the same factorisation run beside it, on other streams: the kernels that
+read the failure word decide for a whole CTA at once, the failing column is the first one, and the solver is usable
+afterwards. Tolerance 1e-10 relative as in test_gpu_dense.py."""
+import numpy as np
+import pytest
+import torch
+
+from test_gpu_dense import relerr
+from test_gpu_dense_tiles import spd
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n", [130, 700, 1500])
+def test_failure_beside_running_updates(bls, n):
+    A, rng = spd(n, 11)
+    D = bls.DenseCholesky(n)
+    S = torch.from_numpy(np.triu(A).ravel(order="F")).to("cuda").view(n, n)
+    diag = torch.diagonal(S)
+    g = rng.standard_normal(n)
+    for column in sorted(rng.choice(n, 40, replace=False)):
+        good = diag[column].item()
+        diag[column] = -5.0
+        assert not D.factor(S.view(-1)) and D.failed_column == column + 1
+        diag[column] = good
+        assert D.factor(S.view(-1)) and D.failed_column == 0
+        x = D.solve(torch.from_numpy(g).to("cuda"))
+    assert relerr(x.cpu().numpy(), np.linalg.solve(A, g)) <= 1e-10
