@@ -20,6 +20,8 @@ constexpr int NB = 64;      // panel width and tile size
 constexpr int GROUP = 4;    // panels per group
 constexpr int TS = NB + 2;  // row stride of a tile in shared memory (16-byte rows)
 
+constexpr int64_t kWaitLimit = 1 << 22;   // some seconds
+
 struct DenseSolver {
   bls_ctx* ctx = nullptr;
   int64_t n = 0, ld = 0;   // ld: n rounded up to whole tiles, the order and leading dimension of W
@@ -28,7 +30,8 @@ struct DenseSolver {
   double* rows = nullptr;     // the 64 rows below the next diagonal tile, two buffers
   double* inv16 = nullptr;    // per panel the inverses of its diagonal tile's four 16 x 16 diagonal blocks (column-major)
   double* inv = nullptr;      // per panel the inverse of its 64 x 64 diagonal tile (column-major), for the solve
-  long long* status = nullptr;   // [0]: first failing column (0-based) or -1
+  long long* status = nullptr;   // [0]: first failing column (0-based) or -1; [1]: 1 after a solve whose wait gave up
+  int64_t wait_limit = kWaitLimit;   // polls of a value before a wait of the solve gives up
   bool factored = false;
   // The diagonal tiles run on one high-priority stream, the panels below them and the updates they wait for on another,
   // while the rest of a group's update runs on the caller's stream (created at the first factorisation).
@@ -497,16 +500,19 @@ __global__ void __launch_bounds__(256, AHEAD ? 3 : MT == 128 ? 2 : 4) k_syrk(int
 // L L' x = g in one cooperative launch, CTA b owning the 64 rows of tile b. Forward: it takes y_k of every earlier tile in
 // order (polling it: each value is 8 bytes, all bits set until it is written), subtracts L[b, k] y_k from its rows, then
 // multiplies them by the inverse of its diagonal tile and posts y_b. Backward the same from the last tile up with L'. A
-// tile's 64 x 64 block of L is loaded before its poll. A poll that gives up passes NaNs on (nothing waits for ever).
+// tile's 64 x 64 block of L is loaded before its poll. A poll that gives up after `limit` tries
+// raises the fault word, which the next synchronising call reports, and passes NaNs on, so that nothing waits for ever.
 // n = 6000: 1.8 ms as two launches per tile with a substitution by one warp in each, 0.29 ms now.
 constexpr unsigned long long kUnwritten = ~0ull;
-__device__ __forceinline__ double poll_value(const double* p) {
+__device__ __forceinline__ double poll_value(const double* p, int64_t limit, long long* fault) {
   unsigned long long v = kUnwritten;
-  for (int i = 0; i < (1 << 22); ++i) {
+  for (int64_t i = 0; i < limit; ++i) {
     asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
     if (v != kUnwritten) break;
   }
-  return v == kUnwritten ? __longlong_as_double(0x7ff8000000000000ll) : __longlong_as_double((long long)v);
+  if (v != kUnwritten) return __longlong_as_double((long long)v);
+  asm volatile("st.relaxed.gpu.global.u64 [%0], 1;" ::"l"(fault) : "memory");
+  return __longlong_as_double(0x7ff8000000000000ll);
 }
 __device__ __forceinline__ void post_value(double* p, double v) {
   unsigned long long b = (unsigned long long)__double_as_longlong(v);
@@ -515,7 +521,7 @@ __device__ __forceinline__ void post_value(double* p, double v) {
 }
 
 __global__ void __launch_bounds__(256) k_solve(int64_t n, int64_t ld, const double* __restrict__ W, const double* __restrict__ inv,
-                                               const double* g, double* x, double* y) {
+                                               const double* g, double* x, double* y, int64_t limit, long long* fault) {
   __shared__ double rt[NB];   // the tile's current right-hand side
   __shared__ double xk[NB];
   __shared__ double part[4][NB];
@@ -540,7 +546,7 @@ __global__ void __launch_bounds__(256) k_solve(int64_t n, int64_t ld, const doub
   };
   for (int k = 0; k < b; ++k) {
     load(W + row0 + ld * NB * (int64_t)k, ld);
-    if (tid < NB) xk[tid] = poll_value(yf + NB * (int64_t)k + tid);
+    if (tid < NB) xk[tid] = poll_value(yf + NB * (int64_t)k + tid, limit, fault);
     __syncthreads();
     const double v = mul(xk);
     if (q == 0) rt[r] -= v;
@@ -578,7 +584,7 @@ __global__ void __launch_bounds__(256) k_solve(int64_t n, int64_t ld, const doub
   for (int k = nt - 1; k > b; --k) {
     load_t(W + NB * (int64_t)k + ld * row0, ld);
     __syncthreads();   // every thread has read the previous xk (first: rt is written)
-    if (tid < NB) xk[tid] = poll_value(yb + NB * (int64_t)k + tid);
+    if (tid < NB) xk[tid] = poll_value(yb + NB * (int64_t)k + tid, limit, fault);
     __syncthreads();
     const double v = mul_t(xk);
     if (lane < 8) rt[8 * warp + lane] -= v;
@@ -669,6 +675,13 @@ static void launch_factor_body(DenseSolver* D, cudaStream_t s, cudaStream_t p) {
   then(u, D->ev_update, s);
 }
 
+// An earlier solve's fault word as read back: cleared and raised as an error.
+static void report_fault(DenseSolver* D, long long fault) {
+  if (fault == 0) return;
+  BLS_CUDA(cudaMemsetAsync(D->status + 1, 0, sizeof(long long), D->ctx->stream));
+  throw Error(BLS_ECUDA, "a wait of an earlier solve did not complete within its limit: that solve's x is not valid");
+}
+
 template <class T>
 static int factor(DenseSolver* D, const T* S, double lambda, const double* s_r, int64_t* failed_column) {
   if (!S) throw Error(BLS_EINVAL, "S is NULL");
@@ -714,12 +727,13 @@ static int factor(DenseSolver* D, const T* S, double lambda, const double* s_r, 
   }
   BLS_CUDA(cudaGraphLaunch(D->factor_graph, s));
   BLS_CUDA(cudaGetLastError());
-  long long h = -1;
-  BLS_CUDA(cudaMemcpyAsync(&h, st, sizeof(long long), cudaMemcpyDeviceToHost, s));
+  long long h[2] = {-1, 0};
+  BLS_CUDA(cudaMemcpyAsync(h, st, sizeof(h), cudaMemcpyDeviceToHost, s));
   BLS_CUDA(cudaStreamSynchronize(s));
-  D->factored = h < 0;
-  if (failed_column) *failed_column = h < 0 ? 0 : h + 1;
-  return h < 0 ? BLS_OK : BLS_NOT_PD;
+  D->factored = h[0] < 0;
+  if (failed_column) *failed_column = h[0] < 0 ? 0 : h[0] + 1;
+  report_fault(D, h[1]);
+  return h[0] < 0 ? BLS_OK : BLS_NOT_PD;
 }
 
 }  // namespace bls
@@ -750,13 +764,14 @@ int bls_dense_solver_create(bls_ctx* ctx, int64_t n, bls_dense_solver** out) {
     D->n = n;
     D->ld = (n + NB - 1) / NB * NB;
     const size_t w = (size_t)(D->ld * D->ld), r = 2 * NB * NB, v16 = 16 * (size_t)D->ld, v = NB * (size_t)D->ld, y = 2 * (size_t)D->ld;
-    D->mem.alloc(sizeof(double) * (w + r + v16 + v + y) + sizeof(long long));   // every part a multiple of 128 doubles
+    D->mem.alloc(sizeof(double) * (w + r + v16 + v + y) + 2 * sizeof(long long));   // every part a multiple of 128 doubles
     D->W = D->mem.as<double>();
     D->rows = D->W + w;
     D->inv16 = D->rows + r;
     D->inv = D->inv16 + v16;
     D->y = D->inv + v;
     D->status = reinterpret_cast<long long*>(D->y + y);
+    BLS_CUDA(cudaMemsetAsync(D->status, 0, 2 * sizeof(long long), ctx->stream));
     *out = D.release();
     return BLS_OK;
   })
@@ -808,11 +823,29 @@ int bls_dense_cholesky_solve(bls_dense_solver* D, const double* g, double* x) {
     BLS_CUDA(cudaMemsetAsync(y, 0xff, sizeof(double) * 2 * (size_t)D->ld, s));
     int64_t n_arg = n, ld_arg = D->ld;
     const double* inv = D->inv;
-    void* args[] = {&n_arg, &ld_arg, &W, &inv, &g, &x, &y};
+    long long* fault = D->status + 1;
+    void* args[] = {&n_arg, &ld_arg, &W, &inv, &g, &x, &y, &D->wait_limit, &fault};
     BLS_CUDA(cudaLaunchCooperativeKernel((const void*)k_solve, dim3((unsigned)D->solve_grid), dim3(256), args, 0, s));
     BLS_CUDA(cudaGetLastError());
     return BLS_OK;
   })
+}
+
+int bls_dense_solver_check(bls_dense_solver* D) {
+  DENSE_GUARD({
+    if (!D) throw Error(BLS_EINVAL, "solver is NULL");
+    long long fault = 0;
+    BLS_CUDA(cudaMemcpyAsync(&fault, D->status + 1, sizeof(fault), cudaMemcpyDeviceToHost, D->ctx->stream));
+    BLS_CUDA(cudaStreamSynchronize(D->ctx->stream));
+    report_fault(D, fault);
+    return BLS_OK;
+  })
+}
+
+int bls_dense_solver_set_wait_limit(bls_dense_solver* D, int64_t polls) {
+  if (!D || polls < 1 || polls > kWaitLimit) return BLS_EINVAL;
+  D->wait_limit = polls;
+  return BLS_OK;
 }
 
 }  // extern "C"

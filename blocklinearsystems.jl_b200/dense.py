@@ -50,10 +50,15 @@ class DenseCholesky:
         return rc != BLS_NOT_PD
 
     def solve(self, g: torch.Tensor, x: torch.Tensor | None = None) -> torch.Tensor:
-        """x = S^-1 g from the last successful factor()."""
+        """x = S^-1 g from the last successful factor(). Does not synchronise; see check()."""
         _dev(g, "g", self.n, torch.float64)
         if x is None:
             x = torch.empty_like(g)
         _dev(x, "x", self.n, torch.float64)
         check(_lib.gpu().bls_dense_cholesky_solve(self.handle, dptr(g), dptr(x)))
         return x
+
+    def check(self) -> None:
+        """Synchronise and raise BlsError when a solve() since the last check() or factor() gave up one of its bounded
+        waits on the device (its x is not valid); the next factor() raises it too."""
+        check(_lib.gpu().bls_dense_solver_check(self.handle))

@@ -478,12 +478,18 @@ int bls_pcg_solve_refined(bls_pcg_plan* plan, bls_schur_plan* schur, int dtype, 
  * 312-320): a solver for n x n systems (n <= 16384) owning an FP64 working matrix. bls_dense_cholesky reads S
  * (dtype, column-major, its upper triangle: reduce_schur_dense!'s output) and factors it as L L' in FP64; a pivot that
  * is not positive returns BLS_NOT_PD with failed_column = its column, 1-based. bls_dense_cholesky_solve: x = S^-1 g
- * (FP64 device vectors) from the last successful factorisation. */
+ * (FP64 device vectors) from the last successful factorisation, without synchronising. Its tiles wait for one another
+ * on the device, each wait bounded; where one gives up, x is not valid and the next bls_dense_cholesky,
+ * bls_dense_cholesky_shifted or bls_dense_solver_check on the solver returns BLS_ECUDA, once (the factorisation that
+ * reports it has been done all the same). bls_dense_solver_check synchronises. bls_dense_solver_set_wait_limit: the
+ * polls of a wait before it gives up, 1 to 2^22 (some seconds, the default). */
 typedef struct bls_dense_solver bls_dense_solver;
 int bls_dense_solver_create(bls_ctx* ctx, int64_t n, bls_dense_solver** out);
 int bls_dense_solver_destroy(bls_dense_solver* solver);
 int bls_dense_cholesky(bls_dense_solver* solver, int dtype, const void* S_dev, int64_t* failed_column);
 int bls_dense_cholesky_solve(bls_dense_solver* solver, const double* g_dev, double* x_dev);
+int bls_dense_solver_check(bls_dense_solver* solver);
+int bls_dense_solver_set_wait_limit(bls_dense_solver* solver, int64_t polls);
 
 /* The same factorisation of S + lambda diag(s_r) (s_r a device vector of n FP64 entries, added to the diagonal in FP64
  * as S is read): the damped reduced normal equations of the QR route, J~'J~ from bls_reduced_normal_dense plus

@@ -26,3 +26,29 @@ def test_failure_beside_running_updates(bls, n):
         assert D.factor(S.view(-1)) and D.failed_column == 0
         x = D.solve(torch.from_numpy(g).to("cuda"))
     assert relerr(x.cpu().numpy(), np.linalg.solve(A, g)) <= 1e-10
+
+
+def test_a_wait_that_gives_up_is_reported(bls):
+    """With one poll allowed per wait the later tiles cannot have the first one's values: the solve ends, its x is marked
+    by NaNs, and the next synchronising call raises, once. The solver goes on working."""
+    n = 640
+    A, rng = spd(n, 5)
+    D = bls.DenseCholesky(n)
+    S = torch.from_numpy(np.triu(A).ravel(order="F")).to("cuda")
+    g = rng.standard_normal(n)
+    want = np.linalg.solve(A, g)
+    limit = bls._lib.gpu().bls_dense_solver_set_wait_limit
+    assert limit(D.handle, 0) == bls._lib.BLS_EINVAL
+    assert D.factor(S)
+    for report in (D.check, lambda: D.factor(S)):
+        assert limit(D.handle, 1) == 0
+        x = D.solve(torch.from_numpy(g).to("cuda"))
+        assert torch.isnan(x).any()
+        with pytest.raises(bls.BlsError, match="wait"):
+            report()
+        D.check()
+        assert limit(D.handle, 1 << 22) == 0
+        x = D.solve(torch.from_numpy(g).to("cuda"))
+        D.check()
+        assert relerr(x.cpu().numpy(), want) <= 1e-10
+    assert D.factor(S) and D.failed_column == 0
