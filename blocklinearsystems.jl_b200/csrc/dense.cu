@@ -33,6 +33,7 @@ struct DenseSolver {
   long long* status = nullptr;   // [0]: first failing column (0-based) or -1; [1]: 1 after a solve whose wait gave up
   int64_t wait_limit = kWaitLimit;   // polls of a value before a wait of the solve gives up
   bool factored = false;
+  bool prepared = false;   // k_step's shared-memory limit is set
   // The diagonal tiles run on one high-priority stream, the panels below them and the updates they wait for on another,
   // while the rest of a group's update runs on the caller's stream (created at the first factorisation).
   cudaStream_t panel_stream = nullptr;
@@ -62,7 +63,7 @@ struct DenseSolver {
 // sides are read and written in contiguous runs.
 template <class T>
 __global__ void __launch_bounds__(256) k_dense_load(int64_t n, int64_t ld, const T* __restrict__ S, double* __restrict__ W, double lambda,
-                                                    const double* __restrict__ s_r, long long* __restrict__ status) {
+                                                    const double* __restrict__ s_r, double* __restrict__ rows, long long* __restrict__ status) {
   __shared__ double t[32][33];
   if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) status[0] = -1;
   if (blockIdx.y > blockIdx.x) return;
@@ -80,6 +81,7 @@ __global__ void __launch_bounds__(256) k_dense_load(int64_t n, int64_t ld, const
     double v = t[x][y + k];
     if (s_r && i == j && i < n) v += lambda * s_r[j];
     W[i + ld * j] = v;
+    if (j0 < NB && i0 >= NB && i0 < 2 * NB) rows[(i - NB) + NB * j] = v;   // the rows below tile 0, for the first k_step
   }
 }
 
@@ -113,8 +115,8 @@ __device__ __forceinline__ void cp_async8(double* smem, const double* gmem) {
 // useless. (One warp holding two rows a lane and shuffling the 15 entries of a column: a 64-bit shuffle takes 11 cycles of
 // issue and an FP64 multiply-add 5, 430 cycles a column.) Then all warps subtract the sub-panel's rank-16
 // product from the rest of the tile (3 x 3 entries a thread, or 2 x 2, or one) after which the last inverts the sub-panel's 16 x
-// 16 diagonal block into V (column-major; a lane per column). Returns (to every thread) the first column whose pivot is not
-// positive or not finite, or -1.
+// 16 diagonal block into V (column-major; a lane per column). The sub-panels from column `cols` on are the identity
+// padding and stay as they are. Returns (to every thread) the first column whose pivot is not positive or not finite, or -1.
 template <int NA>
 __device__ __forceinline__ void rank16(double (*T)[TS], int c0, int tid) {   // rows and columns c0 + 16 .. c0 + 16 + 16 NA
   const int tx = tid & 15, ty = tid >> 4, base = c0 + 16;
@@ -143,9 +145,9 @@ __device__ __forceinline__ void rank16(double (*T)[TS], int c0, int tid) {   // 
       if (a > b || ty <= tx) T[base + tx + 16 * a][base + ty + 16 * b] -= acc[a][b];
 }
 
-__device__ int factor_tile(double (*T)[TS], double* dv, double (*V)[16][16], int* failed) {
+__device__ int factor_tile(double (*T)[TS], double* dv, double (*V)[16][16], int* failed, int cols) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  for (int c0 = 0; c0 < NB; c0 += 16) {
+  for (int c0 = 0; c0 < cols; c0 += 16) {
     if (warp < 2) {
       const int r = c0 + 32 * warp + lane;
       const bool own = r < NB;
@@ -177,9 +179,12 @@ __device__ int factor_tile(double (*T)[TS], double* dv, double (*V)[16][16], int
     }
     __syncthreads();
     if (*failed >= 0) return *failed;   // uniform
-    if (c0 == 0) rank16<3>(T, 0, tid);
-    else if (c0 == 16) rank16<2>(T, 16, tid);
-    else if (c0 == 32) rank16<1>(T, 32, tid);
+    const bool more = c0 + 16 < cols;
+    if (more) {
+      if (c0 == 0) rank16<3>(T, 0, tid);
+      else if (c0 == 16) rank16<2>(T, 16, tid);
+      else rank16<1>(T, 32, tid);
+    }
     if (warp == 7 && lane < 16) {   // column `lane` of the inverse: v[i] = s[i] / L[i, i], then s[k] -= L[k, i] v[i] below it
       double v[16];
 #pragma unroll
@@ -194,7 +199,7 @@ __device__ int factor_tile(double (*T)[TS], double* dv, double (*V)[16][16], int
       for (int i = 0; i < 16; ++i) V[c0 / 16][lane][i] = v[i];
     }
     // the next sub-panel's warps wait for the product only; the inverses are done by the barrier at the end
-    if (c0 + 16 < NB) __syncthreads();
+    if (more) __syncthreads();
   }
   __syncthreads();
   return -1;
@@ -202,11 +207,11 @@ __device__ int factor_tile(double (*T)[TS], double* dv, double (*V)[16][16], int
 
 // The 64 rows of X solved against the factored tile (X L' = A), by 256 threads in four steps of 16 columns: a thread
 // holds 4 columns of one row, subtracts the products of the columns already solved, and the 16 x 16 diagonal block is
-// applied through its inverse. X[c][r] in place; Z is scratch. (A thread per row with its 64 entries in registers, fully
+// applied through its inverse. X[c][r] in place; Z is scratch; the steps from column `cols` on (identity padding) are left out. (A thread per row with its 64 entries in registers, fully
 // unrolled, was bound by fetching its 64 KB of instructions: 25 us a panel.)
-__device__ __forceinline__ void solve_rows(double (*X)[NB], double (*Z)[NB], const double (*T)[TS], const double (*V)[16][16], int tid) {
+__device__ __forceinline__ void solve_rows(double (*X)[NB], double (*Z)[NB], const double (*T)[TS], const double (*V)[16][16], int tid, int cols = NB) {
   const int r = tid & 63, q = 4 * (tid >> 6);
-  for (int b = 0; b < NB; b += 16) {
+  for (int b = 0; b < cols; b += 16) {
     double acc[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) acc[j] = X[b + q + j][r];
@@ -249,15 +254,16 @@ struct PanelSmem {
   double Z[16][NB];
 };
 
-// The CTA's 64 x 64 inverse: the identity solved against the tile (X L' = I, so X[i][j] = inverse[i][j]), for the solve.
-__device__ __forceinline__ void tile_inverse(PanelSmem& s, double* __restrict__ inv, int64_t k0, int tid) {
+// The 64 x 64 inverse of the factored tile T: the identity solved against it (X L' = I, so X[i][j] = inverse[i][j]), for
+// the solve.
+__device__ __forceinline__ void tile_inverse(PanelSmem& s, const double (*T)[TS], double* __restrict__ inv, int64_t k0, int tid, int cols = NB) {
 #pragma unroll
   for (int k = 0; k < NB * NB / 256; ++k) {
     const int e = tid + 256 * k;
     s.X[e >> 6][e & 63] = (e >> 6) == (e & 63) ? 1.0 : 0.0;
   }
   __syncthreads();
-  solve_rows(s.X, s.Z, s.T, s.V, tid);
+  solve_rows(s.X, s.Z, T, s.V, tid, cols);
 #pragma unroll
   for (int k = 0; k < NB * NB / 256; ++k) {
     const int e = tid + 256 * k, i = e & 63, j = e >> 6;
@@ -267,7 +273,8 @@ __device__ __forceinline__ void tile_inverse(PanelSmem& s, double* __restrict__ 
 
 // The diagonal tiles, one CTA after the other: the chain that every panel waits for. For panel k (k0 = 64 k) it solves the
 // 64 rows below the diagonal tile (a copy of them, `rows`: k_trsm_panel solves the same rows in W meanwhile), subtracts
-// their rank-64 product from the next diagonal tile and factors that; `first`: it factors tile 0. A non-positive or
+// their rank-64 product from the next diagonal tile and factors that; `first`: it factors tile 0. `cols`: columns of the
+// tile to factor that are not padding. A non-positive or
 // non-finite pivot records its column and nothing is written. Bound by the latency of its 64 columns, one after another
 // (14 us a tile; 17 to 21 before, with the rows' 10 us and the update's 9 us as launches of their own between the tiles):
 // a factorisation takes 30 us a panel where the updates do not bound it (n = 1000: 0.535 -> 0.484 ms), 40 before.
@@ -276,7 +283,7 @@ struct StepSmem {
   double next[NB][TS];
 };
 __global__ void __launch_bounds__(256, 1) k_step(int64_t ld, double* __restrict__ W, const double* __restrict__ rows, double* __restrict__ inv16,
-                                                 int64_t k0, int first, long long* __restrict__ status) {
+                                                 double* __restrict__ inv, int64_t k0, int first, int cols, long long* __restrict__ status) {
   extern __shared__ __align__(16) unsigned char dense_smem[];
   StepSmem& s = *reinterpret_cast<StepSmem*>(dense_smem);
   __shared__ int failed;
@@ -326,7 +333,7 @@ __global__ void __launch_bounds__(256, 1) k_step(int64_t ld, double* __restrict_
       }
     __syncthreads();
   }
-  const int bad = factor_tile(s.next, s.p.dv, s.p.V, &failed);
+  const int bad = factor_tile(s.next, s.p.dv, s.p.V, &failed, cols);
   if (bad >= 0) {
     if (tid == 0) status[0] = d0 + bad;
     return;
@@ -338,6 +345,7 @@ __global__ void __launch_bounds__(256, 1) k_step(int64_t ld, double* __restrict_
   }
 #pragma unroll
   for (int k = 0; k < 4; ++k) inv16[d0 * 16 + tid + 256 * k] = (&s.p.V[0][0][0])[tid + 256 * k];
+  if (d0 + NB == ld) tile_inverse(s.p, s.next, inv, d0, tid, cols);   // no panel below it: its inverse is formed here
 }
 
 // Whether a pivot has failed, as thread 0 sees it (false in every other thread). k_step runs beside the kernels that ask
@@ -347,16 +355,7 @@ __device__ __forceinline__ bool stopped(const long long* status) {
   return threadIdx.x == 0 && *reinterpret_cast<const volatile long long*>(status) >= 0;
 }
 
-// Copies the 64 rows below tile 0 for the first k_step.
-__global__ void __launch_bounds__(256) k_first_rows(int64_t ld, const double* __restrict__ W, double* __restrict__ rows) {
-#pragma unroll
-  for (int k = 0; k < NB * NB / 256; ++k) {
-    const int e = threadIdx.x + 256 * k;
-    rows[e] = W[(NB + (e & 63)) + ld * (e >> 6)];
-  }
-}
-
-// The panel below the diagonal tile factored by k_step: a CTA per 64 rows, and one for the tile's inverse.
+// The panel below a diagonal tile factored by k_step: a CTA per 64 rows, and one for the tile's inverse.
 __global__ void __launch_bounds__(256) k_trsm_panel(int64_t ld, double* __restrict__ W, const double* __restrict__ inv16,
                                                     double* __restrict__ inv, int64_t k0, const long long* __restrict__ status) {
   extern __shared__ __align__(16) unsigned char dense_smem[];
@@ -377,7 +376,7 @@ __global__ void __launch_bounds__(256) k_trsm_panel(int64_t ld, double* __restri
   run_cp_wait<0>();
   if (__syncthreads_or(stop)) return;
   if (!rows) {
-    tile_inverse(s, inv, k0, tid);
+    tile_inverse(s, s.T, inv, k0, tid);
     return;
   }
   solve_rows(s.X, s.Z, s.T, s.V, tid);
@@ -634,13 +633,17 @@ static void launch_factor_body(DenseSolver* D, cudaStream_t s, cudaStream_t p) {
   };
   then(s, D->ev_join, p);
   BLS_CUDA(cudaStreamWaitEvent(u, D->ev_join, 0));
-  launch_prio(k_step, dim3(1), 256, sizeof(StepSmem), p, prio, ld, W, (const double*)rows, v16, (int64_t)0, 1, st);
-  if (nt > 1) launch_prio(k_first_rows, dim3(1), 256, 0, p, prio, ld, (const double*)W, rows);
+  auto step = [&](int64_t k0, int first, const double* below_rows) {
+    const int64_t d0 = first ? k0 : k0 + NB;
+    launch_prio(k_step, dim3(1), 256, sizeof(StepSmem), p, prio, ld, W, below_rows, v16, inv, k0, first, (int)std::min<int64_t>(NB, D->n - d0), st);
+  };
+  step(0, 1, rows);
   bool next_pending = false;
   for (int64_t g0 = 0; g0 < nt; g0 += GROUP) {
     const int64_t g1 = std::min(nt, g0 + GROUP);   // the group's panels
     for (int64_t k = g0; k < g1; ++k) {
       const int64_t below = nt - k - 1;
+      if (below == 0) break;   // the last tile's inverse is k_step's
       // u: the panel's rows, once its tile is factored; p: the next tile, once the previous panel's update (and, for a
       // group's first panel, the previous group's) is done
       then(p, D->ev_tile, u);
@@ -650,8 +653,8 @@ static void launch_factor_body(DenseSolver* D, cudaStream_t s, cudaStream_t p) {
         BLS_CUDA(cudaStreamWaitEvent(u, D->ev_next, 0));
       }
       launch_prio(k_trsm_panel, dim3((unsigned)(below + 1)), 256, sizeof(PanelSmem), u, prio, ld, W, (const double*)v16, inv, k * NB, cst);
-      if (below == 0) break;
-      launch_prio(k_step, dim3(1), 256, sizeof(StepSmem), p, prio, ld, W, (const double*)(rows + (k & 1) * NB * NB), v16, k * NB, 0, st);
+      step(k * NB, 0, rows + (k & 1) * NB * NB);
+      if (below == 1) break;   // nothing but the next diagonal tile is left
       // the group's remaining columns and the next group's first one, which the next panels need
       const int64_t cols = std::min(nt, g1 + 1) - k - 1;
       launch_prio(k_syrk<64, true>, dim3((unsigned)below, (unsigned)cols), 256, (size_t)syrk_smem<64, true>(), u, prio, ld, W, k * NB, NB,
@@ -689,7 +692,11 @@ static int factor(DenseSolver* D, const T* S, double lambda, const double* s_r, 
   const int64_t n = D->n;
   double* W = D->W;
   long long* st = D->status;
-  if (!D->panel_stream) {
+  if (!D->prepared) {
+    BLS_CUDA(cudaFuncSetAttribute(k_step, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(StepSmem)));
+    D->prepared = true;
+  }
+  if (D->ld > NB && !D->panel_stream) {
     int lo = 0, hi = 0;
     BLS_CUDA(cudaDeviceGetStreamPriorityRange(&lo, &hi));
     D->panel_priority = hi;
@@ -701,12 +708,13 @@ static int factor(DenseSolver* D, const T* S, double lambda, const double* s_r, 
     BLS_CUDA(cudaFuncSetAttribute(k_syrk<64, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, syrk_smem<64, true>()));
     BLS_CUDA(cudaFuncSetAttribute(k_syrk<64, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, syrk_smem<64, false>()));
     BLS_CUDA(cudaFuncSetAttribute(k_syrk<128, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, syrk_smem<128, false>()));
-    BLS_CUDA(cudaFuncSetAttribute(k_step, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(StepSmem)));
     BLS_CUDA(cudaFuncSetAttribute(k_trsm_panel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(PanelSmem)));
   }
   const unsigned tiles = (unsigned)(D->ld / 32);
-  k_dense_load<T><<<dim3(tiles, tiles), 256, 0, s>>>(n, D->ld, S, W, lambda, s_r, st);
-  if (!D->factor_graph) {
+  k_dense_load<T><<<dim3(tiles, tiles), 256, 0, s>>>(n, D->ld, S, W, lambda, s_r, D->rows, st);
+  if (D->ld == NB) {   // one tile: one launch
+    k_step<<<1, 256, sizeof(StepSmem), s>>>(D->ld, W, D->rows, D->inv16, D->inv, 0, 1, (int)n, st);
+  } else if (!D->factor_graph) {
     if (!D->cap_stream) BLS_CUDA(cudaStreamCreateWithFlags(&D->cap_stream, cudaStreamNonBlocking));
     BLS_CUDA(cudaStreamBeginCapture(D->cap_stream, cudaStreamCaptureModeThreadLocal));
     cudaGraph_t gr = nullptr;
@@ -725,7 +733,7 @@ static int factor(DenseSolver* D, const T* S, double lambda, const double* s_r, 
       throw Error(BLS_ECUDA, std::string("instantiating the factorisation: ") + cudaGetErrorString(e));
     }
   }
-  BLS_CUDA(cudaGraphLaunch(D->factor_graph, s));
+  if (D->ld > NB) BLS_CUDA(cudaGraphLaunch(D->factor_graph, s));
   BLS_CUDA(cudaGetLastError());
   long long h[2] = {-1, 0};
   BLS_CUDA(cudaMemcpyAsync(h, st, sizeof(h), cudaMemcpyDeviceToHost, s));

@@ -52,3 +52,17 @@ def test_a_wait_that_gives_up_is_reported(bls):
         D.check()
         assert relerr(x.cpu().numpy(), want) <= 1e-10
     assert D.factor(S) and D.failed_column == 0
+
+
+@pytest.mark.parametrize("n", [1, 2, 15, 16, 17, 33, 48, 49, 65, 80, 81, 96, 97, 113, 127])
+def test_padding_in_the_last_tile(bls, n):
+    """The last tile's padding is left out in steps of 16 columns, and its inverse is formed with it."""
+    A, rng = spd(n, n + 1)
+    D = bls.DenseCholesky(n)
+    S = torch.from_numpy(np.triu(A).ravel(order="F")).to("cuda")
+    for _ in range(2):
+        assert D.factor(S)
+        g = rng.standard_normal(n)
+        assert relerr(D.solve(torch.from_numpy(g).to("cuda")).cpu().numpy(), np.linalg.solve(A, g)) <= 1e-10
+    A[n - 1, n - 1] = -1.0
+    assert not D.factor(torch.from_numpy(np.triu(A).ravel(order="F")).to("cuda")) and D.failed_column == n
