@@ -11,6 +11,7 @@
 #include <algorithm>
 #include <cmath>
 #include <memory>
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -28,7 +29,7 @@ struct DenseSolver {
   DevBuf mem;      // what follows, in one allocation (a solver's creation and destruction cost what its allocations do)
   double* W = nullptr;        // ld x ld FP64, column-major; L in its lower triangle after a successful factorisation
   double* rows = nullptr;     // the 64 rows below the next diagonal tile, two buffers
-  double* inv16 = nullptr;    // per panel the inverses of its diagonal tile's four 16 x 16 diagonal blocks (column-major)
+  double* dinv = nullptr;     // 1 / L[j, j]
   double* inv = nullptr;      // per panel the inverse of its 64 x 64 diagonal tile (column-major), for the solve
   long long* status = nullptr;   // [0]: first failing column (0-based) or -1; [1]: 1 after a solve whose wait gave up
   int64_t wait_limit = kWaitLimit;   // polls of a value before a wait of the solve gives up
@@ -114,9 +115,8 @@ __device__ __forceinline__ void cp_async8(double* smem, const double* gmem) {
 // the exchange through shared memory and one multiply-add. The test of a pivot is off it: a bad one only makes what follows
 // useless. (One warp holding two rows a lane and shuffling the 15 entries of a column: a 64-bit shuffle takes 11 cycles of
 // issue and an FP64 multiply-add 5, 430 cycles a column.) Then all warps subtract the sub-panel's rank-16
-// product from the rest of the tile (3 x 3 entries a thread, or 2 x 2, or one) after which the last inverts the sub-panel's 16 x
-// 16 diagonal block into V (column-major; a lane per column). The sub-panels from column `cols` on are the identity
-// padding and stay as they are. Returns (to every thread) the first column whose pivot is not positive or not finite, or -1.
+// product from the rest of the tile (3 x 3 entries a thread, or 2 x 2, or one). The sub-panels from column `cols` on are the
+// identity padding and stay as they are. Returns (to every thread) the first column whose pivot is not positive or not finite, or -1.
 template <int NA>
 __device__ __forceinline__ void rank16(double (*T)[TS], int c0, int tid) {   // rows and columns c0 + 16 .. c0 + 16 + 16 NA
   const int tx = tid & 15, ty = tid >> 4, base = c0 + 16;
@@ -145,7 +145,7 @@ __device__ __forceinline__ void rank16(double (*T)[TS], int c0, int tid) {   // 
       if (a > b || ty <= tx) T[base + tx + 16 * a][base + ty + 16 * b] -= acc[a][b];
 }
 
-__device__ int factor_tile(double (*T)[TS], double* dv, double (*V)[16][16], int* failed, int cols) {
+__device__ int factor_tile(double (*T)[TS], double* dv, int* failed, int cols) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   for (int c0 = 0; c0 < cols; c0 += 16) {
     if (warp < 2) {
@@ -185,20 +185,6 @@ __device__ int factor_tile(double (*T)[TS], double* dv, double (*V)[16][16], int
       else if (c0 == 16) rank16<2>(T, 16, tid);
       else rank16<1>(T, 32, tid);
     }
-    if (warp == 7 && lane < 16) {   // column `lane` of the inverse: v[i] = s[i] / L[i, i], then s[k] -= L[k, i] v[i] below it
-      double v[16];
-#pragma unroll
-      for (int i = 0; i < 16; ++i) v[i] = i == lane ? 1.0 : 0.0;
-#pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        v[i] *= dv[c0 + i];
-#pragma unroll
-        for (int k = i + 1; k < 16; ++k) v[k] = fma(-T[c0 + k][c0 + i], v[i], v[k]);
-      }
-#pragma unroll
-      for (int i = 0; i < 16; ++i) V[c0 / 16][lane][i] = v[i];
-    }
-    // the next sub-panel's warps wait for the product only; the inverses are done by the barrier at the end
     if (more) __syncthreads();
   }
   __syncthreads();
@@ -206,10 +192,12 @@ __device__ int factor_tile(double (*T)[TS], double* dv, double (*V)[16][16], int
 }
 
 // The 64 rows of X solved against the factored tile (X L' = A), by 256 threads in four steps of 16 columns: a thread
-// holds 4 columns of one row, subtracts the products of the columns already solved, and the 16 x 16 diagonal block is
-// applied through its inverse. X[c][r] in place; Z is scratch; the steps from column `cols` on (identity padding) are left out. (A thread per row with its 64 entries in registers, fully
-// unrolled, was bound by fetching its 64 KB of instructions: 25 us a panel.)
-__device__ __forceinline__ void solve_rows(double (*X)[NB], double (*Z)[NB], const double (*T)[TS], const double (*V)[16][16], int tid, int cols = NB) {
+// subtracts from 4 columns of one row the products of the columns already solved, then a thread per row substitutes through
+// the 16 x 16 diagonal block, its 16 values in registers (dv: 1 / L[j, j]). X[c][r] in place; Z is scratch; the steps from
+// column `cols` on (identity padding) are left out. (A thread per row with its 64 entries in registers, fully unrolled, was
+// bound by fetching its 64 KB of instructions: 25 us a panel. The diagonal blocks applied through explicit inverses took
+// longer than this with the inverses' own time, n = 1000 0.477 ms in all against 0.440, and cost backward stability, see k_solve.)
+__device__ __forceinline__ void solve_rows(double (*X)[NB], double (*Z)[NB], const double (*T)[TS], const double* dv, int tid, int cols = NB) {
   const int r = tid & 63, q = 4 * (tid >> 6);
   for (int b = 0; b < cols; b += 16) {
     double acc[4];
@@ -227,28 +215,26 @@ __device__ __forceinline__ void solve_rows(double (*X)[NB], double (*Z)[NB], con
 #pragma unroll
     for (int j = 0; j < 4; ++j) Z[q + j][r] = acc[j];
     __syncthreads();
-    double out[4] = {0.0, 0.0, 0.0, 0.0};
-#pragma unroll 4
-    for (int k = 0; k < q + 4; ++k) {   // the inverse is lower triangular: column q + j takes k <= q + j
-      const double z = Z[k][r];
+    if (tid < NB) {
+      double z[16];
 #pragma unroll
-      for (int j = 0; j < 4; j += 2) {
-        const double2 v = *reinterpret_cast<const double2*>(&V[b / 16][k][q + j]);
-        out[j] = fma(z, v.x, out[j]);
-        out[j + 1] = fma(z, v.y, out[j + 1]);
+      for (int j = 0; j < 16; ++j) z[j] = Z[j][r];
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        z[j] *= dv[b + j];
+#pragma unroll
+        for (int k = j + 1; k < 16; ++k) z[k] = fma(-z[j], T[b + k][b + j], z[k]);
       }
-    }
 #pragma unroll
-    for (int j = 0; j < 4; ++j) X[b + q + j][r] = out[j];
+      for (int j = 0; j < 16; ++j) X[b + j][r] = z[j];
+    }
     __syncthreads();
   }
 }
 
-// shared memory of the panel kernels: the diagonal tile, the 16 x 16 inverses, 1 / L[j, j], the CTA's 64 panel rows and
-// their scratch
+// shared memory of the panel kernels: the diagonal tile, 1 / L[j, j], the CTA's 64 panel rows and their scratch
 struct PanelSmem {
   double T[NB][TS];
-  double V[NB / 16][16][16];
   double dv[NB];
   double X[NB][NB];   // X[column][row]
   double Z[16][NB];
@@ -263,7 +249,7 @@ __device__ __forceinline__ void tile_inverse(PanelSmem& s, const double (*T)[TS]
     s.X[e >> 6][e & 63] = (e >> 6) == (e & 63) ? 1.0 : 0.0;
   }
   __syncthreads();
-  solve_rows(s.X, s.Z, T, s.V, tid, cols);
+  solve_rows(s.X, s.Z, T, s.dv, tid, cols);
 #pragma unroll
   for (int k = 0; k < NB * NB / 256; ++k) {
     const int e = tid + 256 * k, i = e & 63, j = e >> 6;
@@ -276,13 +262,13 @@ __device__ __forceinline__ void tile_inverse(PanelSmem& s, const double (*T)[TS]
 // their rank-64 product from the next diagonal tile and factors that; `first`: it factors tile 0. `cols`: columns of the
 // tile to factor that are not padding. A non-positive or
 // non-finite pivot records its column and nothing is written. Bound by the latency of its 64 columns, one after another
-// (14 us a tile; 17 to 21 before, with the rows' 10 us and the update's 9 us as launches of their own between the tiles):
-// a factorisation takes 30 us a panel where the updates do not bound it (n = 1000: 0.535 -> 0.484 ms), 40 before.
+// (with the rows' solve and the update as launches of their own between the tiles a panel took 33 us): a factorisation takes
+// 27 us a panel where the updates do not bound it (n = 1000: 0.535 -> 0.440 ms).
 struct StepSmem {
   PanelSmem p;
   double next[NB][TS];
 };
-__global__ void __launch_bounds__(256, 1) k_step(int64_t ld, double* __restrict__ W, const double* __restrict__ rows, double* __restrict__ inv16,
+__global__ void __launch_bounds__(256, 1) k_step(int64_t ld, double* __restrict__ W, const double* __restrict__ rows, double* __restrict__ dinv,
                                                  double* __restrict__ inv, int64_t k0, int first, int cols, long long* __restrict__ status) {
   extern __shared__ __align__(16) unsigned char dense_smem[];
   StepSmem& s = *reinterpret_cast<StepSmem*>(dense_smem);
@@ -297,8 +283,7 @@ __global__ void __launch_bounds__(256, 1) k_step(int64_t ld, double* __restrict_
       cp_async8(&s.p.X[c][r], rows + e);
       cp_async8(&s.p.T[r][c], W + (k0 + r) + ld * (k0 + c));   // entries above the diagonal are not used
     }
-#pragma unroll
-    for (int k = 0; k < 4; ++k) cp_async8(&s.p.V[0][0][0] + tid + 256 * k, inv16 + k0 * 16 + tid + 256 * k);
+    if (tid < NB) cp_async8(s.p.dv + tid, dinv + k0 + tid);
   }
   run_cp_commit();
   load_tile(s.next, W, ld, d0, tid);
@@ -306,7 +291,7 @@ __global__ void __launch_bounds__(256, 1) k_step(int64_t ld, double* __restrict_
   run_cp_wait<0>();
   __syncthreads();
   if (!first) {
-    solve_rows(s.p.X, s.p.Z, s.p.T, s.p.V, tid);
+    solve_rows(s.p.X, s.p.Z, s.p.T, s.p.dv, tid);
     // next -= X X', 4 x 4 entries a thread: rows 2 tx + {0, 1, 32, 33}, columns 2 ty + {0, 1, 32, 33}
     const int tx = tid & 15, ty = tid >> 4;
     double acc[4][4];
@@ -333,7 +318,7 @@ __global__ void __launch_bounds__(256, 1) k_step(int64_t ld, double* __restrict_
       }
     __syncthreads();
   }
-  const int bad = factor_tile(s.next, s.p.dv, s.p.V, &failed, cols);
+  const int bad = factor_tile(s.next, s.p.dv, &failed, cols);
   if (bad >= 0) {
     if (tid == 0) status[0] = d0 + bad;
     return;
@@ -343,8 +328,7 @@ __global__ void __launch_bounds__(256, 1) k_step(int64_t ld, double* __restrict_
     const int e = tid + 256 * k, rr = e & 63, cc = e >> 6;
     if (cc <= rr) W[(d0 + rr) + ld * (d0 + cc)] = s.next[rr][cc];
   }
-#pragma unroll
-  for (int k = 0; k < 4; ++k) inv16[d0 * 16 + tid + 256 * k] = (&s.p.V[0][0][0])[tid + 256 * k];
+  if (tid < NB) dinv[d0 + tid] = s.p.dv[tid];
   if (d0 + NB == ld) tile_inverse(s.p, s.next, inv, d0, tid, cols);   // no panel below it: its inverse is formed here
 }
 
@@ -356,7 +340,7 @@ __device__ __forceinline__ bool stopped(const long long* status) {
 }
 
 // The panel below a diagonal tile factored by k_step: a CTA per 64 rows, and one for the tile's inverse.
-__global__ void __launch_bounds__(256) k_trsm_panel(int64_t ld, double* __restrict__ W, const double* __restrict__ inv16,
+__global__ void __launch_bounds__(256) k_trsm_panel(int64_t ld, double* __restrict__ W, const double* __restrict__ dinv,
                                                     double* __restrict__ inv, int64_t k0, const long long* __restrict__ status) {
   extern __shared__ __align__(16) unsigned char dense_smem[];
   PanelSmem& s = *reinterpret_cast<PanelSmem*>(dense_smem);
@@ -370,8 +354,7 @@ __global__ void __launch_bounds__(256) k_trsm_panel(int64_t ld, double* __restri
     if (rows) cp_async8(&s.X[c][r], W + (row0 + r) + ld * (k0 + c));
     cp_async8(&s.T[r][c], W + (k0 + r) + ld * (k0 + c));   // entries above the diagonal are not used
   }
-#pragma unroll
-  for (int k = 0; k < 4; ++k) cp_async8(&s.V[0][0][0] + tid + 256 * k, inv16 + k0 * 16 + tid + 256 * k);
+  if (tid < NB) cp_async8(s.dv + tid, dinv + k0 + tid);
   run_cp_commit();
   run_cp_wait<0>();
   if (__syncthreads_or(stop)) return;
@@ -379,7 +362,7 @@ __global__ void __launch_bounds__(256) k_trsm_panel(int64_t ld, double* __restri
     tile_inverse(s, s.T, inv, k0, tid);
     return;
   }
-  solve_rows(s.X, s.Z, s.T, s.V, tid);
+  solve_rows(s.X, s.Z, s.T, s.dv, tid);
 #pragma unroll
   for (int k = 0; k < NB * NB / 256; ++k) {
     const int e = tid + 256 * k, r = e & 63, c = e >> 6;
@@ -499,9 +482,12 @@ __global__ void __launch_bounds__(256, AHEAD ? 3 : MT == 128 ? 2 : 4) k_syrk(int
 // L L' x = g in one cooperative launch, CTA b owning the 64 rows of tile b. Forward: it takes y_k of every earlier tile in
 // order (polling it: each value is 8 bytes, all bits set until it is written), subtracts L[b, k] y_k from its rows, then
 // multiplies them by the inverse of its diagonal tile and posts y_b. Backward the same from the last tile up with L'. A
-// tile's 64 x 64 block of L is loaded before its poll. A poll that gives up after `limit` tries
+// tile's 64 x 64 block of L is loaded before its poll. The diagonal tile's inverse alone would cost backward stability:
+// ||S x - g|| / (||S|| ||x||) reached 6e-12, 8e-10 and 1e-8 on Gaussian kernel matrices of condition 1e8, 1e10 and 1e12, where
+// substitution leaves 5e-17. One step of refinement against the tile itself brings it back to 5e-17, for two more products of
+// 64 x 64 from shared memory: n = 1000 51 -> 60 us, 10000 0.55 -> 0.58 ms. A poll that gives up after `limit` tries
 // raises the fault word, which the next synchronising call reports, and passes NaNs on, so that nothing waits for ever.
-// n = 6000: 1.8 ms as two launches per tile with a substitution by one warp in each, 0.29 ms now.
+// n = 10000: 2.3 ms as two launches per tile with a substitution by one warp in each, 0.58 ms now.
 constexpr unsigned long long kUnwritten = ~0ull;
 __device__ __forceinline__ double poll_value(const double* p, int64_t limit, long long* fault) {
   unsigned long long v = kUnwritten;
@@ -519,14 +505,28 @@ __device__ __forceinline__ void post_value(double* p, double v) {
   asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(b) : "memory");
 }
 
-__global__ void __launch_bounds__(256) k_solve(int64_t n, int64_t ld, const double* __restrict__ W, const double* __restrict__ inv,
+struct SolveSmem {   // the tile of L and its inverse, [column][row], strides that serve both directions without conflicts
+  double L[NB][NB + 1];
+  double inv[NB][NB + 1];
+};
+__global__ void __launch_bounds__(256, 2) k_solve(int64_t n, int64_t ld, const double* __restrict__ W, const double* __restrict__ inv,
                                                const double* g, double* x, double* y, int64_t limit, long long* fault) {
   __shared__ double rt[NB];   // the tile's current right-hand side
   __shared__ double xk[NB];
   __shared__ double part[4][NB];
+  extern __shared__ __align__(16) unsigned char dense_smem[];
+  SolveSmem& sm = *reinterpret_cast<SolveSmem*>(dense_smem);
   const int tid = threadIdx.x, r = tid & 63, q = tid >> 6, lane = tid & 31, warp = tid >> 5;
   const int nt = (int)(ld / NB), b = blockIdx.x;
   const int64_t row0 = NB * (int64_t)b;
+  // the diagonal tile and its inverse come in while the earlier tiles are waited for
+#pragma unroll
+  for (int k = 0; k < NB * NB / 256; ++k) {
+    const int c = q + 4 * k;
+    cp_async8(&sm.L[c][r], W + (row0 + r) + ld * (row0 + c));   // entries above the diagonal are not used
+    cp_async8(&sm.inv[c][r], inv + NB * row0 + r + NB * c);
+  }
+  run_cp_commit();
   double* yf = y;
   double* yb = y + ld;
   if (tid < NB) rt[tid] = row0 + tid < n ? g[row0 + tid] : 0.0;
@@ -553,11 +553,34 @@ __global__ void __launch_bounds__(256) k_solve(int64_t n, int64_t ld, const doub
     // barrier orders xk, the one below part and rt
     __syncthreads();
   }
-  load(inv + NB * row0, NB);
-  __syncthreads();   // rt (b = 0: as it was read from g)
-  const double yv = mul(rt);
+  run_cp_wait<0>();
+  __syncthreads();   // the tile and its inverse, rt (b = 0: as it was read from g)
+  // the tile's system (T: transposed) for rt, in every thread: through the inverse, with one step of refinement
+  auto product = [&](const double (*M)[NB + 1], auto t, bool lower) {
+    double s = 0.0;
+#pragma unroll
+    for (int c = 0; c < 16; ++c) {
+      const int k = 16 * q + c, row = decltype(t)::value ? k : r, col = decltype(t)::value ? r : k;
+      s = fma(lower && row < col ? 0.0 : M[col][row], xk[k], s);
+    }
+    part[q][r] = s;
+    __syncthreads();
+    return (part[0][r] + part[1][r]) + (part[2][r] + part[3][r]);
+  };
+  auto tile_solve = [&](auto t) {
+    if (q == 0) xk[r] = rt[r];
+    __syncthreads();
+    const double x0 = product(sm.inv, t, false);
+    if (q == 0) xk[r] = x0;   // every thread has passed the barrier in product after reading xk
+    __syncthreads();          // and part is read
+    const double res = rt[r] - product(sm.L, t, true);
+    if (q == 0) xk[r] = res;
+    __syncthreads();
+    return x0 + product(sm.inv, t, false);
+  };
+  const double yv = tile_solve(std::false_type());
   if (q == 0) post_value(yf + row0 + r, yv);
-  __syncthreads();   // every thread has read rt
+  __syncthreads();   // every thread has read rt and part
   if (q == 0) rt[r] = yv;
   // backward: a block's column sums, a warp per 8 columns, lanes over its rows
   double w0[8], w1[8];
@@ -588,13 +611,11 @@ __global__ void __launch_bounds__(256) k_solve(int64_t n, int64_t ld, const doub
     const double v = mul_t(xk);
     if (lane < 8) rt[8 * warp + lane] -= v;
   }
-  load_t(inv + NB * row0, NB);
-  __syncthreads();
-  const double xv = mul_t(rt);
-  if (lane < 8) {
-    const int64_t i = row0 + 8 * warp + lane;
-    post_value(yb + i, xv);
-    if (i < n) x[i] = xv;
+  __syncthreads();   // rt, and xk is read
+  const double xv = tile_solve(std::true_type());
+  if (q == 0) {
+    post_value(yb + row0 + r, xv);
+    if (row0 + r < n) x[row0 + r] = xv;
   }
 }
 
@@ -619,7 +640,7 @@ static void launch_prio(void (*kernel)(Args...), dim3 grid, unsigned block, size
 static void launch_factor_body(DenseSolver* D, cudaStream_t s, cudaStream_t p) {
   const int64_t ld = D->ld, nt = ld / NB;
   double* W = D->W;
-  double* v16 = D->inv16;
+  double* dinv = D->dinv;
   double* inv = D->inv;
   long long* st = D->status;
   const long long* cst = st;
@@ -635,7 +656,7 @@ static void launch_factor_body(DenseSolver* D, cudaStream_t s, cudaStream_t p) {
   BLS_CUDA(cudaStreamWaitEvent(u, D->ev_join, 0));
   auto step = [&](int64_t k0, int first, const double* below_rows) {
     const int64_t d0 = first ? k0 : k0 + NB;
-    launch_prio(k_step, dim3(1), 256, sizeof(StepSmem), p, prio, ld, W, below_rows, v16, inv, k0, first, (int)std::min<int64_t>(NB, D->n - d0), st);
+    launch_prio(k_step, dim3(1), 256, sizeof(StepSmem), p, prio, ld, W, below_rows, dinv, inv, k0, first, (int)std::min<int64_t>(NB, D->n - d0), st);
   };
   step(0, 1, rows);
   bool next_pending = false;
@@ -652,7 +673,7 @@ static void launch_factor_body(DenseSolver* D, cudaStream_t s, cudaStream_t p) {
         BLS_CUDA(cudaStreamWaitEvent(p, D->ev_next, 0));
         BLS_CUDA(cudaStreamWaitEvent(u, D->ev_next, 0));
       }
-      launch_prio(k_trsm_panel, dim3((unsigned)(below + 1)), 256, sizeof(PanelSmem), u, prio, ld, W, (const double*)v16, inv, k * NB, cst);
+      launch_prio(k_trsm_panel, dim3((unsigned)(below + 1)), 256, sizeof(PanelSmem), u, prio, ld, W, (const double*)dinv, inv, k * NB, cst);
       step(k * NB, 0, rows + (k & 1) * NB * NB);
       if (below == 1) break;   // nothing but the next diagonal tile is left
       // the group's remaining columns and the next group's first one, which the next panels need
@@ -713,7 +734,7 @@ static int factor(DenseSolver* D, const T* S, double lambda, const double* s_r, 
   const unsigned tiles = (unsigned)(D->ld / 32);
   k_dense_load<T><<<dim3(tiles, tiles), 256, 0, s>>>(n, D->ld, S, W, lambda, s_r, D->rows, st);
   if (D->ld == NB) {   // one tile: one launch
-    k_step<<<1, 256, sizeof(StepSmem), s>>>(D->ld, W, D->rows, D->inv16, D->inv, 0, 1, (int)n, st);
+    k_step<<<1, 256, sizeof(StepSmem), s>>>(D->ld, W, D->rows, D->dinv, D->inv, 0, 1, (int)n, st);
   } else if (!D->factor_graph) {
     if (!D->cap_stream) BLS_CUDA(cudaStreamCreateWithFlags(&D->cap_stream, cudaStreamNonBlocking));
     BLS_CUDA(cudaStreamBeginCapture(D->cap_stream, cudaStreamCaptureModeThreadLocal));
@@ -771,12 +792,12 @@ int bls_dense_solver_create(bls_ctx* ctx, int64_t n, bls_dense_solver** out) {
     D->ctx = ctx;
     D->n = n;
     D->ld = (n + NB - 1) / NB * NB;
-    const size_t w = (size_t)(D->ld * D->ld), r = 2 * NB * NB, v16 = 16 * (size_t)D->ld, v = NB * (size_t)D->ld, y = 2 * (size_t)D->ld;
-    D->mem.alloc(sizeof(double) * (w + r + v16 + v + y) + 2 * sizeof(long long));   // every part a multiple of 128 doubles
+    const size_t w = (size_t)(D->ld * D->ld), r = 2 * NB * NB, dv = (size_t)D->ld, v = NB * (size_t)D->ld, y = 2 * (size_t)D->ld;
+    D->mem.alloc(sizeof(double) * (w + r + dv + v + y) + 2 * sizeof(long long));   // every part a multiple of 64 doubles
     D->W = D->mem.as<double>();
     D->rows = D->W + w;
-    D->inv16 = D->rows + r;
-    D->inv = D->inv16 + v16;
+    D->dinv = D->rows + r;
+    D->inv = D->dinv + dv;
     D->y = D->inv + v;
     D->status = reinterpret_cast<long long*>(D->y + y);
     BLS_CUDA(cudaMemsetAsync(D->status, 0, 2 * sizeof(long long), ctx->stream));
@@ -823,7 +844,8 @@ int bls_dense_cholesky_solve(bls_dense_solver* D, const double* g, double* x) {
       int per_sm = 0, nsm = 0, dev = 0;
       BLS_CUDA(cudaGetDevice(&dev));
       BLS_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-      BLS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_solve, 256, 0));
+      BLS_CUDA(cudaFuncSetAttribute(k_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SolveSmem)));
+      BLS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_solve, 256, sizeof(SolveSmem)));
       if (nt > (int64_t)nsm * per_sm) throw Error(BLS_EUNSUPPORTED, "the device is too small for this system's solve");
       D->solve_grid = (int)nt;
     }
@@ -833,7 +855,7 @@ int bls_dense_cholesky_solve(bls_dense_solver* D, const double* g, double* x) {
     const double* inv = D->inv;
     long long* fault = D->status + 1;
     void* args[] = {&n_arg, &ld_arg, &W, &inv, &g, &x, &y, &D->wait_limit, &fault};
-    BLS_CUDA(cudaLaunchCooperativeKernel((const void*)k_solve, dim3((unsigned)D->solve_grid), dim3(256), args, 0, s));
+    BLS_CUDA(cudaLaunchCooperativeKernel((const void*)k_solve, dim3((unsigned)D->solve_grid), dim3(256), args, sizeof(SolveSmem), s));
     BLS_CUDA(cudaGetLastError());
     return BLS_OK;
   })
