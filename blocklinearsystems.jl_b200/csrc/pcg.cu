@@ -418,10 +418,18 @@ __global__ void k_add(int64_t n, double* __restrict__ x, const double* __restric
 // ---------------------------------------------------------------------------------------------------------------
 // The inverse of every 6 x 6 diagonal block of S (symmetric from its upper triangle), a thread per block in registers:
 // the Cholesky factor with k_factor_blocks's pivot test (the lowest failing block into *failed), its inverse, L^-T L^-1.
+// It also adds |g|^2 up into *gg, for the kernel that follows.
 template <class T>
 __global__ void __launch_bounds__(64) k_block_inverse6(int64_t nrb, const int64_t* __restrict__ dbase, const int32_t* __restrict__ dstride,
-                                                       const T* __restrict__ S, double* __restrict__ Minv, long long* __restrict__ failed) {
+                                                       const T* __restrict__ S, double* __restrict__ Minv, long long* __restrict__ failed,
+                                                       const double* __restrict__ g, double* __restrict__ gg) {
   const int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  double s2 = 0.0;
+  if (b < nrb)
+#pragma unroll
+    for (int i = 0; i < 6; ++i) s2 += g[6 * b + i] * g[6 * b + i];
+  s2 = warp_sum_d(s2);
+  if ((threadIdx.x & 31) == 0 && s2 != 0.0) atomicAdd(gg, s2);
   if (b >= nrb) return;
   double L[6][6];
   const T* B = S + dbase[b];
@@ -473,7 +481,7 @@ __global__ void __launch_bounds__(64) k_block_inverse6(int64_t nrb, const int64_
     }
 }
 
-// Scalars of a solve, zero on entry: the iterations' sums in four slots by turns (zeroed two iterations ahead), a start's
+// Scalars of a solve, zero on entry but |g|^2 (gg, k_block_inverse6): the iterations' sums in four slots by turns (zeroed two iterations ahead), a start's
 // (its explicit residual) per start.
 struct PcgScalars {
   double pq[4], rz[4], rr[4];
@@ -542,7 +550,11 @@ __global__ void __launch_bounds__(32 * pcg_warps<T>(), 1) k_pcg_cols(PcgArgs<T> 
   extern __shared__ double acc_smem[];   // per warp kPcgWindow sums
   PcgControl* c = a.ctl;
   PcgScalars* sum = &c->sum;
-  if (c->failed != LLONG_MAX) return;   // uniform across the grid
+  const double gg = sum->gg;
+  if (c->failed != LLONG_MAX || gg == 0.0) {   // uniform across the grid; g = 0: the host sets x = 0
+    if (blockIdx.x == 0 && threadIdx.x == 0) c->out[2] = gg;
+    return;
+  }
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int64_t nwarps = (int64_t)gridDim.x * NW, w = (int64_t)blockIdx.x * NW + warp;
   // The warps' shares: every column costs as much as kColumnCost blocks (its loads one after another, 1.5 us), so that the
@@ -728,12 +740,12 @@ __global__ void __launch_bounds__(32 * pcg_warps<T>(), 1) k_pcg_cols(PcgArgs<T> 
     return z;
   };
   int64_t it = 0;
-  double rr = 0.0, gg = 0.0;
+  double rr = 0.0;
   for (int run = 0;; ++run) {
     // the explicit residual of x
     product(a.x, nullptr, 0.0);
     if (!barrier()) break;
-    double urz = 0.0, urr = 0.0, ugg = 0.0;
+    double urz = 0.0, urr = 0.0;
     rows([&](int64_t i, int64_t b, bool on) {
       const double g = on ? __ldg(a.g + i) : 0.0, r = on ? g - a.q[i] : 0.0;
       const double z = precondition6(b, on, r);
@@ -744,15 +756,9 @@ __global__ void __launch_bounds__(32 * pcg_warps<T>(), 1) k_pcg_cols(PcgArgs<T> 
       }
       urz += r * z;
       urr += r * r;
-      ugg += g * g;
     });
     add(urz, urr, &sum->srz[run], &sum->srr[run]);
-    if (run == 0) {
-      __syncthreads();   // red is read
-      add(ugg, 0.0, &sum->gg, nullptr);
-    }
     if (!barrier()) break;
-    gg = *reinterpret_cast<volatile double*>(&sum->gg);
     rr = *reinterpret_cast<volatile double*>(&sum->srr[run]);
     double rz = *reinterpret_cast<volatile double*>(&sum->srz[run]), rz_old = 0.0;
     const double t2 = a.tol * a.tol * gg;
@@ -993,7 +999,7 @@ static int pcg_solve_cols(PCGPlan* P, const T* S, const double* g, double* x, do
   BLS_CUDA(cudaMemcpyAsync(ctl, h, sizeof(PcgControl), cudaMemcpyHostToDevice, s));
   BLS_CUDA(cudaMemsetAsync(P->q.p, 0, sizeof(double) * P->nr, s));
   k_block_inverse6<T><<<grid_for(P->nrb, 64), 64, 0, s>>>(P->nrb, P->diag_base.as<int64_t>(), P->diag_stride.as<int32_t>(), S,
-                                                          P->Minv.as<double>(), &ctl->failed);
+                                                          P->Minv.as<double>(), &ctl->failed, g, &ctl->sum.gg);
   int& grid = P->pcg_grid[sizeof(T) == 4 ? 0 : 1];
   constexpr int NW = pcg_warps<T>();
   const int smem = NW * kPcgWindow * (int)sizeof(double);
