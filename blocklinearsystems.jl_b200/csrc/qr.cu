@@ -84,6 +84,7 @@ struct QRPlan {
   DevBuf ls_u, ls_v, ls_h, ls_hbar, ls_t, ls_sqd, ls_part, ls_L, ls_acc, ls_flag;
   DevBuf ls_chunk;      // the first table of every chunk of k_lsmr_pass, and ntables
   int64_t ls_nchunks = 0;
+  int ls_chunk_bytes = 0;   // a chunk's bytes in FP64 (kLsmrChunks)
   double* ls_host = nullptr;
   DevBuf status;
   long long* host_status = nullptr;
@@ -1359,7 +1360,11 @@ static void check_jt_pattern(const QRPlan* P, int64_t nrows, int64_t ncols, cons
     }
 }
 
-constexpr int kLsmrChunk = 64 * 1024;   // bytes of tables (in FP64) that a CTA of k_lsmr_pass takes
+// Bytes of tables, in FP64, that a CTA of k_lsmr_pass takes (in FP32 half of them): the first size that holds all but an
+// eighth of the bytes of J~ in whole tables is the plan's. A table that does not fit is read from memory twice, row by row:
+// with 64 KB for every plan, 10,000 tables of 20 couplings (a fifth of them above 64 KB) took 1.91 ms a solve, 1.35 with
+// 104 KB; 3,000 tables of 25 to 34 couplings (mostly above 104 KB) 1.17 with 64 KB, 1.37 with 104, 0.90 with 208.
+constexpr int kLsmrChunks[3] = {64 * 1024, 104 * 1024, 208 * 1024};
 
 static QRPlan* qr_plan_create(bls_ctx* ctx, const bls_qr_plan_desc* d) {
   if (!d || d->nrblocks < 1 || d->neblocks < 1 || d->ntables < d->neblocks) throw Error(BLS_EINVAL, "a QR plan needs retained blocks, eliminated blocks and their tables");
@@ -1595,11 +1600,20 @@ static QRPlan* qr_plan_create(bls_ctx* ctx, const bls_qr_plan_desc* d) {
     upload(P->u_runpos, runpos, s);
     P->q_total.alloc(sizeof(double));
   }
-  {   // k_lsmr_pass's chunks: consecutive tables of at most kLsmrChunk bytes in FP64 (a larger table is a chunk of its own)
+  {   // k_lsmr_pass's chunks: consecutive tables of at most that many bytes in FP64 (a larger table is a chunk of its own)
     std::vector<int32_t> chunk;
+    for (int bytes : kLsmrChunks) {
+      P->ls_chunk_bytes = bytes;
+      int64_t over = 0;
+      for (int64_t t = 0; t < nt; ++t) {
+        const int64_t len = d->raw_offsets[t + 1] - d->raw_offsets[t];
+        if (8 * len > bytes) over += len;
+      }
+      if (8 * over <= P->raw_len) break;
+    }
     int64_t lo = 0;
     for (int64_t t = 0; t < nt; ++t)
-      if (t == 0 || 8 * (d->raw_offsets[t + 1] - lo) > kLsmrChunk) {
+      if (t == 0 || 8 * (d->raw_offsets[t + 1] - lo) > P->ls_chunk_bytes) {
         chunk.push_back((int32_t)t);
         lo = d->raw_offsets[t];
       }
@@ -1938,19 +1952,23 @@ __global__ void k_lsmr_bwd(int64_t nrb, int dmax, const int32_t* __restrict__ r_
   t[boff_r[b] + i] = lsmr_bwd(Linv + doff[b], r_dims[b], i, v + boff_r[b], sc);
 }
 
+// The lanes of a warp that share this one's item, 2^lg (up to 8) side by side
+__device__ __forceinline__ unsigned lane_group(int lg) { return ((1u << (1 << lg)) - 1) << (threadIdx.x & 31 & -(1 << lg)); }
+
 // One pass over J~ for a solve's two products with it. A CTA takes a chunk of consecutive tables (QRPlan::ls_chunk: as many
-// as fit kLsmrChunk bytes), brings them into shared memory with one bulk copy (a table that does not fit, or an F off a
+// as fit the plan's size), brings them into shared memory with one bulk copy (a table that does not fit, or an F off a
 // 16-byte boundary, is read where it is), and then
 //   INIT: forms per (entry, pair of columns) the parts of the diagonal blocks of J~'J~ (diag[entry * np + pair]);
-//   else: a thread per reduced row, u = J~ t - a u, acc += |u|^2; the CTAs past the chunks take the damping rows,
-//         u = sqd .* t - a u;
-// and a thread per (entry, column) forms the parts of J~' u (part[entry * dmax + column]). Every sum is FP64.
+//   else: up to eight lanes per reduced row (as many as its rows leave threads for) share its entries, u = J~ t - a u,
+//         acc += |u|^2; the CTAs past the chunks take the damping rows, u = sqd .* t - a u;
+// and up to eight lanes per (entry, column) form the parts of J~' u (part[entry * dmax + column]). Every sum is FP64. (One
+// lane each left most of a CTA idle on wide tables: 10,000 FP64 tables of 10 couplings 1.61 ms a solve, 0.94 now.)
 // 31,007 tables (178 MB) in FP64: an iteration's two products 47 + 44 us and the start's 90 + 45 as kernels of their own
 // that read J~ from memory, 79 and 98 now; what is left are the chains of lookups from a row to its table, its entries and
 // their variables, several per CTA and only partly hidden by the other two CTAs of an SM. Chunks of 24, 32 and 48 KB, four
 // lanes per row and the first lookups before the wait are within 3% of this.
-template <class T, bool INIT>
-__global__ void __launch_bounds__(256) k_lsmr_pass(int nchunks, int64_t mt, int64_t nr, int dmax, const int32_t* __restrict__ chunk,
+template <class T, bool INIT, int NT>
+__global__ void __launch_bounds__(NT) k_lsmr_pass(int nchunks, int64_t mt, int64_t nr, int dmax, const int32_t* __restrict__ chunk,
                                                    const int32_t* __restrict__ red_tab, const int32_t* __restrict__ t_rows,
                                                    const int32_t* __restrict__ t_cols, const int32_t* __restrict__ t_top,
                                                    const int64_t* __restrict__ t_raw, const int64_t* __restrict__ t_red,
@@ -1964,7 +1982,7 @@ __global__ void __launch_bounds__(256) k_lsmr_pass(int nchunks, int64_t mt, int6
   const int tid = threadIdx.x;
   double nn = 0.0;
   if ((int)blockIdx.x >= nchunks) {
-    const int64_t i = ((int64_t)blockIdx.x - nchunks) * 256 + tid;
+    const int64_t i = ((int64_t)blockIdx.x - nchunks) * NT + tid;
     if (i < nr) {
       const double z = sqd[i] * t[i] - a * u[mt + i];
       u[mt + i] = z;
@@ -1979,6 +1997,7 @@ __global__ void __launch_bounds__(256) k_lsmr_pass(int nchunks, int64_t mt, int6
   const int64_t e0 = t_ptr[ta], ne = t_ptr[tl + 1] - e0;
   int64_t row = 0, r1 = 0, x_off = 0;   // the thread's row, the chunk's end, the row's place in it
   int M_row = 0, e_lo = 0, e_hi = 0;
+  int lg = 0, sub = 0;   // 2^lg lanes share a row's entries, this thread the ones from `sub` on
   int4 q_row = make_int4(0, 0, 0, 0);
   auto find_row = [&] {
     const int tb = red_tab[row];
@@ -1986,7 +2005,7 @@ __global__ void __launch_bounds__(256) k_lsmr_pass(int nchunks, int64_t mt, int6
     x_off = (t_raw[tb] - raw0) + t_top[tb] + (row - t_red[tb]);
     e_lo = t_ptr[tb];
     e_hi = t_ptr[tb + 1];
-    if (e_lo < e_hi) q_row = meta[e_lo];
+    if (e_lo + sub < e_hi) q_row = meta[e_lo + sub];
   };
   const bool staged = len * (int64_t)sizeof(T) + 32 <= room;
   if (staged) {
@@ -2000,8 +2019,11 @@ __global__ void __launch_bounds__(256) k_lsmr_pass(int nchunks, int64_t mt, int6
     }
   }
   if (!INIT) {   // the first row's lookups run while the tables are in flight
-    row = t_red[ta] + tid;
+    row = t_red[ta];
     r1 = t_red[tl] + (t_rows[tl] - t_top[tl]);
+    while (lg < 3 && (r1 - row) << (lg + 1) <= NT) ++lg;
+    sub = tid & ((1 << lg) - 1);
+    row += tid >> lg;
     if (row < r1) find_row();
   }
   if (staged) {
@@ -2017,7 +2039,7 @@ __global__ void __launch_bounds__(256) k_lsmr_pass(int nchunks, int64_t mt, int6
     }
   }
   if (INIT) {
-    for (int64_t id = tid; id < ne * np; id += 256) {
+    for (int64_t id = tid; id < ne * np; id += NT) {
       const int64_t e = e0 + id / np;
       const int p = (int)(id % np);
       int cb = (int)((sqrtf(8.0f * p + 1.0f) - 1.0f) * 0.5f);
@@ -2038,8 +2060,8 @@ __global__ void __launch_bounds__(256) k_lsmr_pass(int nchunks, int64_t mt, int6
     while (row < r1) {
       const T* x = base + x_off;
       double y = 0.0;
-      for (int e = e_lo; e < e_hi; ++e) {
-        const int4 q = e == e_lo ? q_row : meta[e];
+      for (int e = e_lo + sub; e < e_hi; e += 1 << lg) {
+        const int4 q = e == e_lo + sub ? q_row : meta[e];
         const T* col = x + (int64_t)q.x * M_row;
         if (q.z == 6) {   // the common camera block: six independent loads in flight
           T f[6];
@@ -2048,18 +2070,25 @@ __global__ void __launch_bounds__(256) k_lsmr_pass(int nchunks, int64_t mt, int6
 #pragma unroll
           for (int j = 0; j < 6; ++j) y += (double)f[j] * t[q.y + j];
         } else {
+#pragma unroll 3
           for (int j = 0; j < q.z; ++j) y += (double)col[(int64_t)j * M_row] * t[q.y + j];
         }
       }
-      const double z = y - a * u[row];
-      u[row] = z;
-      nn += z * z;
-      row += 256;
+      for (int o = 1 << lg >> 1; o > 0; o >>= 1) y += __shfl_xor_sync(lane_group(lg), y, o);
+      if (sub == 0) {
+        const double z = y - a * u[row];
+        u[row] = z;
+        nn += z * z;
+      }
+      row += NT >> lg;
       if (row < r1) find_row();
     }
     block_sum_add(nn, acc);   // its barrier also orders the chunk's u
   }
-  for (int64_t id = tid; id < ne * dmax; id += 256) {
+  int lc = 0;   // 2^lc lanes share a column's rows
+  while (lc < 3 && (ne * dmax) << (lc + 1) <= NT) ++lc;
+  const int from = tid & ((1 << lc) - 1);
+  for (int64_t id = tid >> lc; id < ne * dmax; id += NT >> lc) {
     const int64_t e = e0 + id / dmax;
     const int j = (int)(id % dmax);
     const int4 q = meta[e];
@@ -2069,8 +2098,9 @@ __global__ void __launch_bounds__(256) k_lsmr_pass(int nchunks, int64_t mt, int6
     const double* ur = u + t_red[tb];
     double s = 0.0;
 #pragma unroll 4
-    for (int i = 0; i < rows; ++i) s += (double)col[i] * ur[i];
-    part[e * dmax + j] = s;
+    for (int i = from; i < rows; i += 1 << lc) s += (double)col[i] * ur[i];
+    for (int o = 1 << lc >> 1; o > 0; o >>= 1) s += __shfl_xor_sync(lane_group(lc), s, o);
+    if (from == 0) part[e * dmax + j] = s;
   }
 }
 
@@ -2175,10 +2205,13 @@ static int lsmr_reduced(QRPlan* P, const T* F, const double* Fr, double lambda, 
   // the start's pass (diagonal blocks and J~' r~) and an iteration's
   auto pass = [&](auto init, double a) {
     constexpr bool INIT = decltype(init)::value;
-    const int room = P->bulk && (reinterpret_cast<uintptr_t>(F) & 15) == 0 ? kLsmrChunk / 8 * (int)sizeof(T) + 32 : 0;
-    auto kern = k_lsmr_pass<T, INIT>;
-    if (room > 48 * 1024) BLS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, room));
-    kern<<<(unsigned)(P->ls_nchunks + (INIT ? 0 : (nr + 255) / 256)), 256, room, s>>>(
+    // 512 threads where two CTAs or one fit an SM, 256 where three or four do (1.85 -> 1.59 ms for 20,000 FP64 tables of
+    // 15 couplings of 3-variable cameras, 104 KB; 0.72 -> 0.85 ms for 10,000 FP32 tables of 20 couplings, 52 KB)
+    const int bytes = P->ls_chunk_bytes / 8 * (int)sizeof(T), nt = bytes > 80 * 1024 ? 512 : 256;
+    const int room = P->bulk && (reinterpret_cast<uintptr_t>(F) & 15) == 0 ? bytes + 32 : 0;
+    auto kern = nt == 512 ? k_lsmr_pass<T, INIT, 512> : k_lsmr_pass<T, INIT, 256>;
+    set_smem(reinterpret_cast<const void*>(kern), (size_t)room);
+    kern<<<(unsigned)(P->ls_nchunks + (INIT ? 0 : (nr + nt - 1) / nt)), nt, room, s>>>(
         (int)P->ls_nchunks, mt, nr, dm, P->ls_chunk.as<int32_t>(), P->red_tab.as<int32_t>(), P->t_rows.as<int32_t>(),
         P->t_cols.as<int32_t>(), P->t_top.as<int32_t>(), P->t_raw.as<int64_t>(), P->t_red.as<int64_t>(), P->t_ptr.as<int32_t>(),
         P->u_meta.as<int4>(), F, F + P->raw_len, room, sqd, t, a, u, part, np, P->ls_part.as<double>(), acc,
