@@ -614,12 +614,19 @@ __global__ void k_qr_free(int64_t t0, int64_t nt, const int32_t* __restrict__ t_
 // accumulate_qr_entry! (src/qr_reduced.jl:375-405) per table. MODE 0: S blocks (upper triangle of diagonal blocks) and
 // J~'r~ into g; MODE 1: the full diagonal blocks D (reduced_diagonal_blocks!, :484-512). from_raw: the same products
 // over the data rows of the raw tables, J'J of the retained columns and J'r (the retained part of the assembly).
-// WHOLE: tables with more than 16 pairs take a whole 6 x 6 block per lane; the form without it, for classes of smaller
-// tables, is held to 64 registers in FP32, eight CTAs an SM. Bound by the additions into S and by the latency of a table
+// WHOLE, for the classes of larger tables, takes the registers it needs (in FP32 a lane takes a whole 6 x 6 block of a table
+// with more than 16 pairs); the forms of smaller tables are held to as many as let eight CTAs (FP32) or five run on an SM:
+// unbounded, 128 registers in FP64, 100,000 tables of three or four cameras took 301 us instead of 269 (289 before the early
+// lookups; bounded, tables of ten cameras 577 instead of 518). Sizes other than 6: eight rows by three columns per step;
+// a column at a time, each entry of X was converted to FP64 for each of them (FP32, 9-variable cameras, the diagonal blocks
+// 649 us, 246 now). Bound by the additions into S and by the latency of a table
 // (its copy, its lookups) at the tables that shared memory holds. 500 x 100,000, all classes: FP32 534 us with a scalar atomic
 // per entry, 374 now; FP64 732, 659 now.
+__host__ __device__ constexpr int gram_ctas(int mode, int bytes, bool all6, bool whole) {
+  return whole ? 1 : bytes == 4 ? (all6 ? 8 : 5) : !all6 ? 1 : mode == 0 ? 5 : 6;
+}
 template <class T, int MODE, bool ALL6, bool WHOLE>
-__global__ void __launch_bounds__(32 * QR_MAX_WARPS, sizeof(T) == 4 && ALL6 && !WHOLE ? 8 : 1) k_qr_gram(int64_t ntab, int warp_bytes, const int32_t* __restrict__ tables,
+__global__ void __launch_bounds__(32 * QR_MAX_WARPS, gram_ctas(MODE, sizeof(T), ALL6, WHOLE)) k_qr_gram(int64_t ntab, int warp_bytes, const int32_t* __restrict__ tables,
                                                               const int32_t* __restrict__ t_rows, const int32_t* __restrict__ t_cols,
                                                               const int32_t* __restrict__ t_top, const int64_t* __restrict__ t_raw,
                                                               const int64_t* __restrict__ t_res, const int32_t* __restrict__ t_ptr,
@@ -653,6 +660,15 @@ __global__ void __launch_bounds__(32 * QR_MAX_WARPS, sizeof(T) == 4 && ALL6 && !
   // on its way (each is a chain of two or three loads: 447 us -> 386 on 500 x 100,000 in FP32, and 374 with WHOLE).
   const int npairs = kt * (kt + 1) / 2;
   struct Unit { int u1, u2, w0, r2; int64_t base, stride; };   // w0 < 0: none
+  auto place = [&](Unit& v, int p) {   // where the unit's block goes
+    if (MODE == 0) {
+      const int k = tp_blk[tp_ptr[t] + p];
+      v.stride = blk_stride ? (int64_t)blk_stride[k] : dense_nr;
+      v.base = blk_base[k] + v.w0 * v.stride;
+    } else {
+      v.r2 = u_ret[u0 + v.u2];
+    }
+  };
   auto unit_of = [&](int q, int G) {
     Unit v{0, 0, -1, 0, 0, 0};
     const int upp = (dmax + G - 1) / G;
@@ -664,13 +680,7 @@ __global__ void __launch_bounds__(32 * QR_MAX_WARPS, sizeof(T) == 4 && ALL6 && !
     while (u2l * (u2l + 1) / 2 > p) --u2l;
     v.u2 = u2l;
     v.u1 = p - u2l * (u2l + 1) / 2;
-    if (MODE == 0) {
-      const int k = tp_blk[tp_ptr[t] + p];
-      v.stride = blk_stride ? (int64_t)blk_stride[k] : dense_nr;
-      v.base = blk_base[k] + v.w0 * v.stride;
-    } else {
-      v.r2 = u_ret[u0 + v.u2];
-    }
+    if (ALL6) place(v, p);
     return v;
   };
   // the variable of column j of the table
@@ -686,7 +696,7 @@ __global__ void __launch_bounds__(32 * QR_MAX_WARPS, sizeof(T) == 4 && ALL6 && !
     }
     return gi;
   };
-  const bool whole = WHOLE && npairs > 16;   // a whole block per lane
+  const bool whole = WHOLE && sizeof(T) == 4 && npairs > 16;   // a whole block per lane
   Unit first{0, 0, -1, 0, 0, 0};
   int first_var = 0;
   bool looked_up = ALL6;
@@ -770,7 +780,7 @@ __global__ void __launch_bounds__(32 * QR_MAX_WARPS, sizeof(T) == 4 && ALL6 && !
     constexpr int G = decltype(g_const)::value;   // columns of the pair's block per work unit
     const int upp = (dmax + G - 1) / G;
     for (int q = lane; q < npairs * upp; q += 32) {
-      const Unit v = looked_up && q == lane ? first : unit_of(q, G);
+      Unit v = looked_up && q == lane ? first : unit_of(q, G);
       const int u1l = v.u1, u2l = v.u2, w0 = v.w0;
       const bool diag = u1l == u2l;
       if (MODE == 1 && !diag) continue;
@@ -778,6 +788,7 @@ __global__ void __launch_bounds__(32 * QR_MAX_WARPS, sizeof(T) == 4 && ALL6 && !
       if (w0 >= d2) continue;
       const int ilo = span ? max(span[u1l].x, span[u2l].x) : 0, ihi = span ? min(span[u1l].y, span[u2l].y) : n;
       if (ilo >= ihi) continue;
+      if (!ALL6) place(v, u2l * (u2l + 1) / 2 + u1l);   // not for the units that have nothing to add
       const T* X = B + u_col[u0 + u1l] * ns;
       const T* Y = B + (u_col[u0 + u2l] + w0) * ns;
       const int64_t stride = MODE == 0 ? v.stride : d2;
@@ -816,24 +827,35 @@ __global__ void __launch_bounds__(32 * QR_MAX_WARPS, sizeof(T) == 4 && ALL6 && !
               if (MODE == 1 || !diag || a <= w0 + w) atomicAdd(out + w * stride + a, acc[w][a]);
         }
       } else if (!ALL6) {
-        for (int w = w0; w < d2 && w < w0 + G; ++w) {
-          double acc[16];
+        // eight rows of the unit's columns at a time, an entry of X converted once for all of them
+        for (int a0 = 0; a0 < d1 && (MODE == 1 || !diag || a0 < w0 + G); a0 += 8) {
+          double acc[G][8];
 #pragma unroll
-          for (int a = 0; a < 16; ++a) acc[a] = 0.0;
+          for (int w = 0; w < G; ++w)
+#pragma unroll
+            for (int a = 0; a < 8; ++a) acc[w][a] = 0.0;
           for (int i = ilo; i < ihi; ++i) {
-            const double y = (double)Y[(w - w0) * ns + i];
+            double y[G];
 #pragma unroll
-            for (int a = 0; a < 16; ++a)
-              if (a < d1) acc[a] += (double)X[a * ns + i] * y;
+            for (int w = 0; w < G; ++w) y[w] = w0 + w < d2 ? (double)Y[w * ns + i] : 0.0;
+#pragma unroll
+            for (int a = 0; a < 8; ++a)
+              if (a0 + a < d1) {
+                const double x = (double)X[(a0 + a) * ns + i];
+#pragma unroll
+                for (int w = 0; w < G; ++w) acc[w][a] += x * y[w];
+              }
           }
 #pragma unroll
-          for (int a = 0; a < 16; ++a)
-            if (a < d1 && (MODE == 1 || !diag || a <= w)) atomicAdd(out + (w - w0) * stride + a, T(acc[a]));
+          for (int w = 0; w < G; ++w)
+#pragma unroll
+            for (int a = 0; a < 8; ++a)
+              if (w0 + w < d2 && a0 + a < d1 && (MODE == 1 || !diag || a0 + a <= w0 + w)) atomicAdd(out + w * stride + a0 + a, T(acc[w][a]));
         }
       }
     }
   };
-  if constexpr (WHOLE) {
+  if constexpr (WHOLE && sizeof(T) == 4) {
     if (whole) units(std::integral_constant<int, 6>{});
     else units(std::integral_constant<int, 3>{});
   } else {
@@ -1722,6 +1744,8 @@ static void gram(QRPlan* P, T* S, bool dense, double* g, const T* F, const doubl
     // a table of 3 KB or more can have 16 pairs (5 entries of 6 columns by 10 rows)
     if constexpr (std::is_same<T, float>::value && MODE == 0)
       if (P->all6 && wb >= 3072) kern = k_qr_gram<T, MODE, true, true>;
+    if constexpr (std::is_same<T, double>::value)   // shared memory holds fewer than 20 of these tables
+      if (P->all6 && wb >= 11 * 1024) kern = k_qr_gram<T, MODE, true, true>;
     const int wpc = std::max(1, tables_per_cta(wb, 32, warp_cap(reinterpret_cast<const void*>(kern))));
     const size_t smem = (size_t)(wb * wpc);
     set_smem(reinterpret_cast<const void*>(kern), smem);
