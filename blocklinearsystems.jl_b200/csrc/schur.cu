@@ -54,7 +54,9 @@ struct RunSchedule {
   int tile_bytes = 0, blob_bytes = 0, smem = 0, wr = 0, ts = 0, mdr = 0, mde = 0;
   int grid = 0;    // resident CTAs per SM x SMs (set at the first launch)
   DevBuf items_d, segs, blob;
-  int64_t bytes() const { return (int64_t)(items_d.bytes + segs.bytes + blob.bytes); }
+  int64_t nsplit = 0;      // FP32: columns of several items
+  DevBuf split, dpart;     // these columns, and their items' sums of the diagonal block
+  int64_t bytes() const { return (int64_t)(items_d.bytes + segs.bytes + blob.bytes + split.bytes + dpart.bytes); }
 };
 
 struct SchurPlan {
@@ -2676,6 +2678,7 @@ static void launch_runs(SchurPlan* P, T* S, bool dense, double* g, const T* C, c
   a.prob_of_cam = poc;
   a.prob_fail = pf;
   a.queue = reinterpret_cast<unsigned long long*>(&P->status.as<Status>()->pad);
+  a.dpart = R.dpart.as<double>();
   a.tile_bytes = R.tile_bytes;
   a.blob_bytes = R.blob_bytes;
   a.wr = R.wr;
@@ -2683,6 +2686,8 @@ static void launch_runs(SchurPlan* P, T* S, bool dense, double* g, const T* C, c
   a.mdr = R.mdr;
   a.mde = R.mde;
   kern<<<(unsigned)std::min<int64_t>(R.items, R.grid), kRunThreads, R.smem, P->ctx->stream>>>(a);
+  if constexpr (F32)
+    if (R.nsplit) k_runs_diag<T><<<grid_for(R.nsplit * R.mdr * R.mdr, 128), 128, 0, P->ctx->stream>>>(a, R.nsplit, R.split.as<int4>());
 }
 
 // A 6/3 plan's layout, read back from its device copies (for a schedule that is built after plan creation). Synchronises.
@@ -2804,7 +2809,7 @@ static int reduce(SchurPlan* P, T* S, bool dense, double* g, const double* b_r, 
   }
   if (use_runs) {
     k_g_init<<<grid_for(P->nr, 256), 256, 0, s>>>(g, b_r, s_r, P->nr, st, poc, pf);
-    P->launches += 2;
+    P->launches += 2 + (RS.nsplit > 0);
     if (ev0) BLS_CUDA(cudaEventRecord(ev0, s));
     launch_runs<T>(P, S, dense, g, C, s_r, s_e, poc, pf);
     if (ev1) BLS_CUDA(cudaEventRecord(ev1, s));
