@@ -1492,8 +1492,10 @@ __global__ void __launch_bounds__(128) k_backsub3(int64_t neb, int64_t Clen, con
   }
 }
 
-// Any sizes, MDE bounding the eliminated ones: eight lanes per point share the columns of each of its couplings, their
-// sums added up by shuffles, then a lane per variable.
+// Any sizes, MDE bounding the eliminated ones: eight lanes per point share its couplings' columns, 2^lw of them a coupling
+// (as many as the retained blocks have variables, up to eight), their sums added up by shuffles, then a lane per variable.
+// (All eight at one coupling left seven of them idle with 1-variable cameras: 300,000 points of one variable, FP64, 97 us, 34
+// now with the sums of one variable kept apart from those of four; a thread per point 46.)
 template <class T, int MDE>
 __global__ void __launch_bounds__(256) k_backsub(int64_t neb, const int32_t* __restrict__ e_dims, const int32_t* __restrict__ eoffsets,
                                                  const int32_t* __restrict__ boffsets_e, const int32_t* __restrict__ eliminated_ptr,
@@ -1501,7 +1503,7 @@ __global__ void __launch_bounds__(256) k_backsub(int64_t neb, const int32_t* __r
                                                  const int32_t* __restrict__ r_dims, const int32_t* __restrict__ boffsets_r,
                                                  const T* __restrict__ C, const double* __restrict__ Einv, const double* __restrict__ z,
                                                  const double* __restrict__ x_r, const double* __restrict__ s_r, const double* __restrict__ s_e,
-                                                 double* __restrict__ x_e) {
+                                                 double* __restrict__ x_e, int lw) {
   const int64_t e = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 3;
   const int l = threadIdx.x & 7;
   const bool on = e < neb;
@@ -1513,10 +1515,10 @@ __global__ void __launch_bounds__(256) k_backsub(int64_t neb, const int32_t* __r
     se[i] = s_e && i < de ? s_e[so + i] : 1.0;
   }
   if (on)
-    for (int c = eliminated_ptr[e]; c < eliminated_ptr[e + 1]; ++c) {
+    for (int c = eliminated_ptr[e] + (l >> lw); c < eliminated_ptr[e + 1]; c += 8 >> lw) {
       const int r = entry_retained[c], dr = r_dims[r], ro = boffsets_r[r];
       const T* cb = C + coffsets[c];
-      for (int ir = l; ir < dr; ir += 8) {
+      for (int ir = l & ((1 << lw) - 1); ir < dr; ir += 1 << lw) {
         const double x = x_r[ro + ir], f = s_r ? s_r[ro + ir] : 1.0;
 #pragma unroll
         for (int i = 0; i < MDE; ++i)
@@ -3149,11 +3151,13 @@ static void backsub(SchurPlan* P, double* x_e, const double* x_r, const T* C, co
                                                                P->entry_retained.as<int32_t>(), P->entry_eliminated.as<int32_t>(), C,
                                                                P->Einv64.as<double>(), P->z.as<double>(), x_r, s_r, s_e, x_e);
   };
+  int lw = 0;
+  while (lw < 3 && (1 << lw) < P->max_dr) ++lw;
   auto any = [&](auto kern) {
     kern<<<grid, 256, 0, s>>>(P->neblocks, P->e_dims.as<int32_t>(), P->eoffsets.as<int32_t>(), P->boffsets_e.as<int32_t>(),
                               P->eliminated_ptr.as<int32_t>(), P->entry_retained.as<int32_t>(), P->coffsets.as<int32_t>(),
                               P->r_dims.as<int32_t>(), P->boffsets_r.as<int32_t>(), C, P->Einv64.as<double>(), P->z.as<double>(), x_r, s_r,
-                              s_e, x_e);
+                              s_e, x_e, lw);
   };
   switch (P->uniform_dr) {
     case 6: uniform(k_backsub3<T, 6>); break;
@@ -3161,7 +3165,8 @@ static void backsub(SchurPlan* P, double* x_e, const double* x_r, const T* C, co
     case 8: uniform(k_backsub3<T, 8>); break;
     case 9: uniform(k_backsub3<T, 9>); break;
     default:
-      if (P->max_de <= 4) any(k_backsub<T, 4>);
+      if (P->max_de == 1) any(k_backsub<T, 1>);
+      else if (P->max_de <= 4) any(k_backsub<T, 4>);
       else any(k_backsub<T, 16>);
   }
   BLS_CUDA(cudaGetLastError());
