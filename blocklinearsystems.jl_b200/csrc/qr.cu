@@ -1010,8 +1010,9 @@ __global__ void __launch_bounds__(256) k_jtj_quadform(int64_t nt, int64_t neb, i
   if (lane == 0 && part != 0.0) atomicAdd(total, part);
 }
 
-// qr_backsubstitute_group! (src/qr_reduced.jl:24-93), FP64: eight lanes per eliminated table over its entries' columns, the
-// sums added up by shuffles, then U x_e = q - B x_r solved by one lane; MDE rows at a time from the last, so that a table
+// qr_backsubstitute_group! (src/qr_reduced.jl:24-93), FP64: eight lanes per eliminated table over its entries' columns, 2^lw
+// of them an entry (as many as the retained blocks have variables, up to eight: with all eight at one entry, 1-variable
+// cameras left seven idle, 200,000 tables 147 us, 76 now; a thread per table 80), the sums added up by shuffles, then U x_e = q - B x_r solved by one lane; MDE rows at a time from the last, so that a table
 // of any size keeps its sums in registers. 31,007 tables, FP64: 129 us with a thread per table, accumulating in x_e in
 // global memory, 41 us now; 3,000 tables: 87 us, 13 now.
 template <class T, int MDE>
@@ -1020,7 +1021,7 @@ __global__ void __launch_bounds__(256) k_qr_backsub(int64_t ne_tab, const int32_
                              const int32_t* __restrict__ u_col, const int32_t* __restrict__ u_ret, const int32_t* __restrict__ r_dims,
                              const int32_t* __restrict__ boff_r, const int32_t* __restrict__ e_dims, const int32_t* __restrict__ boff_e,
                              const T* __restrict__ F, const double* __restrict__ Fr, const double* __restrict__ x_r, double* x_e,
-                             const double* __restrict__ w = nullptr) {
+                             const double* __restrict__ w, int lw) {
   const int64_t e = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 3;
   const int l = threadIdx.x & 7;
   const unsigned group = 0xffu << (threadIdx.x & 24);
@@ -1041,10 +1042,10 @@ __global__ void __launch_bounds__(256) k_qr_backsub(int64_t ne_tab, const int32_
 #pragma unroll
         for (int i = 0; i <= j; ++i) U[j][i] = j < n ? (double)Uc[(int64_t)j * M + i] : 1.0;
     }
-    for (int u = t_ptr[e]; u < t_ptr[e + 1]; ++u) {
+    for (int u = t_ptr[e] + (l >> lw); u < t_ptr[e + 1]; u += 8 >> lw) {
       const int r = u_ret[u], dr = r_dims[r], ro = boff_r[r];
       const T* cb = F + off + (int64_t)u_col[u] * M + i0;
-      for (int j = l; j < dr; j += 8) {
+      for (int j = l & ((1 << lw) - 1); j < dr; j += 1 << lw) {
         const double xj = x_r[ro + j];
 #pragma unroll
         for (int i = 0; i < MDE; ++i)
@@ -2168,11 +2169,13 @@ __global__ void k_lsmr_init(int64_t mt, int64_t nr, double lambda, const double*
 template <class T>
 static void launch_qr_backsub(QRPlan* P, const T* F, const double* Fr, const double* x_r, double* x_e, const double* w) {
   if (P->neblocks == 0) return;
-  auto kern = P->max_de <= 4 ? k_qr_backsub<T, 4> : k_qr_backsub<T, 16>;
+  auto kern = P->max_de == 1 ? k_qr_backsub<T, 1> : P->max_de <= 4 ? k_qr_backsub<T, 4> : P->max_de <= 8 ? k_qr_backsub<T, 8> : k_qr_backsub<T, 16>;
+  int lw = 0;
+  while (lw < 3 && (1 << lw) < P->max_dr) ++lw;
   kern<<<(unsigned)grid_for(8 * P->neblocks, 256), 256, 0, P->ctx->stream>>>(
       P->neblocks, P->t_rows.as<int32_t>(), P->t_cols.as<int32_t>(), P->t_raw.as<int64_t>(), P->t_res.as<int64_t>(), P->t_ptr.as<int32_t>(),
       P->u_col.as<int32_t>(), P->u_ret.as<int32_t>(), P->r_dims.as<int32_t>(), P->boff_r.as<int32_t>(), P->e_dims.as<int32_t>(),
-      P->boff_e.as<int32_t>(), F, Fr, x_r, x_e, w);
+      P->boff_e.as<int32_t>(), F, Fr, x_r, x_e, w, lw);
 }
 
 struct LsmrOut {
