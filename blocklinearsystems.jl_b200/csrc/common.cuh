@@ -60,6 +60,22 @@ __device__ __forceinline__ void red_column6(float* col, const float v[6]) {
     default: atomicAdd(col, v[0]); red4(col + 1, v[1], v[2], v[3], v[4]); atomicAdd(col + 5, v[5]); break;
   }
 }
+// Four or eight entries of a column the same way
+__device__ __forceinline__ void red_column4(float* col, const float* v) {
+  switch ((reinterpret_cast<uintptr_t>(col) >> 2) & 3) {
+    case 0: red4(col, v[0], v[1], v[2], v[3]); break;
+    case 2: red2(col, v[0], v[1]); red2(col + 2, v[2], v[3]); break;
+    default: atomicAdd(col, v[0]); red2(col + 1, v[1], v[2]); atomicAdd(col + 3, v[3]); break;
+  }
+}
+__device__ __forceinline__ void red_column8(float* col, const float* v) {
+  switch ((reinterpret_cast<uintptr_t>(col) >> 2) & 3) {
+    case 0: red4(col, v[0], v[1], v[2], v[3]); red4(col + 4, v[4], v[5], v[6], v[7]); break;
+    case 1: atomicAdd(col, v[0]); red2(col + 1, v[1], v[2]); red4(col + 3, v[3], v[4], v[5], v[6]); atomicAdd(col + 7, v[7]); break;
+    case 2: red2(col, v[0], v[1]); red4(col + 2, v[2], v[3], v[4], v[5]); red2(col + 6, v[6], v[7]); break;
+    default: atomicAdd(col, v[0]); red4(col + 1, v[1], v[2], v[3], v[4]); red2(col + 5, v[5], v[6]); atomicAdd(col + 7, v[7]); break;
+  }
+}
 __device__ __forceinline__ void red_column6(double* col, const double v[6]) {
 #pragma unroll
   for (int i = 0; i < 6; ++i) atomicAdd(col + i, v[i]);

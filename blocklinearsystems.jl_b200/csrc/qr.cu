@@ -615,15 +615,15 @@ __global__ void k_qr_free(int64_t t0, int64_t nt, const int32_t* __restrict__ t_
 // J~'r~ into g; MODE 1: the full diagonal blocks D (reduced_diagonal_blocks!, :484-512). from_raw: the same products
 // over the data rows of the raw tables, J'J of the retained columns and J'r (the retained part of the assembly).
 // WHOLE, for the classes of larger tables, takes the registers it needs (in FP32 a lane takes a whole 6 x 6 block of a table
-// with more than 16 pairs); the forms of smaller tables are held to as many as let eight CTAs (FP32) or five run on an SM:
-// unbounded, 128 registers in FP64, 100,000 tables of three or four cameras took 301 us instead of 269 (289 before the early
-// lookups; bounded, tables of ten cameras 577 instead of 518). Sizes other than 6: eight rows by three columns per step;
-// a column at a time, each entry of X was converted to FP64 for each of them (FP32, 9-variable cameras, the diagonal blocks
-// 649 us, 246 now). Bound by the additions into S and by the latency of a table
+// with more than 16 pairs); the forms of smaller tables are held to as many as let gram_ctas of them run on an SM: unbounded,
+// 128 registers in FP64, 100,000 tables of three or four cameras took 301 us instead of 269 (289 without the early lookups;
+// bounded, tables of ten cameras 577 instead of 518). Sizes other than 6: eight rows by three columns per step; a column at a
+// time, each entry of X was converted to FP64 for each of them (FP32, 9-variable cameras, the diagonal blocks 649 us, 228
+// now). Bound by the additions into S and by the latency of a table
 // (its copy, its lookups) at the tables that shared memory holds. 500 x 100,000, all classes: FP32 534 us with a scalar atomic
 // per entry, 374 now; FP64 732, 659 now.
 __host__ __device__ constexpr int gram_ctas(int mode, int bytes, bool all6, bool whole) {
-  return whole ? 1 : bytes == 4 ? (all6 ? 8 : 5) : !all6 ? 1 : mode == 0 ? 5 : 6;
+  return whole ? 1 : bytes == 4 ? (all6 ? 8 : 5) : !all6 ? 4 : mode == 0 ? 5 : 6;
 }
 template <class T, int MODE, bool ALL6, bool WHOLE>
 __global__ void __launch_bounds__(32 * QR_MAX_WARPS, gram_ctas(MODE, sizeof(T), ALL6, WHOLE)) k_qr_gram(int64_t ntab, int warp_bytes, const int32_t* __restrict__ tables,
@@ -696,7 +696,7 @@ __global__ void __launch_bounds__(32 * QR_MAX_WARPS, gram_ctas(MODE, sizeof(T), 
     }
     return gi;
   };
-  const bool whole = WHOLE && sizeof(T) == 4 && npairs > 16;   // a whole block per lane
+  const bool whole = WHOLE && ALL6 && sizeof(T) == 4 && npairs > 16;   // a whole block per lane
   Unit first{0, 0, -1, 0, 0, 0};
   int first_var = 0;
   bool looked_up = ALL6;
@@ -846,16 +846,36 @@ __global__ void __launch_bounds__(32 * QR_MAX_WARPS, gram_ctas(MODE, sizeof(T), 
                 for (int w = 0; w < G; ++w) acc[w][a] += x * y[w];
               }
           }
+          if constexpr (MODE == 0 && sizeof(T) == 4) {
 #pragma unroll
-          for (int w = 0; w < G; ++w)
+            for (int w = 0; w < G; ++w) {
+              if (w0 + w >= d2) break;
+              T v[8];   // below the diagonal -0.0, which leaves every value unchanged
 #pragma unroll
-            for (int a = 0; a < 8; ++a)
-              if (w0 + w < d2 && a0 + a < d1 && (MODE == 1 || !diag || a0 + a <= w0 + w)) atomicAdd(out + w * stride + a0 + a, T(acc[w][a]));
+              for (int a = 0; a < 8; ++a) v[a] = !diag || a0 + a <= w0 + w ? T(acc[w][a]) : T(-0.0);
+              T* col = out + w * stride + a0;
+              const int rows = d1 - a0;
+              if (rows >= 8) {
+                red_column8(col, v);
+              } else {
+                if (rows >= 4) red_column4(col, v);
+#pragma unroll
+                for (int a = 0; a < 8; ++a)
+                  if (a < rows && (rows < 4 || a >= 4)) atomicAdd(col + a, v[a]);
+              }
+            }
+          } else {
+#pragma unroll
+            for (int w = 0; w < G; ++w)
+#pragma unroll
+              for (int a = 0; a < 8; ++a)
+                if (w0 + w < d2 && a0 + a < d1 && (MODE == 1 || !diag || a0 + a <= w0 + w)) atomicAdd(out + w * stride + a0 + a, T(acc[w][a]));
+          }
         }
       }
     }
   };
-  if constexpr (WHOLE && sizeof(T) == 4) {
+  if constexpr (WHOLE && ALL6 && sizeof(T) == 4) {
     if (whole) units(std::integral_constant<int, 6>{});
     else units(std::integral_constant<int, 3>{});
   } else {
@@ -1745,8 +1765,10 @@ static void gram(QRPlan* P, T* S, bool dense, double* g, const T* F, const doubl
     // a table of 3 KB or more can have 16 pairs (5 entries of 6 columns by 10 rows)
     if constexpr (std::is_same<T, float>::value && MODE == 0)
       if (P->all6 && wb >= 3072) kern = k_qr_gram<T, MODE, true, true>;
-    if constexpr (std::is_same<T, double>::value)   // shared memory holds fewer than 20 of these tables
-      if (P->all6 && wb >= 11 * 1024) kern = k_qr_gram<T, MODE, true, true>;
+    if (wb >= 11 * 1024) {   // shared memory holds fewer than 20 of these tables
+      if (!P->all6) kern = k_qr_gram<T, MODE, false, true>;
+      else if (std::is_same<T, double>::value) kern = k_qr_gram<T, MODE, true, true>;
+    }
     const int wpc = std::max(1, tables_per_cta(wb, 32, warp_cap(reinterpret_cast<const void*>(kern))));
     const size_t smem = (size_t)(wb * wpc);
     set_smem(reinterpret_cast<const void*>(kern), smem);
