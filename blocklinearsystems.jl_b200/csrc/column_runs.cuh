@@ -571,7 +571,7 @@ static bool runs_contiguous(const RunInput& in) {
 }
 
 template <class T>
-static bool build_run_schedule(RunSchedule& R, const RunInput& in, int exact, int mdr, int mde, cudaStream_t s) {
+static bool build_run_schedule(RunSchedule& R, const RunInput& in, int exact, int mdr, int mde, cudaStream_t s, SmallBufs& small) {
   constexpr int EPC = 16 / (int)sizeof(T);
   R.exact = exact;
   R.mdr = mdr;
@@ -752,27 +752,34 @@ static bool build_run_schedule(RunSchedule& R, const RunInput& in, int exact, in
     }
   }
   if (bad) return false;
-  std::vector<int4> items, segs;
-  std::vector<uint4> blob;
-  size_t n_i = 0, n_s = 0, n_b = 0;
-  for (auto& o : out) { n_i += o.items.size(); n_s += o.segs.size(); n_b += o.blob.size(); }
+  // the columns' parts one after another (the blob is tens of MB: uninitialised memory, filled by all threads)
+  std::vector<int64_t> at_i(in.nrb + 1, 0), at_s(in.nrb + 1, 0), at_b(in.nrb + 1, 0);
+  for (int64_t r = 0; r < in.nrb; ++r) {
+    at_i[r + 1] = at_i[r] + (int64_t)out[r].items.size();
+    at_s[r + 1] = at_s[r] + (int64_t)out[r].segs.size();
+    at_b[r + 1] = at_b[r] + (int64_t)out[r].blob.size();
+  }
+  const int64_t n_b = at_b[in.nrb];
   if (n_b >= INT32_MAX) return false;
-  items.reserve(n_i);
-  segs.reserve(n_s);
-  blob.reserve(n_b);
-  for (auto& o : out) {
-    const int32_t s0 = (int32_t)segs.size(), b0 = (int32_t)blob.size();
-    for (size_t i = 0; i < o.items.size(); i += 2) {
-      items.push_back(make_int4(o.items[i].x, o.items[i].y + s0, o.items[i].z, o.items[i].w));
-      items.push_back(o.items[i + 1]);
+  std::vector<int4> items(at_i[in.nrb]), segs(at_s[in.nrb]);
+  const HostArray<uint4> blob(n_b);
+#pragma omp parallel for schedule(dynamic, 8)
+  for (int64_t r = 0; r < in.nrb; ++r) {
+    ColOut& o = out[r];
+    for (size_t i = 0; i < o.items.size(); ++i) {
+      items[at_i[r] + i] = o.items[i];
+      if (i % 2 == 0) items[at_i[r] + i].y += (int32_t)at_s[r];
     }
-    for (const int4& x : o.segs) segs.push_back(make_int4(x.x + b0, x.y, x.z, x.w));
-    blob.insert(blob.end(), o.blob.begin(), o.blob.end());
+    for (size_t i = 0; i < o.segs.size(); ++i) {
+      segs[at_s[r] + i] = o.segs[i];
+      segs[at_s[r] + i].x += (int32_t)at_b[r];
+    }
+    if (!o.blob.empty()) std::memcpy(blob.get() + at_b[r], o.blob.data(), sizeof(uint4) * o.blob.size());
     o = ColOut();
   }
-  upload(R.items_d, items, s);
-  upload(R.segs, segs, s);
-  upload(R.blob, blob, s);
+  small.add(R.items_d, items, s);
+  small.add(R.segs, segs, s);
+  small.add(R.blob, blob, s);
   std::vector<int4> split;   // FP32: the split columns
   for (size_t i = 0; sizeof(T) == 4 && i < items.size(); i += 2)
     if (items[i].w == 0) {
@@ -781,10 +788,9 @@ static bool build_run_schedule(RunSchedule& R, const RunInput& in, int exact, in
     }
   R.nsplit = (int64_t)split.size();
   if (R.nsplit) {
-    upload(R.split, split, s);
-    R.dpart.alloc(sizeof(double) * (items.size() / 2) * mdr * mdr);
+    small.add(R.split, split, s);
+    small.reserve(R.dpart, sizeof(double) * (items.size() / 2) * mdr * mdr);
   }
-  BLS_CUDA(cudaStreamSynchronize(s));   // the uploads read this function's vectors
   R.items = (int64_t)items.size() / 2;
   R.tile_bytes = (int)((tile + 15) / 16 * 16);
   R.blob_bytes = (int)(16 * max_chunks);

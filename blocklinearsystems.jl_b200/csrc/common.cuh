@@ -2,6 +2,8 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <cstdint>
+#include <cstring>
+#include <memory>
 #include <mutex>
 #include <set>
 #include <string>
@@ -102,16 +104,19 @@ inline void allow_smem(const void* kernel) {
 
 inline int grid_for(int64_t n, int threads) { return (int)((n + threads - 1) / threads); }
 
-// A device buffer that frees itself.
+// A device buffer that frees itself (unless it is a part of another one, see SmallBufs).
 struct DevBuf {
   void* p = nullptr;
   size_t bytes = 0;
+  bool owned = true;
   DevBuf() = default;
   DevBuf(const DevBuf&) = delete;
   DevBuf& operator=(const DevBuf&) = delete;
-  ~DevBuf() { if (p) cudaFree(p); }
+  ~DevBuf() { if (p && owned) cudaFree(p); }
   void alloc(size_t b) {
-    if (p) { cudaFree(p); p = nullptr; }
+    if (p && owned) cudaFree(p);
+    p = nullptr;
+    owned = true;
     bytes = b;
     if (b) BLS_CUDA(cudaMalloc(&p, b));
   }
@@ -123,6 +128,75 @@ void upload(DevBuf& buf, const std::vector<T>& v, cudaStream_t s) {
   buf.alloc(v.size() * sizeof(T));
   if (!v.empty()) BLS_CUDA(cudaMemcpyAsync(buf.p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, s));
 }
+
+// A host array that is not initialised (a large std::vector is, by one thread).
+template <class T>
+struct HostArray {
+  std::unique_ptr<T[]> p;
+  int64_t n = 0;
+  HostArray() = default;
+  explicit HostArray(int64_t count) : p(new T[count > 0 ? (size_t)count : 1]), n(count) {}
+  T* get() const { return p.get(); }
+  T& operator[](int64_t i) const { return p[(size_t)i]; }
+};
+
+// Many small device arrays in one allocation and few copies (an allocation takes up to 0.4 ms): add() takes an array's
+// contents, reserve() room without contents, and flush() makes the allocation and points the buffers into it; `arena` has to
+// outlive them, and this object the copies. Above kSmall bytes a buffer gets its own allocation at once.
+class SmallBufs {
+ public:
+  template <class T>
+  void add(DevBuf& b, const T* v, int64_t n, cudaStream_t s) {
+    const size_t bytes = (size_t)n * sizeof(T);
+    if (bytes > kSmall) {
+      b.alloc(bytes);
+      BLS_CUDA(cudaMemcpyAsync(b.p, v, bytes, cudaMemcpyHostToDevice, s));
+      return;
+    }
+    b.alloc(0);
+    if (!bytes) return;
+    if (chunks.empty() || used + bytes > kChunk) {
+      chunks.emplace_back(new unsigned char[kChunk]);
+      used = 0;
+    }
+    std::memcpy(chunks.back().get() + used, v, bytes);
+    parts.push_back({&b, (chunks.size() - 1) * kChunk + used, bytes, true});
+    used = (used + bytes + 255) / 256 * 256;
+  }
+  template <class T>
+  void add(DevBuf& b, const std::vector<T>& v, cudaStream_t s) { add(b, v.data(), (int64_t)v.size(), s); }
+  template <class T>
+  void add(DevBuf& b, const HostArray<T>& v, cudaStream_t s) { add(b, v.get(), v.n, s); }
+  void reserve(DevBuf& b, size_t bytes) {
+    if (bytes > kSmall) {
+      b.alloc(bytes);
+      return;
+    }
+    b.alloc(0);
+    parts.push_back({&b, room, bytes, false});
+    room += (bytes + 255) / 256 * 256;
+  }
+  void flush(DevBuf& arena, cudaStream_t s) {
+    const size_t contents = chunks.empty() ? 0 : (chunks.size() - 1) * kChunk + used;
+    arena.alloc(contents + room);
+    unsigned char* base = arena.as<unsigned char>();
+    for (size_t i = 0; i < chunks.size(); ++i)
+      BLS_CUDA(cudaMemcpyAsync(base + i * kChunk, chunks[i].get(), i + 1 < chunks.size() ? kChunk : used, cudaMemcpyHostToDevice, s));
+    for (const Part& x : parts) {
+      x.buf->p = base + (x.contents ? 0 : contents) + x.off;
+      x.buf->bytes = x.bytes;
+      x.buf->owned = false;
+    }
+    parts.clear();
+  }
+
+ private:
+  static constexpr size_t kSmall = 1 << 20, kChunk = 4 << 20;
+  struct Part { DevBuf* buf; size_t off, bytes; bool contents; };
+  std::vector<Part> parts;
+  std::vector<std::unique_ptr<unsigned char[]>> chunks;
+  size_t used = 0, room = 0;   // bytes of the last chunk, bytes reserved
+};
 
 // One block of symmetrifyfull!: data[src ...] (rd x cd, column-major) to mat's rows rs.. and columns cs.., and
 // transposed to rows cs.. and columns rs.. unless diag.

@@ -132,6 +132,7 @@ struct SchurPlan {
   cudaEvent_t ev_free = nullptr, ev_points = nullptr, ev_in[kStages + 1] = {};
   // scratch: E^-1 (FP64, and FP32 for the mixed form), z, status
   DevBuf Einv64, Einv32, z, status;
+  DevBuf arena, runs_arena[2];   // the small ones of these and of the structure's arrays; those of run schedules built later
   DevBuf acc1;     // one FP64 accumulator (bls_hessian_bilinear)
   DevBuf w_apply;  // per point E^-1 C x of bls_schur_apply_elimination (ne doubles, allocated at its first call)
   DevBuf t_apply;  // per point C x of bls_schur_apply_elimination on the 3-variable fast path (3 neblocks doubles)
@@ -152,12 +153,15 @@ struct SchurPlan {
   }
 };
 
-static std::vector<int32_t> to32(const int64_t* a, int64_t n, const char* what) {
-  std::vector<int32_t> v((size_t)n);
+static HostArray<int32_t> to32(const int64_t* a, int64_t n, const char* what) {
+  HostArray<int32_t> v(n);
+  int out = 0;
+#pragma omp parallel for reduction(| : out) if (n > 65536)
   for (int64_t i = 0; i < n; ++i) {
-    if (a[i] < INT32_MIN || a[i] > INT32_MAX) throw Error(BLS_EUNSUPPORTED, std::string(what) + " exceeds the 32-bit index range of this build");
+    out |= a[i] < INT32_MIN || a[i] > INT32_MAX;
     v[i] = (int32_t)a[i];
   }
+  if (out) throw Error(BLS_EUNSUPPORTED, std::string(what) + " exceeds the 32-bit index range of this build");
   return v;
 }
 
@@ -2150,15 +2154,15 @@ static SchurPlan* plan_create(bls_ctx* ctx, const bls_schur_plan_desc* d) {
       }
     }
     const int64_t nnz = Scolptr[nr];
-    if (d->diag_inds)
-      for (int64_t i = 0; i < nr; ++i)
-        if (d->diag_inds[i] < 0 || d->diag_inds[i] >= nnz) throw Error(BLS_EINVAL, "diag_inds out of range");
-    if (d->r_to_s_map)
-      for (int64_t i = 0; i < d->R_length; ++i)
-        if (d->r_to_s_map[i] < -1 || d->r_to_s_map[i] >= nnz) throw Error(BLS_EINVAL, "r_to_s_map out of range");
-    if (d->S_rowval)
-      for (int64_t q = 0; q < nnz; ++q)
-        if (d->S_rowval[q] < 0 || d->S_rowval[q] >= nr) throw Error(BLS_EINVAL, "S_rowval out of range");
+    auto within = [](const int64_t* a, int64_t n, int64_t lo, int64_t hi) {
+      int out = 0;
+#pragma omp parallel for reduction(| : out) if (n > 65536)
+      for (int64_t i = 0; i < n; ++i) out |= a[i] < lo || a[i] >= hi;
+      return out == 0;
+    };
+    if (d->diag_inds && !within(d->diag_inds, nr, 0, nnz)) throw Error(BLS_EINVAL, "diag_inds out of range");
+    if (d->r_to_s_map && !within(d->r_to_s_map, d->R_length, -1, nnz)) throw Error(BLS_EINVAL, "r_to_s_map out of range");
+    if (d->S_rowval && !within(d->S_rowval, nnz, 0, nr)) throw Error(BLS_EINVAL, "S_rowval out of range");
   }
   for (int64_t e = 0; e < neb; ++e)
     for (int64_t c = d->eliminated_ptr[e]; c < d->eliminated_ptr[e + 1]; ++c)
@@ -2175,46 +2179,51 @@ static SchurPlan* plan_create(bls_ctx* ctx, const bls_schur_plan_desc* d) {
     }
   // pair lists per block, cut into items (columns in parallel; each column's pairs keep ascending c2 per block)
   std::vector<int64_t> col_npairs(nrb, 0);
-  std::vector<std::vector<int32_t>> col_c1(nrb), col_c2(nrb), col_cnt(nrb);
+  std::vector<std::vector<int32_t>> col_c1(nrb), col_c2(nrb), col_cnt(nrb), col_slots(nrb);   // col_slots: 6/3 plans only
   int64_t missing = -1;
-#pragma omp parallel for schedule(dynamic, 8)
-  for (int64_t r2 = 0; r2 < nrb; ++r2) {
-    const int64_t kb = bcolptr[r2], ke = bcolptr[r2 + 1], nbc = ke - kb;
-    std::vector<int32_t> cnt(nbc + 1, 0);
-    std::vector<int32_t> slot_of;   // slot of each pair in visit order
-    std::vector<int32_t> pc1, pc2;
-    for (int32_t q = rptr[r2]; q < rptr[r2 + 1]; ++q) {
-      const int32_t c2 = rentry[q];
-      const int64_t e = entry_elim[c2];
-      for (int64_t c1 = d->eliminated_ptr[e]; c1 <= c2; ++c1) {
-        const int64_t r1 = d->entry_retained[c1];
-        const int64_t* lo = browval.data() + kb;
-        const int64_t* hi = browval.data() + ke;
-        const int64_t* f = std::lower_bound(lo, hi, r1);
-        if (f == hi || *f != r1) {
+#pragma omp parallel
+  {
+    std::vector<int32_t> slot_at(nrb, -1), pc1, pc2, pos;   // slot_at: the slot of each block row in the thread's column
+#pragma omp for schedule(dynamic, 8)
+    for (int64_t r2 = 0; r2 < nrb; ++r2) {
+      const int64_t kb = bcolptr[r2], nbc = bcolptr[r2 + 1] - kb;
+      for (int64_t k = 0; k < nbc; ++k) slot_at[browval[kb + k]] = (int32_t)k;
+      std::vector<int32_t> cnt(nbc + 1, 0);
+      std::vector<int32_t> slot_of;   // slot of each pair in visit order
+      pc1.clear();
+      pc2.clear();
+      for (int32_t q = rptr[r2]; q < rptr[r2 + 1]; ++q) {
+        const int32_t c2 = rentry[q];
+        const int64_t e = entry_elim[c2];
+        for (int64_t c1 = d->eliminated_ptr[e]; c1 <= c2; ++c1) {
+          const int64_t r1 = d->entry_retained[c1];
+          const int32_t sl = slot_at[r1];
+          if (sl < 0) {
 #pragma omp critical
-          missing = r1 * nrb + r2;
-          continue;
+            missing = r1 * nrb + r2;
+            continue;
+          }
+          slot_of.push_back(sl);
+          pc1.push_back((int32_t)c1);
+          pc2.push_back(c2);
+          cnt[sl + 1] += 1;
         }
-        const int32_t sl = (int32_t)(f - lo);
-        slot_of.push_back(sl);
-        pc1.push_back((int32_t)c1);
-        pc2.push_back(c2);
-        cnt[sl + 1] += 1;
       }
+      for (int64_t i = 0; i < nbc; ++i) cnt[i + 1] += cnt[i];
+      std::vector<int32_t> o1(pc1.size()), o2(pc2.size());
+      pos.assign(cnt.begin(), cnt.end() - 1);
+      for (size_t i = 0; i < pc1.size(); ++i) {
+        const int32_t sl = slot_of[i];
+        o1[pos[sl]] = pc1[i];
+        o2[pos[sl]++] = pc2[i];
+      }
+      for (int64_t k = 0; k < nbc; ++k) slot_at[browval[kb + k]] = -1;
+      col_npairs[r2] = (int64_t)o1.size();
+      col_c1[r2].swap(o1);
+      col_c2[r2].swap(o2);
+      col_cnt[r2].swap(cnt);
+      if (P->uniform36) col_slots[r2].swap(slot_of);
     }
-    for (int64_t i = 0; i < nbc; ++i) cnt[i + 1] += cnt[i];
-    std::vector<int32_t> o1(pc1.size()), o2(pc2.size());
-    std::vector<int32_t> pos(cnt.begin(), cnt.end() - 1);
-    for (size_t i = 0; i < pc1.size(); ++i) {
-      const int32_t sl = slot_of[i];
-      o1[pos[sl]] = pc1[i];
-      o2[pos[sl]++] = pc2[i];
-    }
-    col_c1[r2].swap(o1);
-    col_c2[r2].swap(o2);
-    col_cnt[r2].swap(cnt);
-    col_npairs[r2] = (int64_t)pc1.size();
   }
   if (missing >= 0)
     throw Error(BLS_EPATTERN, "The sparse pattern has no block (" + std::to_string(missing / nrb + 1) + ", " + std::to_string(missing % nrb + 1) + ")");
@@ -2222,54 +2231,65 @@ static SchurPlan* plan_create(bls_ctx* ctx, const bls_schur_plan_desc* d) {
   for (int64_t r2 = 0; r2 < nrb; ++r2) npairs += col_npairs[r2];
   if (npairs >= INT32_MAX) throw Error(BLS_EUNSUPPORTED, "more than 2^31 coupling pairs are not supported");
   P->npairs = npairs;
-  std::vector<int32_t> pair_c1(npairs), pair_c2(npairs), it_block, it_start, it_info;
-  int64_t off = 0;
+  // the columns' lists one after another
+  std::vector<int64_t> pair_at(nrb + 1, 0), item_at(nrb + 1, 0);
   for (int64_t r2 = 0; r2 < nrb; ++r2) {
-    std::copy(col_c1[r2].begin(), col_c1[r2].end(), pair_c1.begin() + off);
-    std::copy(col_c2[r2].begin(), col_c2[r2].end(), pair_c2.begin() + off);
+    int64_t n = 0;
+    for (size_t sl = 0; sl + 1 < col_cnt[r2].size(); ++sl) n += (col_cnt[r2][sl + 1] - col_cnt[r2][sl] + PAIR_CHUNK - 1) / PAIR_CHUNK;
+    pair_at[r2 + 1] = pair_at[r2] + col_npairs[r2];
+    item_at[r2 + 1] = item_at[r2] + n;
+  }
+  const HostArray<int32_t> pair_c1(npairs), pair_c2(npairs);
+  std::vector<int32_t> it_block(item_at[nrb]), it_start(item_at[nrb]), it_info(item_at[nrb]);
+#pragma omp parallel for schedule(dynamic, 8)
+  for (int64_t r2 = 0; r2 < nrb; ++r2) {
+    const int64_t off = pair_at[r2];
+    int64_t it = item_at[r2];
+    std::copy(col_c1[r2].begin(), col_c1[r2].end(), pair_c1.get() + off);
+    std::copy(col_c2[r2].begin(), col_c2[r2].end(), pair_c2.get() + off);
     const auto& cnt = col_cnt[r2];
     for (int64_t sl = 0; sl + 1 < (int64_t)cnt.size(); ++sl) {
       const int32_t a = cnt[sl], b = cnt[sl + 1];
-      if (b == a) continue;
-      const int nchunk = (b - a + PAIR_CHUNK - 1) / PAIR_CHUNK;
-      for (int32_t x = a; x < b; x += PAIR_CHUNK) {
-        it_block.push_back((int32_t)(bcolptr[r2] + sl));
-        it_start.push_back((int32_t)(off + x));
-        it_info.push_back(std::min(PAIR_CHUNK, b - x) | ((nchunk == 1 ? 1 : 0) << 16));
+      const bool solo = b - a <= PAIR_CHUNK;
+      for (int32_t x = a; x < b; x += PAIR_CHUNK, ++it) {
+        it_block[it] = (int32_t)(bcolptr[r2] + sl);
+        it_start[it] = (int32_t)(off + x);
+        it_info[it] = std::min(PAIR_CHUNK, b - x) | ((solo ? 1 : 0) << 16);
       }
     }
-    off += col_npairs[r2];
     std::vector<int32_t>().swap(col_c1[r2]);
     std::vector<int32_t>().swap(col_c2[r2]);
   }
   P->nitems = (int64_t)it_block.size();
   // fast path: uniform 6/3 blocks in the canonical layout, and pairs that pack into {c1, e | (c2 - c1) << 24}
-  std::vector<int2> packed;
+  HostArray<int2> packed;
   if (P->uniform36 && neb < (1 << 24)) {
     bool canon = true;
     for (int64_t e = 0; e < neb && canon; ++e) canon = d->eoffsets[e] == 9 * e;
     for (int64_t c = 0; c < nc && canon; ++c) canon = d->coffsets[c] == 18 * c;
     if (canon) {
-      packed.resize(npairs);
-      for (int64_t q = 0; q < npairs && canon; ++q) {
-        const int32_t c1 = pair_c1[q], c2 = pair_c2[q];
-        const int32_t dc = c2 - c1;
-        if (dc < 0 || dc > 127) canon = false;
-        packed[q] = make_int2(c1, entry_elim[c2] | (dc << 24));
+      packed = HostArray<int2>(npairs);
+      int far = 0;
+#pragma omp parallel for reduction(| : far) if (npairs > 65536)
+      for (int64_t q = 0; q < npairs; ++q) {
+        const int32_t c1 = pair_c1[q], c2 = pair_c2[q], dc = c2 - c1;
+        far |= dc < 0 || dc > 127;
+        packed[q] = make_int2(c1, (int32_t)((uint32_t)entry_elim[c2] | ((uint32_t)dc << 24)));
       }
+      canon = far == 0;
     }
     P->fast36 = canon;
   }
   // column-kernel arrays: visits in the reference's retained_entry order (column by column, ascending coupling)
-  std::vector<int2> vrec;
-  std::vector<int32_t> vbase;
-  std::vector<uint16_t> voff;
+  HostArray<int2> vrec;
+  HostArray<int32_t> vbase;
+  HostArray<uint16_t> voff;
   std::vector<int64_t> cbase;
   std::vector<int32_t> ch;
   if (P->fast36) {
-    vrec.resize(nc);
-    vbase.resize(nc);
-    voff.reserve(npairs);
+    vrec = HostArray<int2>(nc);
+    vbase = HostArray<int32_t>(nc);
+    voff = HostArray<uint16_t>(npairs);
     cbase.resize(nrb);
     ch.resize(nrb);
     for (int64_t r2 = 0; r2 < nrb; ++r2) {
@@ -2277,21 +2297,22 @@ static SchurPlan* plan_create(bls_ctx* ctx, const bls_schur_plan_desc* d) {
       ch[r2] = (int32_t)col_h[r2];
       P->max_col_h = std::max<int64_t>(P->max_col_h, col_h[r2]);
       if (col_h[r2] > 65535) P->fast36 = false;
+    }
+#pragma omp parallel for schedule(dynamic, 8)
+    for (int64_t r2 = 0; r2 < nrb; ++r2) {
+      int64_t o = pair_at[r2];
+      const std::vector<int32_t>& slots = col_slots[r2];   // of the column's pairs in visit order
       for (int32_t q = rptr[r2]; q < rptr[r2 + 1]; ++q) {
         const int32_t c2 = rentry[q];
         const int64_t e = entry_elim[c2], p0 = d->eliminated_ptr[e], j = c2 - p0;
         vrec[q] = make_int2((int32_t)p0, (int32_t)(e | (j << 24)));
-        vbase[q] = (int32_t)voff.size();
-        for (int64_t i = 0; i <= j; ++i) {
-          const int64_t r1 = d->entry_retained[p0 + i];
-          const int64_t* lo = browval.data() + bcolptr[r2];
-          const int64_t* hi = browval.data() + bcolptr[r2 + 1];
-          const int64_t k = std::lower_bound(lo, hi, r1) - browval.data();
-          voff.push_back((uint16_t)brow_off[k]);
-        }
+        vbase[q] = (int32_t)o;
+        for (int64_t i = 0; i <= j; ++i, ++o) voff[o] = (uint16_t)brow_off[bcolptr[r2] + slots[o - pair_at[r2]]];
       }
+      std::vector<int32_t>().swap(col_slots[r2]);
     }
   }
+  SmallBufs small;
   {
     P->points3 = true;
     for (int64_t e = 0; e < neb && P->points3; ++e) P->points3 = d->e_dims[e] == 3 && d->eoffsets[e] == 9 * e;
@@ -2330,8 +2351,8 @@ static SchurPlan* plan_create(bls_ctx* ctx, const bls_schur_plan_desc* d) {
     // cannot be built, or when it is chosen by name: ensure_gather, ensure_runs); every other plan has the runs only
     for (int sd = 0; sd < 2; ++sd) {
       auto runs = [&] {
-        return contiguous && (sd == 0 ? build_run_schedule<float>(P->runs[0], in, run_exact, P->max_dr, P->max_de, s)
-                                      : build_run_schedule<double>(P->runs[1], in, run_exact, P->max_dr, P->max_de, s));
+        return contiguous && (sd == 0 ? build_run_schedule<float>(P->runs[0], in, run_exact, P->max_dr, P->max_de, s, small)
+                                      : build_run_schedule<double>(P->runs[1], in, run_exact, P->max_dr, P->max_de, s, small));
       };
       auto stage = [&] {
         return P->stage_ok[sd] = build_stage_schedule(P.get(), sd, s, nrb, rptr, rentry, entry_elim, d->eliminated_ptr, d->entry_retained,
@@ -2390,86 +2411,87 @@ static SchurPlan* plan_create(bls_ctx* ctx, const bls_schur_plan_desc* d) {
     P->staged = true;
   }
   // uploads
-  upload(P->r_dims, to32(d->r_dims, nrb, "r_dims"), s);
-  upload(P->boffsets_r, to32(boff_r.data(), nrb, "boffsets_r"), s);
-  upload(P->e_dims, to32(d->e_dims, neb, "e_dims"), s);
-  upload(P->boffsets_e, to32(boff_e.data(), neb, "boffsets_e"), s);
-  upload(P->eoffsets, to32(d->eoffsets, neb, "eoffsets"), s);
-  upload(P->eliminated_ptr, to32(d->eliminated_ptr, neb + 1, "eliminated_ptr"), s);
-  upload(P->entry_retained, to32(d->entry_retained, nc, "entry_retained"), s);
-  upload(P->coffsets, to32(d->coffsets, nc, "coffsets"), s);
-  upload(P->entry_eliminated, entry_elim, s);
-  upload(P->retained_ptr, rptr, s);
-  upload(P->retained_entry, rentry, s);
-  upload(P->block_r1, b_r1, s);
-  upload(P->block_r2, b_r2, s);
-  upload(P->block_stride_sparse, b_stride, s);
-  upload(P->block_base_sparse, b_base, s);
-  upload(P->block_base_dense, b_base_dense, s);
+  small.add(P->r_dims, to32(d->r_dims, nrb, "r_dims"), s);
+  small.add(P->boffsets_r, to32(boff_r.data(), nrb, "boffsets_r"), s);
+  small.add(P->e_dims, to32(d->e_dims, neb, "e_dims"), s);
+  small.add(P->boffsets_e, to32(boff_e.data(), neb, "boffsets_e"), s);
+  small.add(P->eoffsets, to32(d->eoffsets, neb, "eoffsets"), s);
+  small.add(P->eliminated_ptr, to32(d->eliminated_ptr, neb + 1, "eliminated_ptr"), s);
+  small.add(P->entry_retained, to32(d->entry_retained, nc, "entry_retained"), s);
+  small.add(P->coffsets, to32(d->coffsets, nc, "coffsets"), s);
+  small.add(P->entry_eliminated, entry_elim, s);
+  small.add(P->retained_ptr, rptr, s);
+  small.add(P->retained_entry, rentry, s);
+  small.add(P->block_r1, b_r1, s);
+  small.add(P->block_r2, b_r2, s);
+  small.add(P->block_stride_sparse, b_stride, s);
+  small.add(P->block_base_sparse, b_base, s);
+  small.add(P->block_base_dense, b_base_dense, s);
   if (P->fast36) {
     {
       int64_t kmax = 0;
       for (int64_t e = 0; e < neb; ++e) kmax = std::max<int64_t>(kmax, d->eliminated_ptr[e + 1] - d->eliminated_ptr[e]);
       P->tiles_ok = P->has_sparse && 18 * kmax <= 2048;
     }
-    upload(P->vis_rec, vrec, s);
-    upload(P->vis_base, vbase, s);
-    upload(P->vis_off, voff, s);
-    upload(P->col_base, cbase, s);
-    upload(P->col_h, ch, s);
-    upload(P->pair_packed, packed, s);
+    small.add(P->vis_rec, vrec, s);
+    small.add(P->vis_base, vbase, s);
+    small.add(P->vis_off, voff, s);
+    small.add(P->col_base, cbase, s);
+    small.add(P->col_h, ch, s);
+    small.add(P->pair_packed, packed, s);
     if (P->staged) {
-      upload(P->st_block, sb_all, s);
-      upload(P->st_start, ss_all, s);
-      upload(P->st_info, si_all, s);
+      small.add(P->st_block, sb_all, s);
+      small.add(P->st_start, ss_all, s);
+      small.add(P->st_info, si_all, s);
     }
   } else {
-    upload(P->pair_c1, pair_c1, s);
-    upload(P->pair_c2, pair_c2, s);
+    small.add(P->pair_c1, pair_c1, s);
+    small.add(P->pair_c2, pair_c2, s);
   }
-  upload(P->item_block, it_block, s);
-  upload(P->item_start, it_start, s);
-  upload(P->item_info, it_info, s);
+  small.add(P->item_block, it_block, s);
+  small.add(P->item_start, it_start, s);
+  small.add(P->item_info, it_info, s);
   if (P->has_sparse) {
     if (d->diag_inds) {
       P->diag_inds_host.assign(d->diag_inds, d->diag_inds + nr);
-      upload(P->diag_inds, P->diag_inds_host, s);
+      small.add(P->diag_inds, P->diag_inds_host, s);
     }
     if (d->r_to_s_map && d->R_length > 0) {
       P->R_length = d->R_length;
-      std::vector<int64_t> m(d->r_to_s_map, d->r_to_s_map + d->R_length);
-      upload(P->r_to_s, m, s);
+      small.add(P->r_to_s, d->r_to_s_map, d->R_length, s);
     }
     if (d->S_rowval) {
-      std::vector<int32_t> rv = to32(d->S_rowval, P->nnzS, "S_rowval");
-      std::vector<int32_t> cl(P->nnzS);
+      const HostArray<int32_t> rv = to32(d->S_rowval, P->nnzS, "S_rowval"), cl(P->nnzS);
+#pragma omp parallel for if (P->nnzS > 65536)
       for (int64_t j = 0; j < nr; ++j)
         for (int64_t q = Scolptr[j]; q < Scolptr[j + 1]; ++q) cl[q] = (int32_t)j;
-      upload(P->S_rowval, rv, s);
-      upload(P->S_col, cl, s);
+      small.add(P->S_rowval, rv, s);
+      small.add(P->S_col, cl, s);
     }
     if (d->diag_inds && P->R_length < INT32_MAX) {
       bool inside = true;
       for (int64_t i = 0; i < nr && inside; ++i) inside = d->diag_inds[i] >= Scolptr[i] && d->diag_inds[i] < Scolptr[i + 1];
       if (inside) {
-        std::vector<int32_t> rf(P->nnzS, -1);
+        const HostArray<int32_t> rf(P->nnzS);
+#pragma omp parallel for if (P->nnzS > 65536)
+        for (int64_t q = 0; q < P->nnzS; ++q) rf[q] = -1;
         for (int64_t i = 0; i < P->R_length; ++i)
           if (d->r_to_s_map[i] >= 0) rf[d->r_to_s_map[i]] = (int32_t)i;
-        upload(P->r_from, rf, s);
-        upload(P->S_colptr, Scolptr, s);
+        small.add(P->r_from, rf, s);
+        small.add(P->S_colptr, Scolptr, s);
         P->reset_fused = true;
       }
     }
   }
-  P->Einv64.alloc(sizeof(double) * std::max<int64_t>(P->E_length, 1));
-  if (!P->fast36) P->Einv32.alloc(sizeof(float) * std::max<int64_t>(P->E_length, 1));
-  P->z.alloc(sizeof(double) * std::max<int64_t>(ne, 1));
-  if (P->fast36) P->Einv12.alloc(sizeof(double) * 12 * neb);   // sized for FP64; the FP32 form uses half
+  small.reserve(P->Einv64, sizeof(double) * std::max<int64_t>(P->E_length, 1));
+  if (!P->fast36) small.reserve(P->Einv32, sizeof(float) * std::max<int64_t>(P->E_length, 1));
+  small.reserve(P->z, sizeof(double) * std::max<int64_t>(ne, 1));
+  if (P->fast36) small.reserve(P->Einv12, sizeof(double) * 12 * neb);   // sized for FP64; the FP32 form uses half
   if (P->stage_ok[0] || P->stage_ok[1] || P->runs[0].ok || P->runs[1].ok) P->kernel = 5;   // column-owned: the default
-  if (P->points3) P->EZ.alloc(sizeof(double) * 12 * neb);
-  P->status.alloc(sizeof(Status));
-  Status init{NONE, NONE, NONE, 0};
-  BLS_CUDA(cudaMemcpyAsync(P->status.p, &init, sizeof(Status), cudaMemcpyHostToDevice, s));
+  if (P->points3) small.reserve(P->EZ, sizeof(double) * 12 * neb);
+  const Status init{NONE, NONE, NONE, 0};
+  small.add(P->status, &init, 1, s);
+  small.flush(P->arena, s);
   BLS_CUDA(cudaMallocHost(&P->host_status, sizeof(Status)));
   BLS_CUDA(cudaStreamSynchronize(s));
   return P.release();
@@ -2748,8 +2770,14 @@ static void ensure_runs(SchurPlan* P) {
   for (int64_t c = 0; c < P->ncoup; ++c) co[c] = 18 * c;
   const RunInput in{P->nrblocks, P->neblocks, P->C_length, rd.data(), ed.data(), L.eptr.data(), L.eret.data(), co.data(), &L.rptr, &L.rentry,
                     &L.entry_elim, &L.bcolptr, &L.browval};
-  if (!P->runs[0].ok) build_run_schedule<float>(P->runs[0], in, 6, 6, 3, P->ctx->stream);
-  if (!P->runs[1].ok) build_run_schedule<double>(P->runs[1], in, 6, 6, 3, P->ctx->stream);
+  for (int sd = 0; sd < 2; ++sd) {
+    if (P->runs[sd].ok) continue;
+    SmallBufs small;
+    if (sd == 0 ? build_run_schedule<float>(P->runs[0], in, 6, 6, 3, P->ctx->stream, small)
+                : build_run_schedule<double>(P->runs[1], in, 6, 6, 3, P->ctx->stream, small))
+      small.flush(P->runs_arena[sd], P->ctx->stream);
+    BLS_CUDA(cudaStreamSynchronize(P->ctx->stream));
+  }
 }
 
 // Whether the plan's choice of kernel is k_runs / k_runs_any (where its schedule exists): always for block sizes other
