@@ -7,9 +7,9 @@ every problem: the union's S is block diagonal by problem, and each kernel launc
 problem's damping lambda_p is folded into its scalings (lambda_p * scaling, formed in FP64 exactly as the kernels form
 lambda * scaling; the batch runs with lambda = 1), so every problem's result is the one its own call would give.
 Each problem fails on its own (problem_status): a singular point in problem p leaves p's S reset and its g_S as it was,
-and the other problems are reduced, as separate reference calls would. autotune() times the phase-2 schedules that
-keep that (the block-column owned schedule with staged point operands at several unit sizes, the block-owned pair
-lists) and keeps the fastest; capture() records reset + reduce of the batch as one CUDA graph that step() replays.
+and the other problems are reduced, as separate reference calls would. autotune() times the phase-2 kernels that
+keep that (the block-column owned runs, the gather at several unit sizes, the block-owned pair lists) and keeps the
+fastest; capture() records reset + reduce of the batch as one CUDA graph that step() replays.
 """
 from __future__ import annotations
 
@@ -124,6 +124,7 @@ class BatchedReduction:
         self.nobs = int(sum(p.nobs for p in problems))
         self.graph = None
         self.schedule = "pairs"
+        self.kernel = "stage"   # the plan's own choice, until autotune()
         self.stage_unit = 16
 
     def run(self, sync: bool = True) -> bool:
@@ -134,13 +135,13 @@ class BatchedReduction:
     STAGE_UNITS = (8, 16, 24, 32)
 
     def autotune(self, reps: int = 5) -> dict:
-        """Time the phase-2 schedules that keep per-problem failure on the batch, after a warm-up run each, and keep
-        the fastest: the block-column owned schedule with staged point operands at each unit size of STAGE_UNITS
-        (pairs per thread between two writes to the column tile; keys "stage/8", ...) and the block-owned pair lists
-        ("pairs"). The schedule is left at the winner (stage_unit holds its unit size)."""
-        times = {}
-
-        def timed(key):
+        """Time the phase-2 kernels that keep per-problem failure on the batch, after a warm-up run each, and keep the
+        fastest (`kernel`, as SchurReductionWorkspace.set_kernel takes it): "runs", "gather" at each unit size of
+        STAGE_UNITS (pairs per thread between two writes to the column tile), and "pairs". Returned are the times in ms
+        of the column-owned schedule at each unit size (keys "stage/8", ...: the faster of the runs, which have no
+        units, and the gather at that size) and of the block-owned pair lists ("pairs"); `schedule` and `stage_unit`
+        hold the winner in these terms."""
+        def timed():
             self.run()
             torch.cuda.synchronize()
             a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
@@ -149,20 +150,31 @@ class BatchedReduction:
                 self.run(sync=False)
             b.record()
             torch.cuda.synchronize()
-            times[key] = a.elapsed_time(b) / reps
+            return a.elapsed_time(b) / reps
 
-        self.ws.set_kernel("stage")
+        def choose(kernel, name):
+            """Whether choosing `kernel` launches `name` (a plan may lack a schedule)."""
+            self.ws.set_kernel(kernel)
+            return self.ws.phase2_kernel_name(self.dtype).startswith(name)
+
+        times, kernels = {}, {}
+        runs = timed() if choose("runs", "k_runs") else float("inf")
+        gather = choose("gather", "k_stage36")
         for u in self.STAGE_UNITS:
-            self.ws.set_stage_unit(u)
-            timed(f"stage/{u}")
+            t = float("inf")
+            if gather:
+                self.ws.set_stage_unit(u)
+                t = timed()
+            times[f"stage/{u}"], kernels[f"stage/{u}"] = min((runs, "runs"), (t, "gather"))
         self.ws.set_kernel("pairs")
-        timed("pairs")
+        times["pairs"], kernels["pairs"] = timed(), "pairs"
         best = min(times, key=times.get)
-        self.schedule = best.split("/")[0]
+        self.schedule, self.kernel = best.split("/")[0], kernels[best]
         if self.schedule == "stage":
             self.stage_unit = int(best.split("/")[1])
-            self.ws.set_stage_unit(self.stage_unit)
-        self.ws.set_kernel(self.schedule)
+            if gather:
+                self.ws.set_stage_unit(self.stage_unit)
+        self.ws.set_kernel(self.kernel)
         self.graph = None
         return times
 

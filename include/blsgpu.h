@@ -200,11 +200,11 @@ int bls_schur_plan_instrument(bls_schur_plan* plan, int timing);
  * couplings gathered (sparse S; otherwise as 1). All compute the same reduction; the choice is kept for comparisons and
  * for autotuning. */
 int bls_schur_plan_set_kernel(bls_schur_plan* plan, int which);
-/* No counterpart in the reference (a tuning knob of this build's schedule): rebuild the column-owned schedule (which = 5)
- * with units of at most `unit` pairs for both storage types (1..4096; at plan creation 20 for FP32 storage and 16 for
- * FP64), a unit being one thread's run of one S block's
- * pairs between two writes to the column tile. Sparse plans on the 6/3 fast path only (BLS_EUNSUPPORTED otherwise);
- * on failure the previous schedule stays. Synchronises. */
+/* No counterpart in the reference (a tuning knob of this build's schedule): rebuild the gathering schedule (which = 7) of
+ * both storage types with units of at most `unit` pairs (1..4096; at plan creation 20 for FP32 storage and 16 for FP64),
+ * a unit being one thread's run of one S block's pairs between two writes to the column tile. A schedule that is not
+ * built yet (5 prefers the runs there) takes the size when it is; the runs have no units. Sparse plans on the 6/3 fast
+ * path only (BLS_EUNSUPPORTED otherwise); on failure the previous schedule stays. Synchronises. */
 int bls_schur_plan_set_stage_unit(bls_schur_plan* plan, int unit);
 /* No counterpart in the reference (a batch of the reference's calls in one plan): declare that the plan's structure is
  * the disjoint union of `nprob` independent problems, problem p owning eliminated blocks [point_off[p],
