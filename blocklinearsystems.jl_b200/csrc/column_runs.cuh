@@ -18,7 +18,7 @@
 // column leave their sums of its diagonal block in dpart, and k_runs_diag adds them up in FP64 and subtracts them once: S
 // holds R there, far larger than an item's part, and every subtraction rounds it (60 cameras, 6,000 points, several items a
 // column, S against 64 bits over three inputs: 9.0e-8 to 1.2e-7 with a subtraction per item, 5.3e-8 to 6.4e-8 now; the
-// launch costs 5 us).
+// launch costs 3 us).
 #pragma once
 
 constexpr int kRunThreads = 128;
@@ -536,11 +536,13 @@ __global__ void __launch_bounds__(kRunThreads, 2) k_runs_any(RunArgs<T> a) {
   }
 }
 
-// FP32: the diagonal blocks of the split columns ({r2, first item, items, block}): a thread per entry of the upper triangle
+// FP32: the diagonal blocks of the split columns ({r2, first item, items, block}): a thread per entry of the upper triangle.
+// Launched beside the end of k_runs (programmatic serialisation), it waits for that kernel's results itself.
 template <class T>
 __global__ void __launch_bounds__(128) k_runs_diag(RunArgs<T> a, int64_t nsplit, const int4* __restrict__ split) {
   const int64_t id = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   const int per = a.mdr * a.mdr, e = (int)(id % per), w = e / a.mdr, rho = e - w * a.mdr;
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   if (id / per >= nsplit || !live(a.st)) return;
   const int4 c = __ldg(split + id / per);
   if (rho > w || w >= __ldg(a.r_dims + c.x) || (a.prob_fail && a.prob_fail[a.prob_of_cam[c.x]] != NONE)) return;

@@ -2711,7 +2711,18 @@ static void launch_runs(SchurPlan* P, T* S, bool dense, double* g, const T* C, c
   a.mde = R.mde;
   kern<<<(unsigned)std::min<int64_t>(R.items, R.grid), kRunThreads, R.smem, P->ctx->stream>>>(a);
   if constexpr (F32)
-    if (R.nsplit) k_runs_diag<T><<<grid_for(R.nsplit * R.mdr * R.mdr, 128), 128, 0, P->ctx->stream>>>(a, R.nsplit, R.split.as<int4>());
+    if (R.nsplit) {
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3((unsigned)grid_for(R.nsplit * R.mdr * R.mdr, 128));
+      cfg.blockDim = dim3(128);
+      cfg.stream = P->ctx->stream;
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      attr[0].val.programmaticStreamSerializationAllowed = 1;
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
+      BLS_CUDA(cudaLaunchKernelEx(&cfg, k_runs_diag<T>, a, R.nsplit, (const int4*)R.split.as<int4>()));
+    }
 }
 
 // A 6/3 plan's layout, read back from its device copies (for a schedule that is built after plan creation). Synchronises.
