@@ -559,6 +559,7 @@ __global__ void __launch_bounds__(128) k_runs_diag(RunArgs<T> a, int64_t nsplit,
 // ------------------------------------------------------------------------------------------------------------------
 struct RunInput {
   int64_t nrb, neb, Clen;
+  int nsm;   // the device's SMs
   const int64_t *r_dims, *e_dims, *eptr, *eret, *coffsets;
   const std::vector<int32_t>*rptr, *rentry, *entry_elim;
   const std::vector<int64_t>*bcolptr, *browval;
@@ -613,7 +614,7 @@ static bool build_run_schedule(RunSchedule& R, const RunInput& in, int exact, in
   // its whole tile to S with atomics), else as many as there are resident CTAs, of 24 to 150 visits. 1000 cameras and
   // 200k points, FP32: 250 us; with six per CTA and no lower bound the same there, but a scene of 40 cameras and 8000
   // points took 36 us instead of 25.
-  const int64_t slots = 148 * kCtas;
+  const int64_t slots = in.nsm * kCtas;
   const int64_t avg = std::max<int64_t>({24, nvis / (slots * 4), std::min<int64_t>(150, nvis / slots)});
   const int64_t segv = std::min<int64_t>(avg, kRunMaxVisits);
   struct ColOut {

@@ -102,6 +102,13 @@ inline void allow_smem(const void* kernel) {
   done.insert({kernel, dev});
 }
 
+// The SMs of a device
+inline int sm_count(int device) {
+  int n = 0;
+  BLS_CUDA(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device));
+  return n;
+}
+
 inline int grid_for(int64_t n, int threads) { return (int)((n + threads - 1) / threads); }
 
 // A device buffer that frees itself (unless it is a part of another one, see SmallBufs).

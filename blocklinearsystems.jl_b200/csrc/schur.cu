@@ -2316,7 +2316,7 @@ static SchurPlan* plan_create(bls_ctx* ctx, const bls_schur_plan_desc* d) {
   {
     P->points3 = true;
     for (int64_t e = 0; e < neb && P->points3; ++e) P->points3 = d->e_dims[e] == 3 && d->eoffsets[e] == 9 * e;
-    const RunInput in{nrb, neb, clen, d->r_dims, d->e_dims, d->eliminated_ptr, d->entry_retained, d->coffsets, &rptr, &rentry, &entry_elim, &bcolptr, &browval};
+    const RunInput in{nrb, neb, clen, sm_count(ctx->device), d->r_dims, d->e_dims, d->eliminated_ptr, d->entry_retained, d->coffsets, &rptr, &rentry, &entry_elim, &bcolptr, &browval};
     const bool contiguous = runs_contiguous(in);
     int dr = P->points3 && P->max_dr >= 6 && P->max_dr <= 9 ? P->max_dr : 0;
     for (int64_t r = 0; r < nrb && dr; ++r) dr = d->r_dims[r] == dr ? dr : 0;
@@ -2343,7 +2343,7 @@ static SchurPlan* plan_create(bls_ctx* ctx, const bls_schur_plan_desc* d) {
       for (int64_t r = 0; r < nrb; ++r) cols += rptr[r + 1] > rptr[r];
       const double visits = cols ? (double)nc / cols : 0.0;
       const double kb = neb ? (double)nc / neb * ((double)nb / nrb) : 0.0;   // couplings per point x blocks per column
-      const bool filled = cols >= 148, wide = filled && visits >= 200 && kb >= 800;
+      const bool filled = cols >= in.nsm, wide = filled && visits >= 200 && kb >= 800;
       P->runs_first[0] = !(wide || (filled && visits >= 400 && visits < 1000 && kb >= 300));
       P->runs_first[1] = !(wide || (filled && visits >= 300 && (kb >= 250 || cols < 400)));
     }
@@ -2669,11 +2669,9 @@ static void launch_runs(SchurPlan* P, T* S, bool dense, double* g, const T* C, c
   }
   allow_smem(reinterpret_cast<const void*>(kern));
   if (R.grid == 0) {
-    int per_sm = 0, nsm = 0, dev = 0;
-    BLS_CUDA(cudaGetDevice(&dev));
-    BLS_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+    int per_sm = 0;
     BLS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kRunThreads, R.smem));
-    R.grid = std::max(1, per_sm) * nsm;
+    R.grid = std::max(1, per_sm) * sm_count(P->ctx->device);
   }
   RunArgs<T> a;
   a.items = R.items_d.as<int4>();
@@ -2779,7 +2777,7 @@ static void ensure_runs(SchurPlan* P) {
   const std::vector<int64_t> rd(P->nrblocks, 6), ed(P->neblocks, 3);
   std::vector<int64_t> co(P->ncoup);
   for (int64_t c = 0; c < P->ncoup; ++c) co[c] = 18 * c;
-  const RunInput in{P->nrblocks, P->neblocks, P->C_length, rd.data(), ed.data(), L.eptr.data(), L.eret.data(), co.data(), &L.rptr, &L.rentry,
+  const RunInput in{P->nrblocks, P->neblocks, P->C_length, sm_count(P->ctx->device), rd.data(), ed.data(), L.eptr.data(), L.eret.data(), co.data(), &L.rptr, &L.rentry,
                     &L.entry_elim, &L.bcolptr, &L.browval};
   for (int sd = 0; sd < 2; ++sd) {
     if (P->runs[sd].ok) continue;
@@ -2864,11 +2862,9 @@ static int reduce(SchurPlan* P, T* S, bool dense, double* g, const double* b_r, 
       if (ev0) BLS_CUDA(cudaEventRecord(ev0, s));
       P->launches += 1;
       if (P->stage_grid[sizeof(T) == 4 ? 0 : 1] == 0) {
-        int per_sm = 0, nsm = 0, dev = 0;
-        BLS_CUDA(cudaGetDevice(&dev));
-        BLS_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+        int per_sm = 0;
         BLS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_stage36<T>, stage_nt<T>(), smem));
-        P->stage_grid[sizeof(T) == 4 ? 0 : 1] = std::max(1, per_sm) * nsm;
+        P->stage_grid[sizeof(T) == 4 ? 0 : 1] = std::max(1, per_sm) * sm_count(P->ctx->device);
       }
       const int64_t grid = std::min<int64_t>(SS.items, P->stage_grid[sizeof(T) == 4 ? 0 : 1]);
       k_stage36<T><<<(unsigned)grid, stage_nt<T>(), smem, s>>>(
