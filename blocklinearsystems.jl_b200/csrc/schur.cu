@@ -2327,25 +2327,28 @@ static SchurPlan* plan_create(bls_ctx* ctx, const bls_schur_plan_desc* d) {
     if (gather) {
       // k_runs against k_stage36 for a sparse S of 6 x 6 blocks (against the block-owned pairs it is ahead everywhere).
       // k_stage36 keeps a column's point operands in shared memory for the whole column and adds a block to its tile
-      // once; k_runs brings in every coupling of a point before the visit's, and adds a block once per segment. So the
-      // number of couplings per point times the number of blocks per column decides, with the visits per column (few: a
-      // column is no work for a CTA of k_stage36; above ~1000 in FP32, its items are cut) and the number of columns (few
-      // do not fill k_stage36's CTAs; in FP64 some hundreds fill those better than k_runs's). us, k_stage36 / k_runs, by
-      // visits, blocks and couplings per point; 1,000 to 1,500 cameras where nothing is said:
-      //   FP32  350, 127, 5: 169 / 131      450, 31, 8: 142 / 126      450, 112, 8: 138 / 151     450, 113, 12: 156 / 197
-      //         600, 31, 5: 210 / 167       600, 118, 8 (6,000): 820 / 933      600, 38, 8 (300): 50 / 62
-      //         700, 40, 8: 181 / 187       766, 121, 7.7 (10,000): 1553 / 1760         850, 40, 5: 236 / 224
-      //         850, 87, 5: 229 / 236       1200, 61, 6: 320 / 250      1300, 113, 8: 372 / 367 1300, 114, 12: 487 / 489
-      //   FP64  200, 121, 5: 160 / 150      350, 40, 5: 194 / 170       350, 85, 5: 192 / 208   450, 31, 8: 248 / 216
-      //         600, 31, 5: 332 / 255       600, 31, 8 (6,000): 1467 / 1390     600, 38, 8 (300): 94 / 108
-      //         700, 40, 8: 345 / 343       1200, 61, 6: 401 / 461      1300, 31, 8: 626 / 565  1300, 113, 8: 561 / 652
+      // once; k_runs brings in every coupling of a point before the visit's, and adds a block once per segment. So many
+      // couplings per point times many blocks per column (kb) speak for k_stage36; few visits (a column is no work for a
+      // CTA) and few columns (they don't fill its CTAs) for k_runs; columns of one item each, 0.7 to some per SM, fill
+      // k_stage36's CTAs evenly and k_runs's not. The lines are those of the least loss over 3,160 scenes drawn from 30
+      // to 3,000 cameras, 46 to 2,500 visits and 14 to 116 blocks per column, 3 to 10 couplings per point, timed with
+      // both kernels (a loss against k_stage36 counted three times). Against the faster kernel of each scene the choice
+      // costs 1.1% (FP64) and 1.0% (FP32) on average; it is more than 10% off in 4% of them and at worst 1.3 and 1.4
+      // times. Some of them, us, k_stage36 / k_runs, by columns, visits, blocks and couplings per point:
+      //   FP32  1000, 350, 127, 5: 169 / 131    1000, 450, 112, 8: 138 / 151    1000, 600, 31, 5: 210 / 167
+      //         1000, 1200, 61, 6: 320 / 250    10000, 766, 121, 7.7: 1553 / 1760     300, 600, 38, 8: 50 / 62
+      //         187, 71, 58, 4: 30 / 36 (lost)  275, 780, 38, 4: 54 / 67 (lost)
+      //   FP64  1000, 350, 40, 5: 194 / 170     1000, 450, 31, 8: 248 / 216     1000, 1200, 61, 6: 401 / 461
+      //         6000, 600, 31, 8: 1467 / 1390   300, 600, 38, 8: 94 / 108       93, 1053, 47, 10: 83 / 99
+      //         1000, 200, 121, 5: 160 / 150 (lost)   307, 135, 91, 8: 46 / 58      58, 2296, 27, 3: 47 / 58 (lost)
       int64_t cols = 0;
       for (int64_t r = 0; r < nrb; ++r) cols += rptr[r + 1] > rptr[r];
-      const double visits = cols ? (double)nc / cols : 0.0;
-      const double kb = neb ? (double)nc / neb * ((double)nb / nrb) : 0.0;   // couplings per point x blocks per column
-      const bool filled = cols >= in.nsm, wide = filled && visits >= 200 && kb >= 800;
-      P->runs_first[0] = !(wide || (filled && visits >= 400 && visits < 1000 && kb >= 300));
-      P->runs_first[1] = !(wide || (filled && visits >= 300 && (kb >= 250 || cols < 400)));
+      const double per_sm = (double)cols / in.nsm, visits = cols ? (double)nc / cols : 0.0, blocks = cols ? (double)nb / cols : 0.0;
+      const double kb = neb ? (double)nc / neb * blocks : 0.0;
+      P->runs_first[0] = !((per_sm >= 1 && visits >= 200 && kb >= 800) || (per_sm >= 1.2 && visits >= 400 && visits < 900 && kb >= 300) ||
+                           (per_sm >= 0.7 && per_sm < 2.7 && visits >= 100 && visits < 800 && blocks >= 50));
+      P->runs_first[1] = !((per_sm >= 1.2 && visits >= 120 && kb >= 350) ||
+                           (per_sm >= (visits >= 700 ? 0.6 : 0.7) && per_sm < 5.5 && visits >= 200 && blocks >= 25 && kb >= 100));
     }
     // a plan of 6 x 6 blocks for a sparse S builds per storage type the schedule that "stage" takes (the other one when it
     // cannot be built, or when it is chosen by name: ensure_gather, ensure_runs); every other plan has the runs only
