@@ -195,7 +195,8 @@ int bls_schur_plan_instrument(bls_schur_plan* plan, int timing);
  * per pair list (the default of a plan with neither 6 nor 7), 2 = block owned, a lane per pair and a warp per pair list, 3 = block-column owned with
  * visits staged in chunks (sparse S without conditioning scales; otherwise as 1), 4 = point-major, six lanes per pair,
  * entries added into S with vector reductions (as 1 when S has 2^25 or more blocks), 5 = block-column owned, the faster
- * of 6 and 7 for the plan's columns and storage type (6 for a dense S; the default), 6 = block-column owned with the couplings of a
+ * of 6 and 7 for the plan's columns and storage type (for a dense S 6, or as 1 where the plan's sparse pattern prefers 7;
+ * the default), 6 = block-column owned with the couplings of a
  * column's points staged as contiguous runs, 7 = block-column owned with the point operands of a column staged and the
  * couplings gathered (sparse S; otherwise as 1). All compute the same reduction; the choice is kept for comparisons and
  * for autotuning. */
