@@ -807,6 +807,8 @@ def run_ours_batch(args, rank: int, world: int) -> dict | None:
 
     B64 = bls.batch.BatchedReduction(problems, torch.float64, device=dev.index)
     tunes64 = B64.autotune()
+    chosen = lambda b: b.kernel + (f"/{b.stage_unit}" if b.kernel == "gather" else "")
+    chosen64 = chosen(B64)
     B64.capture()
     ms64 = timed(B64)
     S64 = B64.S.cpu().numpy()
@@ -856,7 +858,7 @@ def run_ours_batch(args, rank: int, world: int) -> dict | None:
                    "observations": nobs, "nnz_S": int(B.U.nnz), "parallelism": f"replicas x{world}",
                    "l2": "flushed between timed steps (256 MB write)",
                    "step": "one CUDA graph replay: reset_schur_sparse + reduce_schur_sparse of all problems (disjoint-union plan)"},
-        "schedule": {"chosen": B.kernel + (f"/{B.stage_unit}" if B.kernel == "gather" else ""), "autotune_ms": tunes, "fp64_chosen": min(tunes64, key=tunes64.get), "fp64_autotune_ms": tunes64},
+        "schedule": {"chosen": chosen(B), "autotune_ms": tunes, "fp64_chosen": chosen64, "fp64_autotune_ms": tunes64},
         "fp64": {"value": world * nobs * args.steps / (ms64 / 1e3), "unit": "obs/s", "ms_per_step": ms64 / args.steps},
         "per_problem_error_vs_fp64": {"max": max(errs), "median": float(np.median(errs)), "norm": "||S_mixed - S_fp64|| / ||S_fp64|| per problem"},
         "e2e": {"value": world * nobs * args.steps / (e2e_ms / 1e3), "unit": "obs/s",
